@@ -673,7 +673,7 @@ def config0_leg(stream) -> dict:
     o.err64()
     o.image()
     cpu_s = time.perf_counter() - t0
-    kernel = s.kernel
+    kernel = s.resident or s.kernel
     s.close()
     return {"workload": f"circle256 GridSolver FP32 Jacobi, 5000 sweeps, 'src' gradient "
                         f"({unknowns} unknowns, {mc.shape[0]}x{mc.shape[1]} crop)",

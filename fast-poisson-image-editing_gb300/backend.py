@@ -307,6 +307,14 @@ class GridSolver(_Solver):
         _abi.call("fpie_grid_kernel", self._h, buf, 64)
         return buf.value.decode()
 
+    @property
+    def resident(self) -> str:
+        """The resident kernel that runs this grid's FP32 Jacobi sweeps, ""
+        if they run on the tile kernel named by ``kernel``."""
+        buf = ctypes.create_string_buffer(64)
+        _abi.call("fpie_grid_resident", self._h, buf, 64)
+        return buf.value.decode()
+
     def reset_images(self, src, mask, tgt, mask_on_src: tuple[int, int],
                      mask_on_tgt: tuple[int, int], gradient: str = "max") -> tuple[int, int, int, int]:
         """Build the inputs on the GPU from uint8 images (GridProcessor.reset semantics).

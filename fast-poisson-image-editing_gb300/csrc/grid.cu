@@ -20,6 +20,7 @@
 #include "grid_kernels.cuh"
 #include "grid_mixed.cuh"
 #include "grid_flow.cuh"
+#include "grid_res.cuh"
 #include "grid_tma.cuh"
 #include "grid_tb.cuh"
 #include "prep.cuh"
@@ -43,6 +44,13 @@ __global__ void grid_inputs_unpack_kernel(GridGeom G, const uint8_t* __restrict_
 
 // ---- layout conversion kernels ------------------------------------------------
 
+// Whether a state value or a masked pixel's gradient lies outside the range
+// in which the resident kernel's quartered sums are exact (grid_res.cu).
+__device__ __forceinline__ bool out_of_range(float v) { return !(fabsf(v) <= 0x1p40f); }
+__device__ __forceinline__ bool grad_out_of_range(float v) {
+  return out_of_range(v) || (v != 0.f && fabsf(v) < 0x1p-60f);
+}
+
 // An equation system that is a 4-neighbour raster stencil, on the grid:
 // unknown i (1..N-1) at crop pixel pos[i] (row-major, G.m per row) gets its
 // X as state and its B as "grad"; every other pixel stays 0 and unmasked,
@@ -52,7 +60,8 @@ __global__ void grid_from_equ_kernel(GridGeom G, int N, const int* __restrict__ 
                                      const float* __restrict__ xe, const float* __restrict__ be,
                                      long long np, uint8_t* __restrict__ mask,
                                      float* __restrict__ x0, float* __restrict__ x1,
-                                     float* __restrict__ g) {
+                                     float* __restrict__ g, unsigned* __restrict__ wild) {
+  bool bad = false;
   for (long long i = 1 + blockIdx.x * (long long)blockDim.x + threadIdx.x; i < N;
        i += (long long)gridDim.x * blockDim.x) {
     const int p = pos[i];
@@ -63,9 +72,12 @@ __global__ void grid_from_equ_kernel(GridGeom G, int N, const int* __restrict__ 
       const float v = xe[c * np + i];
       x0[c * G.plane + q] = v;
       x1[c * G.plane + q] = v;
-      g[c * G.plane + q] = be[c * np + i];
+      const float b = be[c * np + i];
+      g[c * G.plane + q] = b;
+      bad = bad || out_of_range(v) || grad_out_of_range(b);
     }
   }
+  if (bad) *wild = 1;
 }
 
 // The unknowns' state back into planar X (row 0 untouched).
@@ -86,21 +98,26 @@ __global__ void grid_pack_kernel(GridGeom G, const int32_t* __restrict__ mk,
                                  const float* __restrict__ gr,
                                  uint8_t* __restrict__ mask,
                                  float* __restrict__ x0, float* __restrict__ x1,
-                                 float* __restrict__ g) {
+                                 float* __restrict__ g, unsigned* __restrict__ wild) {
   const long long total = (long long)G.n * G.m;
+  bool bad = false;
   for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
        idx < total; idx += (long long)gridDim.x * blockDim.x) {
     const int i = (int)(idx / G.m), j = (int)(idx % G.m);
     const long long p = G.at(i, j);
-    mask[p] = mk[idx] != 0;
+    const bool on = mk[idx] != 0;
+    mask[p] = on;
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
       const float v = t[idx * 3 + c];
       x0[c * G.plane + p] = v;
       x1[c * G.plane + p] = v;
-      g[c * G.plane + p] = gr[idx * 3 + c];
+      const float b = gr[idx * 3 + c];
+      g[c * G.plane + p] = b;
+      bad = bad || out_of_range(v) || (on && grad_out_of_range(b));
     }
   }
+  if (bad) *wild = 1;
 }
 
 __global__ void grid_unpack_kernel(GridGeom G, const float* __restrict__ x,
@@ -177,6 +194,38 @@ struct GridSolverImpl : Solver {
   int ft_k = 0;  // depth the tables were built for
   bool ft_ok = false;
   int flow_grid = 0;
+
+  // ---- resident kernel (grid_res.cu) -------------------------------------------
+  // FP32 Jacobi sweeps of a grid whose tiles all fit on the device at once.
+  ResShape res{0, 0, 0, 0};        // this geometry's shape; rows == 0: none
+  std::string res_pin;          // pinned by name ("" otherwise)
+  void* res_exchange = nullptr; // packets and activity words
+  unsigned* res_ctl = nullptr;  // epoch base, exit count; then the range mark
+  unsigned* wild() const { return res_ctl + kResCtl; }
+  bool maybe_wild = false;      // the range mark may be set
+
+  bool use_res() const {
+    return precision == FPIE_FP32 && !red_black && res.rows > 0 && (!pinned || !res_pin.empty());
+  }
+
+  void run_res(int iters) {
+    if (!res_exchange) {
+      const size_t b = res_exchange_bytes(G);
+      FPIE_CUDA(cudaMalloc(&res_exchange, b));
+      FPIE_CUDA(cudaMemsetAsync(res_exchange, 0, b, stream));
+    }
+    ensure_wait_flag();
+    launch_res(G, res, mask, g, x[cur], x[cur ^ 1], res_exchange, res_ctl, wild(), iters,
+               d_wait_err, spin_limit, stream);
+    post_launch(this);
+    cur ^= 1;
+  }
+
+  // Before a reset writes the planes: no value seen out of range yet.
+  void clear_wild() {
+    if (maybe_wild) FPIE_CUDA(cudaMemsetAsync(wild(), 0, sizeof(unsigned), stream));
+    maybe_wild = false;
+  }
 
   // Reads and clears the wait-error flag (a flow-kernel neighbourhood wait
   // or a TMA copy wait that gave up); call after the stream has been
@@ -298,6 +347,10 @@ struct GridSolverImpl : Solver {
     release_mixed();
     cudaFree(d_wait_err);
     cudaFree(tma_list);
+    cudaFree(res_exchange);
+    cudaFree(res_ctl);
+    res_exchange = nullptr;
+    res_ctl = nullptr;
     cudaFree(flow_inv);
     cudaFree(flow_done);
     cudaFree(flow_rec);
@@ -333,6 +386,7 @@ struct GridSolverImpl : Solver {
       // pointers stay valid).  The halo is still zero; the interior is
       // rewritten by the pack kernel.
       cur = 0;
+      clear_wild();
       ready = false;
       flags_ok = false;  // the new mask may activate other tiles
       mflags_ok = false;
@@ -353,6 +407,10 @@ struct GridSolverImpl : Solver {
     FPIE_CUDA(cudaMalloc(&d_img, (size_t)n * m * 3));
     FPIE_CUDA(cudaMalloc(&d_part, (size_t)L.nparts * 3 * sizeof(double)));
     FPIE_CUDA(cudaMalloc(&d_err, 3 * sizeof(float)));
+    FPIE_CUDA(cudaMalloc(&res_ctl, (kResCtl + 1) * sizeof(unsigned)));
+    FPIE_CUDA(cudaMemsetAsync(res_ctl, 0, (kResCtl + 1) * sizeof(unsigned), stream));
+    maybe_wild = false;
+    res = res_pin.empty() ? res_pick(n, m) : res_named(res_pin.c_str(), n, m);
     FPIE_CUDA(cudaMemsetAsync(x[0], 0, 3 * pb, stream));
     FPIE_CUDA(cudaMemsetAsync(x[1], 0, 3 * pb, stream));
     FPIE_CUDA(cudaMemsetAsync(g, 0, 3 * pb, stream));
@@ -363,8 +421,9 @@ struct GridSolverImpl : Solver {
   void pack(const int32_t* dmask, const float* dtgt, const float* dgrad) {
     const long long total = (long long)G.n * G.m;
     grid_pack_kernel<<<conv_blocks(total), 256, 0, stream>>>(
-        G, dmask, dtgt, dgrad, mask, x[0], x[1], g);
+        G, dmask, dtgt, dgrad, mask, x[0], x[1], g, wild());
     post_launch(this);
+    maybe_wild = true;
     ready = true;
   }
 
@@ -402,8 +461,9 @@ struct GridSolverImpl : Solver {
     FPIE_CUDA(cudaMemsetAsync(mask, 0, (size_t)G.plane, stream));
     if (N > 1) {
       grid_from_equ_kernel<<<conv_blocks(N), 256, 0, stream>>>(G, N, pos, xe, be, np, mask, x[0],
-                                                               x[1], g);
+                                                               x[1], g, wild());
       post_launch(this);
+      maybe_wild = true;
     }
     ready = true;
   }
@@ -637,6 +697,7 @@ struct GridSolverImpl : Solver {
     red_black = on;
     select_variant(on ? red_black_variant() : default_variant());
     pinned = tuned = false;
+    pin_res("");
   }
 
   // k sweeps (k <= depth()) from buffer `from`; flips nothing (caller does).
@@ -782,6 +843,12 @@ struct GridSolverImpl : Solver {
       run_mixed(iters);
       return;
     }
+    if (use_res()) {
+      run_res(iters);
+      return;
+    }
+    FPIE_REQUIRE(res_pin.empty() || red_black, FPIE_ERR_ARG,
+                 "the grid's tiles do not fit on the device: no '" + res_pin + "' sweeps");
     if (!tuned && !pinned) iters -= autotune(iters);
     if (is_flow(variant)) {
       if (iters > 0) run_flow(iters);
@@ -1061,6 +1128,7 @@ struct GridSolverImpl : Solver {
     if (name == "auto") {
       pinned = false;
       tuned = false;
+      pin_res("");
       std::lock_guard<std::mutex> lk(tune_mutex());
       tune_cache().erase({G.n, G.m, red_black});
       return;
@@ -1075,6 +1143,11 @@ struct GridSolverImpl : Solver {
       pinned = true;
       return;
     }
+    if (res_is_name(name.c_str())) {
+      pin_res(name);
+      pinned = true;
+      return;
+    }
     int v = -100;  // unknown
     if (name == "sweep1") v = -1;
     if (name == "p16w8k16t") v = kTma;
@@ -1085,11 +1158,26 @@ struct GridSolverImpl : Solver {
     for (size_t k = 0; k < tb_variants().size(); ++k)
       if (name == tb_variants()[k].name && !tb_variants()[k].red_black) v = (int)k;
     FPIE_REQUIRE(v != -100, FPIE_ERR_ARG, "unknown grid kernel '" + name + "'");
+    pin_res("");
     select_variant(v);
     pinned = true;
   }
 
+  void pin_res(const std::string& name) {
+    res_pin = name;
+    if (x[0]) res = name.empty() ? res_pick(G.n, G.m) : res_named(name.c_str(), G.n, G.m);
+  }
+
+  // Name of the resident kernel the FP32 Jacobi sweeps of this grid run on
+  // ("" if they run on the tile kernel that kernel_name() names).
+  std::string resident_name() const {
+    if (!use_res()) return "";
+    return "p" + std::to_string(res.rows) + "w" + std::to_string(res.warps) + "x" +
+           std::to_string(res.width) + "k" + std::to_string(res.depth) + "r";
+  }
+
   std::string kernel_name() const {
+    if (!res_pin.empty() && precision == FPIE_FP32 && !red_black) return res_pin;
     if (precision != FPIE_FP32)
       return mvariant == kFlow ? std::string("p16w8k16d") : std::string(mixed_variants()[mvariant].name);
     if (variant == kTma) return std::string("p16w8k16t");
@@ -1108,6 +1196,7 @@ struct GridSolverImpl : Solver {
     if (p != precision) {
       precision = p;
       pinned = false;
+      pin_res("");
       drop_graphs();
     }
   }
@@ -1227,6 +1316,14 @@ int fpie_grid_kernel(fpie_solver* s, char* buf, int len) {
   return guarded([&] {
     FPIE_REQUIRE(buf != nullptr && len > 0, FPIE_ERR_ARG, "null or empty buffer");
     const std::string k = grid_of(s)->kernel_name();
+    std::snprintf(buf, (size_t)len, "%s", k.c_str());
+  });
+}
+
+int fpie_grid_resident(fpie_solver* s, char* buf, int len) {
+  return guarded([&] {
+    FPIE_REQUIRE(buf != nullptr && len > 0, FPIE_ERR_ARG, "null or empty buffer");
+    const std::string k = grid_of(s)->resident_name();
     std::snprintf(buf, (size_t)len, "%s", k.c_str());
   });
 }

@@ -262,8 +262,10 @@ int fpie_grid_solve(fpie_solver* s, double tol, int max_sweeps, int check_every,
  * sweeps on 104x104 tiles; FP32 Jacobi only), "p16w8k16dp" / "p16w8k12dp"
  * (the same two with selects only at the unmasked pixels next to masked
  * ones where a region's mask edge is straight; FP32 Jacobi only) or
- * "p16w8k16t" (persistent CTAs prefetching each region by TMA).  Every
- * choice gives bit-identical results. */
+ * "p16w8k16t" (persistent CTAs prefetching each region by TMA), or a
+ * resident kernel ("p8w4x64k16r", ...: tiles held in registers for the whole
+ * step; sweeping a grid whose tiles do not fit at once is FPIE_ERR_ARG).
+ * Every choice gives bit-identical results. */
 int fpie_grid_set_kernel(fpie_solver* s, const char* name);
 
 /* The dependency-flow kernels ("p16w8k16d", "p16w8k12d" and their "dp"
@@ -273,8 +275,15 @@ int fpie_grid_set_kernel(fpie_solver* s, const char* name);
  * FPIE_ERR_TIMEOUT, leaving the state undefined.  Default 2^26. */
 int fpie_grid_set_spin_limit(fpie_solver* s, long long spins);
 
-/* Writes the current grid sweep kernel's name (NUL-terminated) into buf. */
+/* Writes the current grid sweep kernel's name (NUL-terminated) into buf: the
+ * tile kernel that runs the sweeps of grids that are not resident. */
 int fpie_grid_kernel(fpie_solver* s, char* buf, int len);
+
+/* Writes the name of the resident kernel ("p<R>w<W>x<width>k<K>r") that runs the
+ * loaded grid's FP32 Jacobi sweeps, or "" if they run on the tile kernel.
+ * Unless a kernel is pinned, grids whose tiles all fit on the device at once
+ * are resident. */
+int fpie_grid_resident(fpie_solver* s, char* buf, int len);
 
 /* ---- allocation-free grid step ---------------------------------------------
  * No counterpart in the reference: an addition for callers that cannot
