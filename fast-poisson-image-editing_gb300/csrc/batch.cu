@@ -475,7 +475,8 @@ struct Batch {
       alloc(&j.mask, (size_t)j.G.plane);
       alloc(&j.img, (size_t)n * m * 3);
       alloc(&j.parts, (size_t)j.L.nparts * 6 * sizeof(double));
-      alloc(&j.err, 3 * sizeof(float));
+      alloc(&j.err, 4 * sizeof(float));  // and the finish kernel's count
+      FPIE_CUDA(cudaMemsetAsync(j.err, 0, 4 * sizeof(float), stream));
       alloc(&j.norm, 6 * sizeof(double));
       if (precision != FPIE_FP32) {
         const size_t eb = (size_t)j.G.plane * 3 * 2, rb = (size_t)j.G.plane * 3 * sizeof(float);
@@ -929,10 +930,10 @@ struct Batch {
 
   void finish(int id) {
     BatchJob& j = job(id);
-    launch_grid_finish(j.L, j.G, j.mask, j.g, j.x[j.cur], j.img, j.parts, stream);
-    launch_finalize(j.parts, j.L.nparts, j.err, stream);
+    launch_grid_finish(j.L, j.G, j.mask, j.g, j.x[j.cur], j.img, j.parts,
+                       reinterpret_cast<unsigned*>(j.err + 3), j.err, stream);
     FPIE_CUDA(cudaGetLastError());
-    launches += 2;
+    ++launches;
   }
 
   void result(int id, uint8_t* img, float* err) {

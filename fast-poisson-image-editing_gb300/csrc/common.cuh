@@ -114,6 +114,12 @@ inline GridGeom make_geom(int n, int m) {
   return g;
 }
 
+// Rows per thread of kernels whose threads own 4 columns and go downwards:
+// one while the grid has fewer groups of 4 pixels than the device has threads
+// (a chain of dependent row loads would be all that such a kernel takes: 14 us
+// against 6 with 4 rows on a 152x152 grid), up to 8 beyond.
+int rows_per_thread(const GridGeom& g);
+
 // ---- device helpers -----------------------------------------------------------
 // The update keeps the numpy backend's evaluation order exactly:
 // ((((g + up) + down) + left) + right) * 0.25  (x/4 and x*0.25 round alike).
@@ -173,6 +179,71 @@ __device__ __forceinline__ void block_sum3(double& a, double& b, double& c) {
       b += __shfl_down_sync(0xffffffffu, b, o);
       c += __shfl_down_sync(0xffffffffu, c, o);
     }
+  }
+}
+
+// A sum of floats as hi + lo (Knuth's error-free addition): FP64 adds run at
+// about two per SM and cycle here, and the residual sum's made up most of the
+// finish kernels' time.  hi + lo is exact to about 2^-46 of the sum, which the
+// block partials and the total then carry in double.
+struct Sum2 {
+  float hi = 0.f, lo = 0.f;
+};
+__device__ __forceinline__ void sum2_add(Sum2& s, float v) {
+  const float t = __fadd_rn(s.hi, v), b = __fsub_rn(t, s.hi);
+  s.lo = __fadd_rn(s.lo, __fadd_rn(__fsub_rn(s.hi, __fsub_rn(t, b)), __fsub_rn(v, b)));
+  s.hi = t;
+}
+// The value; where hi overflowed or is no number, hi alone.
+__device__ __forceinline__ double sum2_value(const Sum2& s) {
+  return isfinite(s.hi) ? (double)s.hi + (double)s.lo : (double)s.hi;
+}
+
+// Block-wide sums of acc[3] to parts[3 * block ...], and by the last block to
+// arrive the total of all blocks' parts to err[3], in a fixed order.  256
+// threads; every thread of every block calls it.  count: a device word, 0
+// before the first launch; the last block clears it.
+__device__ __forceinline__ void finish_sums(Sum2 (&acc)[3], unsigned block, unsigned blocks,
+                                            double* parts, unsigned* count, float* err) {
+  __shared__ double sh[3][8];
+  __shared__ bool last;
+  const int tid = threadIdx.x + threadIdx.y * blockDim.x, lane = tid & 31, warp = tid >> 5;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const float h = __shfl_down_sync(0xffffffffu, acc[c].hi, o);
+      const float l = __shfl_down_sync(0xffffffffu, acc[c].lo, o);
+      sum2_add(acc[c], h);
+      acc[c].lo = __fadd_rn(acc[c].lo, l);
+    }
+  if (lane == 0)
+#pragma unroll
+    for (int c = 0; c < 3; ++c) sh[c][warp] = sum2_value(acc[c]);
+  __syncthreads();
+  if (tid < 3) {
+    double t = 0.0;
+    for (int w = 0; w < 8; ++w) t += sh[tid][w];
+    parts[3 * (size_t)block + tid] = t;
+    __threadfence();
+  }
+  __syncthreads();
+  if (tid == 0) last = atomicAdd(count, 1u) == blocks - 1;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  double a = 0.0, b = 0.0, c = 0.0;
+  for (unsigned k = tid; k < blocks; k += 256) {
+    a += __ldcg(parts + 3 * (size_t)k);
+    b += __ldcg(parts + 3 * (size_t)k + 1);
+    c += __ldcg(parts + 3 * (size_t)k + 2);
+  }
+  block_sum3(a, b, c);
+  if (tid == 0) {
+    err[0] = (float)a;
+    err[1] = (float)b;
+    err[2] = (float)c;
+    *count = 0;
   }
 }
 

@@ -132,9 +132,10 @@ __global__ void equ_colour_kernel(EquGeom E, const int4* __restrict__ A, int n_m
 __global__ void __launch_bounds__(256)
 equ_finish_kernel(EquGeom E, const int4* __restrict__ A,
                   const float* __restrict__ b, const float* __restrict__ x,
-                  uint8_t* __restrict__ img, double* __restrict__ parts) {
+                  uint8_t* __restrict__ img, double* __restrict__ parts,
+                  unsigned* __restrict__ count, float* __restrict__ err) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  double acc[3] = {0.0, 0.0, 0.0};
+  Sum2 acc[3];
   if (i < E.N) {
     const int4 a = __ldg(A + i);
 #pragma unroll
@@ -145,16 +146,11 @@ equ_finish_kernel(EquGeom E, const int4* __restrict__ A,
       s = __fadd_rn(s, __ldg(xc + a.z));
       s = __fadd_rn(s, __ldg(xc + a.w));
       const float xi = xc[i];
-      acc[c] = fabsf(__fsub_rn(s, __fmul_rn(4.0f, xi)));
+      acc[c].hi = fabsf(__fsub_rn(s, __fmul_rn(4.0f, xi)));
       img[(long long)i * 3 + c] = clip_u8(xi);
     }
   }
-  block_sum3(acc[0], acc[1], acc[2]);
-  if (threadIdx.x == 0) {
-    parts[3 * (long long)blockIdx.x + 0] = acc[0];
-    parts[3 * (long long)blockIdx.x + 1] = acc[1];
-    parts[3 * (long long)blockIdx.x + 2] = acc[2];
-  }
+  finish_sums(acc, blockIdx.x, gridDim.x, parts, count, err);
 }
 
 static int conv_blocks(long long total) { return stride_blocks(total, 256, 32); }
@@ -325,6 +321,8 @@ struct EquSolverImpl : Solver {
   unsigned int* d_bad = nullptr;
   float* h_err = nullptr;
   unsigned int* h_bad = nullptr;
+  int* h_box = nullptr;  // pinned, for the GPU-side reset's bounding box
+  int* d_box = nullptr;  // its accumulators
   int nparts = 0;
   static constexpr int kChunk = 64;
   cudaGraphExec_t chunk[2] = {nullptr, nullptr};
@@ -376,6 +374,8 @@ struct EquSolverImpl : Solver {
     cudaFree(d_bad);
     if (h_err) cudaFreeHost(h_err);
     if (h_bad) cudaFreeHost(h_bad);
+    if (h_box) cudaFreeHost(h_box);
+    cudaFree(d_box);
     if (own_stream) cudaStreamDestroy(own_stream);
   }
 
@@ -667,7 +667,8 @@ struct EquSolverImpl : Solver {
     FPIE_CUDA(cudaMalloc(&b, pb));
     FPIE_CUDA(cudaMalloc(&d_img, (size_t)N * 3));
     FPIE_CUDA(cudaMalloc(&d_part, (size_t)nparts * 3 * sizeof(double)));
-    FPIE_CUDA(cudaMalloc(&d_err, 3 * sizeof(float)));
+    FPIE_CUDA(cudaMalloc(&d_err, 4 * sizeof(float)));  // and the finish kernel's count
+    FPIE_CUDA(cudaMemsetAsync(d_err, 0, 4 * sizeof(float), stream));
     FPIE_CUDA(cudaMemsetAsync(x[0], 0, pb, stream));
     FPIE_CUDA(cudaMemsetAsync(x[1], 0, pb, stream));
     FPIE_CUDA(cudaMemsetAsync(b, 0, pb, stream));
@@ -727,31 +728,34 @@ struct EquSolverImpl : Solver {
     FPIE_REQUIRE(mode >= 0 && mode <= 2, FPIE_ERR_ARG, "gradient mode must be 0 (src), 1 (avg), 2 (max)");
     const size_t sb = (size_t)sh * sw * 3, mb = (size_t)mh * mw * mch, tb = (size_t)th * tw * 3;
     const size_t mpx = (size_t)mh * mw;
-    const size_t head = on_device ? 0 : (sb + mb + tb + 15) / 16 * 16;
-    // staging: images (host path) | box (16 B) | m01 | crop ids (<= mpx ints) | block counts
+    const size_t ms = (sb + 15) / 16 * 16, ts = ms + (mb + 15) / 16 * 16;  // staged mask, target
+    const size_t head = on_device ? 0 : ts + (tb + 15) / 16 * 16;
+    // staging: images (host path) | m01 | crop ids (<= mpx ints) | block counts
     const size_t nb_max = (mpx + 1023) / 1024 + 2;
-    const size_t bytes = head + 16 + (mpx + 15) / 16 * 16 + mpx * 4 + nb_max * 4;
+    const size_t bytes = head + (mpx + 15) / 16 * 16 + mpx * 4 + nb_max * 4;
     AsyncScratch scratch(bytes, stream);
     char* stage = scratch.bytes();
     const uint8_t *dsrc = src, *dmsk = msk, *dtgt = tgt;
     if (!on_device) {
       FPIE_CUDA(cudaMemcpyAsync(stage, src, sb, cudaMemcpyHostToDevice, stream));
-      FPIE_CUDA(cudaMemcpyAsync(stage + sb, msk, mb, cudaMemcpyHostToDevice, stream));
-      FPIE_CUDA(cudaMemcpyAsync(stage + sb + mb, tgt, tb, cudaMemcpyHostToDevice, stream));
+      FPIE_CUDA(cudaMemcpyAsync(stage + ms, msk, mb, cudaMemcpyHostToDevice, stream));
+      FPIE_CUDA(cudaMemcpyAsync(stage + ts, tgt, tb, cudaMemcpyHostToDevice, stream));
       dsrc = reinterpret_cast<uint8_t*>(stage);
-      dmsk = reinterpret_cast<uint8_t*>(stage + sb);
-      dtgt = reinterpret_cast<uint8_t*>(stage + sb + mb);
+      dmsk = reinterpret_cast<uint8_t*>(stage + ms);
+      dtgt = reinterpret_cast<uint8_t*>(stage + ts);
     }
-    int* dbox = reinterpret_cast<int*>(stage + head);
-    uint8_t* m01 = reinterpret_cast<uint8_t*>(stage + head + 16);
-    int* ids = reinterpret_cast<int*>(stage + head + 16 + (mpx + 15) / 16 * 16);
+    uint8_t* m01 = reinterpret_cast<uint8_t*>(stage + head);
+    int* ids = reinterpret_cast<int*>(stage + head + (mpx + 15) / 16 * 16);
     int* counts = ids + mpx;
-    int hbox[4] = {INT32_MAX, -1, INT32_MAX, -1};
-    FPIE_CUDA(cudaMemcpyAsync(dbox, hbox, sizeof(hbox), cudaMemcpyHostToDevice, stream));
-    launch_prep_mask(dmsk, mh, mw, mch, m01, dbox, stream);
+    if (!h_box) FPIE_CUDA(cudaMallocHost(&h_box, 4 * sizeof(int)));
+    if (!d_box) {
+      FPIE_CUDA(cudaMalloc(&d_box, kPrepAcc * sizeof(int)));
+      FPIE_CUDA(cudaMemsetAsync(d_box, 0, kPrepAcc * sizeof(int), stream));
+    }
+    launch_prep_mask(dmsk, mh, mw, mch, m01, d_box, h_box, stream);
     post_launch(this);
-    FPIE_CUDA(cudaMemcpyAsync(hbox, dbox, sizeof(hbox), cudaMemcpyDeviceToHost, stream));
     FPIE_CUDA(cudaStreamSynchronize(stream));
+    const int hbox[4] = {h_box[0], h_box[1], h_box[2], h_box[3]};
     if (hbox[1] < 0)
       throw Error{FPIE_ERR_ARG, "the mask selects no pixel (after clearing its 1-pixel frame)"};
     const int x0 = hbox[0] - 1, x1 = hbox[1] + 2, y0 = hbox[2] - 1, y1 = hbox[3] + 2;
@@ -905,9 +909,9 @@ struct EquSolverImpl : Solver {
 
   void finish(uint8_t* img, float* err) {
     sync_from_grid();
-    equ_finish_kernel<<<nparts, 256, 0, stream>>>(E, A, b, x[cur], img ? img : d_img, d_part);
-    post_launch(this);
-    launch_finalize(d_part, nparts, err ? err : d_err, stream);
+    equ_finish_kernel<<<nparts, 256, 0, stream>>>(E, A, b, x[cur], img ? img : d_img, d_part,
+                                                 reinterpret_cast<unsigned*>(d_err + 3),
+                                                 err ? err : d_err);
     post_launch(this);
   }
 

@@ -44,11 +44,38 @@ __global__ void grid_inputs_unpack_kernel(GridGeom G, const uint8_t* __restrict_
 
 // ---- layout conversion kernels ------------------------------------------------
 
-// Whether a state value or a masked pixel's gradient lies outside the range
-// in which the resident kernel's quartered sums are exact (grid_res.cu).
+// Marks float inputs (state values anywhere, gradients of masked pixels) that
+// lie outside the range in which quartered sums are exact (quarter.cuh).
 __device__ __forceinline__ bool out_of_range(float v) { return !(fabsf(v) <= 0x1p40f); }
 __device__ __forceinline__ bool grad_out_of_range(float v) {
-  return out_of_range(v) || (v != 0.f && fabsf(v) < 0x1p-60f);
+  return out_of_range(v) || (v != 0.f && fabsf(v) < 0x1p-38f);
+}
+
+__global__ void grid_range_kernel(GridGeom G, const uint8_t* __restrict__ mask,
+                                  const float* __restrict__ x, const float* __restrict__ g,
+                                  unsigned* __restrict__ wild) {
+  const int groups = (G.m + 3) / 4;  // the padding past the last column holds zeros
+  const long long total = (long long)G.n * groups;
+  bool bad = false;
+  for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
+       idx += (long long)gridDim.x * blockDim.x) {
+    const int i = (int)(idx / groups), q = (int)(idx - (long long)i * groups);
+    const long long p = G.at(i, 4 * q);
+    const uint32_t mk = __ldg(reinterpret_cast<const uint32_t*>(mask + p));
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const float4 v = ld4(x + c * G.plane + p);
+      bad = bad || out_of_range(v.x) || out_of_range(v.y) || out_of_range(v.z) || out_of_range(v.w);
+      if (mk) {
+        const float4 u = ld4(g + c * G.plane + p);
+        bad = bad || ((mk & 0xffu) && grad_out_of_range(u.x)) ||
+              ((mk & 0xff00u) && grad_out_of_range(u.y)) ||
+              ((mk & 0xff0000u) && grad_out_of_range(u.z)) ||
+              ((mk & 0xff000000u) && grad_out_of_range(u.w));
+      }
+    }
+  }
+  if (bad) *wild = 1;
 }
 
 // An equation system that is a 4-neighbour raster stencil, on the grid:
@@ -60,8 +87,7 @@ __global__ void grid_from_equ_kernel(GridGeom G, int N, const int* __restrict__ 
                                      const float* __restrict__ xe, const float* __restrict__ be,
                                      long long np, uint8_t* __restrict__ mask,
                                      float* __restrict__ x0, float* __restrict__ x1,
-                                     float* __restrict__ g, unsigned* __restrict__ wild) {
-  bool bad = false;
+                                     float* __restrict__ g) {
   for (long long i = 1 + blockIdx.x * (long long)blockDim.x + threadIdx.x; i < N;
        i += (long long)gridDim.x * blockDim.x) {
     const int p = pos[i];
@@ -72,12 +98,9 @@ __global__ void grid_from_equ_kernel(GridGeom G, int N, const int* __restrict__ 
       const float v = xe[c * np + i];
       x0[c * G.plane + q] = v;
       x1[c * G.plane + q] = v;
-      const float b = be[c * np + i];
-      g[c * G.plane + q] = b;
-      bad = bad || out_of_range(v) || grad_out_of_range(b);
+      g[c * G.plane + q] = be[c * np + i];
     }
   }
-  if (bad) *wild = 1;
 }
 
 // The unknowns' state back into planar X (row 0 untouched).
@@ -98,26 +121,21 @@ __global__ void grid_pack_kernel(GridGeom G, const int32_t* __restrict__ mk,
                                  const float* __restrict__ gr,
                                  uint8_t* __restrict__ mask,
                                  float* __restrict__ x0, float* __restrict__ x1,
-                                 float* __restrict__ g, unsigned* __restrict__ wild) {
+                                 float* __restrict__ g) {
   const long long total = (long long)G.n * G.m;
-  bool bad = false;
   for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
        idx < total; idx += (long long)gridDim.x * blockDim.x) {
     const int i = (int)(idx / G.m), j = (int)(idx % G.m);
     const long long p = G.at(i, j);
-    const bool on = mk[idx] != 0;
-    mask[p] = on;
+    mask[p] = mk[idx] != 0;
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
       const float v = t[idx * 3 + c];
       x0[c * G.plane + p] = v;
       x1[c * G.plane + p] = v;
-      const float b = gr[idx * 3 + c];
-      g[c * G.plane + p] = b;
-      bad = bad || out_of_range(v) || (on && grad_out_of_range(b));
+      g[c * G.plane + p] = gr[idx * 3 + c];
     }
   }
-  if (bad) *wild = 1;
 }
 
 __global__ void grid_unpack_kernel(GridGeom G, const float* __restrict__ x,
@@ -150,6 +168,7 @@ struct GridSolverImpl : Solver {
   float* d_err = nullptr;
   float* h_err = nullptr;
   int* h_box = nullptr;  // pinned, for the GPU-side reset's bounding box
+  int* d_box = nullptr;  // its accumulators
   GridLaunch L{};
   static constexpr int kChunk = 64;  // sweeps per captured graph (even)
   cudaGraphExec_t chunk[2] = {nullptr, nullptr};
@@ -157,8 +176,8 @@ struct GridSolverImpl : Solver {
   // Bounded device waits (the flow kernel's neighbourhood waits, the TMA
   // kernel's copy waits) give up after spin_limit rounds and set d_wait_err.
   long long spin_limit = 1LL << 26;  // x ~64 ns sleeps: a few seconds at most
-  int* d_wait_err = nullptr;
-  int* h_wait_err = nullptr;  // pinned
+  int* d_wait_err = nullptr;  // in d_err
+  bool waits = false;         // a launch that may set it was queued
 
   // ---- persistent TMA-prefetch kernel (variant index kTma; by name only) -----
   static constexpr int kTma = -3;
@@ -200,8 +219,9 @@ struct GridSolverImpl : Solver {
   ResShape res{0, 0, 0, 0};        // this geometry's shape; rows == 0: none
   std::string res_pin;          // pinned by name ("" otherwise)
   void* res_exchange = nullptr; // packets and activity words
-  unsigned* res_ctl = nullptr;  // epoch base, exit count; then the range mark
+  unsigned* res_ctl = nullptr;  // epoch base, exit count; range mark; finish count (in d_err)
   unsigned* wild() const { return res_ctl + kResCtl; }
+  unsigned* finish_count() const { return res_ctl + kResCtl + 1; }
   bool maybe_wild = false;      // the range mark may be set
 
   bool use_res() const {
@@ -214,11 +234,19 @@ struct GridSolverImpl : Solver {
       FPIE_CUDA(cudaMalloc(&res_exchange, b));
       FPIE_CUDA(cudaMemsetAsync(res_exchange, 0, b, stream));
     }
-    ensure_wait_flag();
+    waits = true;
     launch_res(G, res, mask, g, x[cur], x[cur ^ 1], res_exchange, res_ctl, wild(), iters,
                d_wait_err, spin_limit, stream);
     post_launch(this);
     cur ^= 1;
+  }
+
+  // After a reset from floats (uint8 images are always in range).
+  void check_range() {
+    grid_range_kernel<<<conv_blocks((long long)G.n * ((G.m + 3) / 4)), 256, 0, stream>>>(
+        G, mask, x[0], g, wild());
+    post_launch(this);
+    maybe_wild = true;
   }
 
   // Before a reset writes the planes: no value seen out of range yet.
@@ -231,15 +259,19 @@ struct GridSolverImpl : Solver {
   // or a TMA copy wait that gave up); call after the stream has been
   // synchronised.
   void check_waits() {
-    if (!d_wait_err) return;
-    FPIE_CUDA(cudaMemcpyAsync(h_wait_err, d_wait_err, sizeof(int), cudaMemcpyDeviceToHost, stream));
+    if (!d_wait_err || !waits) return;
+    FPIE_CUDA(cudaMemcpyAsync(h_err + 3, d_wait_err, sizeof(int), cudaMemcpyDeviceToHost, stream));
     FPIE_CUDA(cudaStreamSynchronize(stream));
-    if (*h_wait_err) {
-      *h_wait_err = 0;
-      FPIE_CUDA(cudaMemsetAsync(d_wait_err, 0, sizeof(int), stream));
-      FPIE_CUDA(cudaStreamSynchronize(stream));
-      throw Error{FPIE_ERR_TIMEOUT, "sweep kernel: a bounded device wait gave up"};
-    }
+    raise_waits();
+  }
+  // The flag as h_err[3] holds it.
+  void raise_waits() {
+    int flag;
+    std::memcpy(&flag, h_err + 3, sizeof flag);
+    if (!flag) return;
+    FPIE_CUDA(cudaMemsetAsync(d_wait_err, 0, sizeof(int), stream));
+    FPIE_CUDA(cudaStreamSynchronize(stream));
+    throw Error{FPIE_ERR_TIMEOUT, "sweep kernel: a bounded device wait gave up"};
   }
   void check_async() override { check_waits(); }
 
@@ -248,6 +280,7 @@ struct GridSolverImpl : Solver {
   void run_flow(int iters) {
     ensure_flow_tables();
     FPIE_CUDA(cudaMemsetAsync(flow_done, 0, (size_t)ft_tiles * 3 * sizeof(int), stream));
+    waits = true;
     launch_flow(G, mask, code, g, x[0], x[1], cur, ft_list, flow_rec, flow_done, ft_tiles_x,
                 ft_tiles, iters, d_wait_err, spin_limit, flow_grid, stream, red_black, ft_k,
                 flow_pin());
@@ -263,6 +296,7 @@ struct GridSolverImpl : Solver {
     ensure_mixed();
     ensure_flow_tables();
     FPIE_CUDA(cudaMemsetAsync(flow_done, 0, (size_t)ft_tiles * 3 * sizeof(int), stream));
+    waits = true;
     launch_flow_mixed(G, mask, g, x[0], x[1], cur, precision == FPIE_MIXED_BF16, e[0], e[1], r,
                       ft_list, flow_rec, flow_done, ft_tiles_x, ft_tiles, iters, d_wait_err,
                       spin_limit, flow_grid, stream);
@@ -291,7 +325,7 @@ struct GridSolverImpl : Solver {
     FPIE_CUDA(cudaGetDevice(&device));
     FPIE_CUDA(cudaStreamCreateWithFlags(&own_stream, cudaStreamNonBlocking));
     stream = own_stream;
-    FPIE_CUDA(cudaMallocHost(&h_err, 3 * sizeof(float)));
+    FPIE_CUDA(cudaMallocHost(&h_err, 4 * sizeof(float)));
   }
 
   ~GridSolverImpl() override {
@@ -299,6 +333,7 @@ struct GridSolverImpl : Solver {
     if (h_err) cudaFreeHost(h_err);
     if (h_norm) cudaFreeHost(h_norm);
     if (h_box) cudaFreeHost(h_box);
+    cudaFree(d_box);
     if (own_stream) cudaStreamDestroy(own_stream);
   }
 
@@ -345,10 +380,8 @@ struct GridSolverImpl : Solver {
     flags_cap = 0;
     flags_ok = false;
     release_mixed();
-    cudaFree(d_wait_err);
     cudaFree(tma_list);
     cudaFree(res_exchange);
-    cudaFree(res_ctl);
     res_exchange = nullptr;
     res_ctl = nullptr;
     cudaFree(flow_inv);
@@ -363,9 +396,7 @@ struct GridSolverImpl : Solver {
     ft_list = nullptr;
     flow_cap = 0;
     ft_ok = false;
-    if (h_wait_err) cudaFreeHost(h_wait_err);
     d_wait_err = nullptr;
-    h_wait_err = nullptr;
     tma_list = nullptr;
     tma_list_cap = 0;
     x[0] = x[1] = g = nullptr;
@@ -406,9 +437,12 @@ struct GridSolverImpl : Solver {
     FPIE_CUDA(cudaMalloc(&code, (size_t)G.plane));
     FPIE_CUDA(cudaMalloc(&d_img, (size_t)n * m * 3));
     FPIE_CUDA(cudaMalloc(&d_part, (size_t)L.nparts * 3 * sizeof(double)));
-    FPIE_CUDA(cudaMalloc(&d_err, 3 * sizeof(float)));
-    FPIE_CUDA(cudaMalloc(&res_ctl, (kResCtl + 1) * sizeof(unsigned)));
-    FPIE_CUDA(cudaMemsetAsync(res_ctl, 0, (kResCtl + 1) * sizeof(unsigned), stream));
+    // One set of control words: err and the wait flag (read back together),
+    // the resident kernel's, the range mark, the finish kernel's count.
+    FPIE_CUDA(cudaMalloc(&d_err, (4 + kResCtl + 2) * sizeof(unsigned)));
+    FPIE_CUDA(cudaMemsetAsync(d_err, 0, (4 + kResCtl + 2) * sizeof(unsigned), stream));
+    d_wait_err = reinterpret_cast<int*>(d_err + 3);
+    res_ctl = reinterpret_cast<unsigned*>(d_err + 4);
     maybe_wild = false;
     res = res_pin.empty() ? res_pick(n, m) : res_named(res_pin.c_str(), n, m);
     FPIE_CUDA(cudaMemsetAsync(x[0], 0, 3 * pb, stream));
@@ -421,9 +455,9 @@ struct GridSolverImpl : Solver {
   void pack(const int32_t* dmask, const float* dtgt, const float* dgrad) {
     const long long total = (long long)G.n * G.m;
     grid_pack_kernel<<<conv_blocks(total), 256, 0, stream>>>(
-        G, dmask, dtgt, dgrad, mask, x[0], x[1], g, wild());
+        G, dmask, dtgt, dgrad, mask, x[0], x[1], g);
     post_launch(this);
-    maybe_wild = true;
+    check_range();
     ready = true;
   }
 
@@ -461,9 +495,9 @@ struct GridSolverImpl : Solver {
     FPIE_CUDA(cudaMemsetAsync(mask, 0, (size_t)G.plane, stream));
     if (N > 1) {
       grid_from_equ_kernel<<<conv_blocks(N), 256, 0, stream>>>(G, N, pos, xe, be, np, mask, x[0],
-                                                               x[1], g, wild());
+                                                               x[1], g);
       post_launch(this);
-      maybe_wild = true;
+      check_range();
     }
     ready = true;
   }
@@ -497,29 +531,27 @@ struct GridSolverImpl : Solver {
                  "gradient mode must be 0 (src), 1 (avg), 2 (max)");
     const size_t sb = (size_t)sh * sw * 3, mb = (size_t)mh * mw * mch, tb = (size_t)th * tw * 3;
     const size_t mpx = (size_t)mh * mw;
-    const size_t head = on_device ? 0 : (sb + mb + tb + 15) / 16 * 16;
-    AsyncScratch scratch(head + 16 + mpx, stream);
+    const size_t ms = (sb + 15) / 16 * 16, ts = ms + (mb + 15) / 16 * 16;  // staged mask, target
+    const size_t head = on_device ? 0 : ts + (tb + 15) / 16 * 16;
+    AsyncScratch scratch(head + mpx, stream);
     char* stage = scratch.bytes();
     const uint8_t *dsrc = src, *dmsk = msk, *dtgt = tgt;
     if (!on_device) {
       FPIE_CUDA(cudaMemcpyAsync(stage, src, sb, cudaMemcpyHostToDevice, stream));
-      FPIE_CUDA(cudaMemcpyAsync(stage + sb, msk, mb, cudaMemcpyHostToDevice, stream));
-      FPIE_CUDA(cudaMemcpyAsync(stage + sb + mb, tgt, tb, cudaMemcpyHostToDevice, stream));
+      FPIE_CUDA(cudaMemcpyAsync(stage + ms, msk, mb, cudaMemcpyHostToDevice, stream));
+      FPIE_CUDA(cudaMemcpyAsync(stage + ts, tgt, tb, cudaMemcpyHostToDevice, stream));
       dsrc = reinterpret_cast<uint8_t*>(stage);
-      dmsk = reinterpret_cast<uint8_t*>(stage + sb);
-      dtgt = reinterpret_cast<uint8_t*>(stage + sb + mb);
+      dmsk = reinterpret_cast<uint8_t*>(stage + ms);
+      dtgt = reinterpret_cast<uint8_t*>(stage + ts);
     }
-    int* dbox = reinterpret_cast<int*>(stage + head);
-    uint8_t* m01 = reinterpret_cast<uint8_t*>(stage + head + 16);
+    uint8_t* m01 = reinterpret_cast<uint8_t*>(stage + head);
     if (!h_box) FPIE_CUDA(cudaMallocHost(&h_box, 4 * sizeof(int)));
-    h_box[0] = INT32_MAX;
-    h_box[1] = -1;
-    h_box[2] = INT32_MAX;
-    h_box[3] = -1;
-    FPIE_CUDA(cudaMemcpyAsync(dbox, h_box, 4 * sizeof(int), cudaMemcpyHostToDevice, stream));
-    launch_prep_mask(dmsk, mh, mw, mch, m01, dbox, stream);
+    if (!d_box) {
+      FPIE_CUDA(cudaMalloc(&d_box, kPrepAcc * sizeof(int)));
+      FPIE_CUDA(cudaMemsetAsync(d_box, 0, kPrepAcc * sizeof(int), stream));
+    }
+    launch_prep_mask(dmsk, mh, mw, mch, m01, d_box, h_box, stream);
     post_launch(this);
-    FPIE_CUDA(cudaMemcpyAsync(h_box, dbox, 4 * sizeof(int), cudaMemcpyDeviceToHost, stream));
     FPIE_CUDA(cudaStreamSynchronize(stream));
     const int b0 = h_box[0], b1 = h_box[1], b2 = h_box[2], b3 = h_box[3];
     if (b1 < 0)
@@ -608,8 +640,7 @@ struct GridSolverImpl : Solver {
     if (listed) {
       prepare_tma();
       tma_grid = tma_ctas(tiles * 3);
-      ensure_wait_flag();
-      if (tiles + 1 > tma_list_cap) {
+        if (tiles + 1 > tma_list_cap) {
         cudaFree(tma_list);
         tma_list = nullptr;
         FPIE_CUDA(cudaMalloc(&tma_list, (size_t)(tiles + 1) * sizeof(int)));
@@ -625,14 +656,6 @@ struct GridSolverImpl : Solver {
       post_launch(this);
     }
     flags_ok = true;
-  }
-
-  void ensure_wait_flag() {
-    if (d_wait_err) return;
-    FPIE_CUDA(cudaMalloc(&d_wait_err, sizeof(int)));
-    FPIE_CUDA(cudaMallocHost(&h_wait_err, sizeof(int)));
-    *h_wait_err = 0;
-    FPIE_CUDA(cudaMemsetAsync(d_wait_err, 0, sizeof(int), stream));
   }
 
   // Flags, active-tile list, records and counters of the flow tiling.
@@ -659,7 +682,6 @@ struct GridSolverImpl : Solver {
       flow_cap = ft_tiles;
     }
     flow_grid = flow_ctas();
-    ensure_wait_flag();
     launch_tile_flags(G, mask, th, tw, kd, ft_tiles_x, ft_tiles, ft_flags, stream);
     post_launch(this);
     launch_tma_list(ft_flags, ft_tiles, ft_list, stream);
@@ -703,6 +725,7 @@ struct GridSolverImpl : Solver {
   // k sweeps (k <= depth()) from buffer `from`; flips nothing (caller does).
   void launch_block(cudaStream_t st, int from, int k) {
     if (variant == kTma) {
+      waits = true;
       launch_tma(G, mask, g, x[from], x[from ^ 1], flags, tma_list, tiles_x, tiles, k, d_wait_err,
                  spin_limit, tma_grid, st);
     } else if (variant < 0) {
@@ -1202,9 +1225,8 @@ struct GridSolverImpl : Solver {
   }
 
   void finish(uint8_t* img, float* err) {
-    launch_grid_finish(L, G, mask, g, x[cur], img ? img : d_img, d_part, stream);
-    post_launch(this);
-    launch_finalize(d_part, L.nparts, err ? err : d_err, stream);
+    launch_grid_finish(L, G, mask, g, x[cur], img ? img : d_img, d_part, finish_count(),
+                       err ? err : d_err, stream);
     post_launch(this);
   }
 
@@ -1220,9 +1242,10 @@ struct GridSolverImpl : Solver {
     // Straight into the caller's (pageable) array: measured on GB300 5x
     // faster than a pinned staging buffer plus a host copy.
     FPIE_CUDA(cudaMemcpyAsync(img_out, d_img, bytes, cudaMemcpyDeviceToHost, stream));
-    FPIE_CUDA(cudaMemcpyAsync(h_err, d_err, 3 * sizeof(float), cudaMemcpyDeviceToHost, stream));
+    // err and the wait flag behind it, in one copy.
+    FPIE_CUDA(cudaMemcpyAsync(h_err, d_err, 4 * sizeof(float), cudaMemcpyDeviceToHost, stream));
     FPIE_CUDA(cudaStreamSynchronize(stream));
-    check_waits();
+    raise_waits();
     std::memcpy(err_out, h_err, 3 * sizeof(float));
   }
 

@@ -8,6 +8,7 @@ namespace fpie {
 struct GridLaunch {
   dim3 sweep_block, sweep_grid;    // one-sweep kernel
   dim3 finish_block, finish_grid;  // residual + image kernel
+  int finish_rows;                 // rows per thread of the latter
   int nparts;                      // residual partials (finish blocks)
 };
 
@@ -18,10 +19,12 @@ void launch_grid_sweep(const GridLaunch& L, const GridGeom& G,
                        const uint8_t* mask, const float* g, const float* xin,
                        float* xout, cudaStream_t st);
 
-// Residual partials (|r| summed per block, double) and the clipped uint8
-// image in the reference's interleaved [n][m][3] layout.
+// The residual sums (err[3]; parts: nparts x 3 doubles of scratch, count: a
+// device word that is 0 between launches) and the clipped uint8 image in the
+// reference's interleaved [n][m][3] layout.
 void launch_grid_finish(const GridLaunch& L, const GridGeom& G,
                         const uint8_t* mask, const float* g, const float* x,
-                        uint8_t* img, double* parts, cudaStream_t st);
+                        uint8_t* img, double* parts, unsigned* count, float* err,
+                        cudaStream_t st);
 
 }  // namespace fpie

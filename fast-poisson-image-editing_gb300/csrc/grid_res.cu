@@ -9,28 +9,9 @@
 // regions are cut as small as lets every SM hold one.  Per sweep: 194x194
 // 0.295 us (0.71 before), 251x389 0.403 (0.83), 176x1457 0.564 (0.83).
 //
-// Update.  A pixel's next value is ((((g + up) + down) + left) + right) / 4
-// in the numpy order.  Scaling by 1/4 commutes with rounding, so with g' =
-// g / 4 it is fma(right, 1/4, fma(left, 1/4, fma(down, 1/4, fma(up, 1/4,
-// g')))): the same bits in four FFMAs instead of four additions and a
-// multiplication.  An unmasked pixel keeps its value by one maximum instead
-// of a select on mask bits: its g' is -inf, so the sum is -inf, and L, the
-// value to keep, wins; a masked pixel's L is a NaN, which a maximum ignores.
-// (Measured per 128x128 region and sweep: 900 cycles; the packed FADD2 sweep
-// with selects 1,220, without any 725.  A packed FADD2 takes two issue slots,
-// so pairing rows gains nothing and costs register moves.)
-//
-// Where the scaling is exact.  A quartered partial sum is inexact only below
-// 2^-126, an unquartered one overflows only above 2^127, and -inf + inf is no
-// number.  So: (1) a reset marks inputs that are not finite, above 2^40, or
-// (gradients) nonzero below 2^-60 (`wild`); with them, the whole launch takes
-// the reference's order of operations (slow_sweep).  Bounded inputs stay
-// bounded: a sweep adds at most max|g| / 4.  (2) Every 16 sweeps each CTA
-// checks its region for nonzero values below 2^-60.  Without any, all values
-// are multiples of 2^-83, and every sweep makes that at most four times
-// finer, so for the next 16 sweeps partial sums are multiples of 2^-117 and
-// exact.  A CTA that finds one takes slow sweeps until its next check and
-// marks the packets it sends; a CTA that receives a marked packet does the
+// The update is quarter.cuh's.  Each CTA looks for values below 2^-60 every
+// 16 sweeps; one that finds some takes slow sweeps until its next look and
+// marks the packets it sends, and a CTA that receives a marked packet does the
 // same.
 //
 // Exchange.  A packet is 8 bytes {value, epoch} in one 64-bit store, two per
@@ -54,6 +35,7 @@
 
 #include "common.cuh"
 #include "grid_res.cuh"
+#include "quarter.cuh"
 
 namespace fpie {
 
@@ -76,8 +58,7 @@ struct ResArgs {
 };
 
 constexpr int kCheck = 16;            // sweeps between range checks
-constexpr unsigned kTiny = 0x21800000u;  // 2^-60
-constexpr unsigned kMasked = 0x7fffffffu;  // L of a masked pixel (a NaN)
+constexpr int kTiny = 60;     // and their limit, 2^-60: exact for 16 sweeps (quarter.cuh)
 
 __device__ __forceinline__ void st_packets(unsigned long long* p, float a, float b, unsigned e) {
   const unsigned long long hi = (unsigned long long)e << 32;
@@ -94,78 +75,6 @@ __device__ __forceinline__ ulonglong2 ld_packets(const unsigned long long* p) {
                : "l"(p)
                : "memory");
   return v;
-}
-
-// One in-place sweep of the strip P (R rows x 4 columns per thread, region rows
-// w * R on; a strip is LW lanes, half a warp where LW = 16), edge rows through shared memory, columns by shuffles.  FWD visits
-// rows downwards, !FWD upwards, each keeping the old row it just replaced: a
-// forward and a backward sweep leave every row in its registers.
-template <int R, int NS, int LW, bool FWD>
-__device__ __forceinline__ void res_sweep(float (&P)[R][4], const float (&Gq)[R][4],
-                                          const float (&L)[R][4], int par, int lane, int w,
-                                          float4 (&edge)[2][2][NS][LW]) {
-  edge[par][0][w][lane] = make_float4(P[0][0], P[0][1], P[0][2], P[0][3]);
-  edge[par][1][w][lane] = make_float4(P[R - 1][0], P[R - 1][1], P[R - 1][2], P[R - 1][3]);
-  __syncthreads();
-  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-  const float4 a4 = w > 0 ? edge[par][1][w - 1][lane] : zero;
-  const float4 b4 = w < NS - 1 ? edge[par][0][w + 1][lane] : zero;
-  const float a[4] = {a4.x, a4.y, a4.z, a4.w}, b[4] = {b4.x, b4.y, b4.z, b4.w};
-  float keep[4];
-#pragma unroll
-  for (int j = 0; j < 4; ++j) keep[j] = FWD ? a[j] : b[j];
-#pragma unroll
-  for (int q = 0; q < R; ++q) {
-    const int i = FWD ? q : R - 1 - q;
-    const float cur[4] = {P[i][0], P[i][1], P[i][2], P[i][3]};
-    const float lf = __shfl_up_sync(0xffffffffu, cur[3], 1, LW);
-    const float rt = __shfl_down_sync(0xffffffffu, cur[0], 1, LW);
-    float t[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-      t[j] = __fmaf_rn(FWD ? keep[j] : (i > 0 ? P[i > 0 ? i - 1 : 0][j] : a[j]), 0.25f, Gq[i][j]);
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-      t[j] = __fmaf_rn(FWD ? (i < R - 1 ? P[i < R - 1 ? i + 1 : i][j] : b[j]) : keep[j], 0.25f, t[j]);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) t[j] = __fmaf_rn(j > 0 ? cur[j > 0 ? j - 1 : 0] : lf, 0.25f, t[j]);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      keep[j] = cur[j];
-      P[i][j] = fmaxf(__fmaf_rn(j < 3 ? cur[j < 3 ? j + 1 : 0] : rt, 0.25f, t[j]), L[i][j]);
-    }
-  }
-}
-
-// The same sweep in the reference's order of operations, for values outside
-// the quartered form's range.  gs: 4, or 1 where Gq is not quartered.
-template <int R, int NS, int LW>
-__device__ __forceinline__ void slow_sweep(float (&P)[R][4], const float (&Gq)[R][4],
-                                           const float (&L)[R][4], float gs, int lane, int w,
-                                           float4 (&edge)[2][2][NS][LW]) {
-  edge[0][0][w][lane] = make_float4(P[0][0], P[0][1], P[0][2], P[0][3]);
-  edge[0][1][w][lane] = make_float4(P[R - 1][0], P[R - 1][1], P[R - 1][2], P[R - 1][3]);
-  __syncthreads();
-  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-  const float4 a4 = w > 0 ? edge[0][1][w - 1][lane] : zero;
-  const float4 b4 = w < NS - 1 ? edge[0][0][w + 1][lane] : zero;
-  const float b[4] = {b4.x, b4.y, b4.z, b4.w};
-  float keep[4] = {a4.x, a4.y, a4.z, a4.w};
-#pragma unroll
-  for (int i = 0; i < R; ++i) {
-    const float cur[4] = {P[i][0], P[i][1], P[i][2], P[i][3]};
-    const float lf = __shfl_up_sync(0xffffffffu, cur[3], 1, LW);
-    const float rt = __shfl_down_sync(0xffffffffu, cur[0], 1, LW);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const float o = jacobi5(__fmul_rn(Gq[i][j], gs), keep[j],
-                              i < R - 1 ? P[i < R - 1 ? i + 1 : i][j] : b[j],
-                              j > 0 ? cur[j > 0 ? j - 1 : 0] : lf, j < 3 ? cur[j < 3 ? j + 1 : 0] : rt);
-      keep[j] = cur[j];
-      if (__float_as_uint(L[i][j]) == kMasked) P[i][j] = o;
-    }
-  }
-  __syncthreads();  // the edge rows are read before the next sweep writes them
 }
 
 // The thread index, read anew: what is computed from it does not stay in
@@ -249,7 +158,7 @@ __global__ void __launch_bounds__(W * 32, 1) grid_res_kernel(ResArgs A) {
       const bool on = (mk >> (8 * j)) & 0xffu;
       P[i][j] = x[j];
       L[i][j] = on ? __uint_as_float(kMasked) : x[j] == x[j] ? x[j] : __uint_as_float(0x7fc00000u);
-      Gq[i][j] = on ? (wild ? gv[j] : __fmul_rn(gv[j], 0.25f)) : __uint_as_float(0xff800000u);
+      Gq[i][j] = on ? (wild ? gv[j] : __fmul_rn(gv[j], 0.25f)) : __uint_as_float(kNegInf);
     }
     // Apron pixels nobody sends keep these values.
     if (r < K || r >= H - K || !core_lane) *reinterpret_cast<float4*>(halo + r * WD + 4 * lane) = x4;
@@ -379,12 +288,12 @@ __global__ void __launch_bounds__(W * 32, 1) grid_res_kernel(ResArgs A) {
         }
       }
       if (done % kCheck == 0) {
-        unsigned least = 0xffffffffu;  // of 2 * |bits| - 1: zeros wrap to the top
+        unsigned least = 0xffffffffu;
 #pragma unroll
         for (int i = 0; i < R; ++i)
 #pragma unroll
-          for (int j = 0; j < 4; ++j) least = min(least, 2u * __float_as_uint(P[i][j]) - 1u);
-        const bool tiny = __syncthreads_or(least < 2u * kTiny - 1u);
+          for (int j = 0; j < 4; ++j) least = min(least, tiny_key(P[i][j]));
+        const bool tiny = __syncthreads_or(least < tiny_limit(kTiny));
         slow = tiny || s_wild || (A.tiles > 1 && slow);
       }
       const int ks = min(A.period, A.sweeps - done);
@@ -392,13 +301,16 @@ __global__ void __launch_bounds__(W * 32, 1) grid_res_kernel(ResArgs A) {
       if (!slow) {
 #pragma unroll 1
         for (; s + 2 <= ks; s += 2) {
-          res_sweep<R, NS, LW, true>(P, Gq, L, 0, lane, w, edge);
-          res_sweep<R, NS, LW, false>(P, Gq, L, 1, lane, w, edge);
+          quarter_sweep<R, NS, LW, false, true>(P, Gq, L, 0, lane, w, edge);
+          quarter_sweep<R, NS, LW, false, false>(P, Gq, L, 1, lane, w, edge);
         }
       }
       // An odd last sweep takes this path too (the same values).
 #pragma unroll 1
-      for (; s < ks; ++s) slow_sweep<R, NS, LW>(P, Gq, L, s_wild ? 1.f : 4.f, lane, w, edge);
+      for (; s < ks; ++s)
+        slow_sweep<R, NS, LW>(
+            P, Gq, [&](int i, int j) { return __float_as_uint(L[i][j]) == kMasked; },
+            s_wild ? 1.f : 4.f, lane, w, edge);
     }
     const int tid = fresh_tid(), ln = tid % LW, st = tid / LW;
     if (ln >= KL && ln < LW - KL) {

@@ -19,11 +19,13 @@ struct PrepArgs {
 };
 
 // Thresholds the mask (3 channels: channel sum >= 384; 1 channel: >= 128),
-// clears its 1-pixel frame into m01 and folds the set pixels' bounding box
-// into box = {row min, row max, col min, col max} (atomics; box must hold
-// {INT_MAX, -1, INT_MAX, -1} before).
-void launch_prep_mask(const uint8_t* mask, int mh, int mw, int mch, uint8_t* m01, int* box,
-                      cudaStream_t st);
+// clears its 1-pixel frame into m01 (16-byte aligned) and writes the set
+// pixels' bounding box to box = {row min, row max, col min, col max} (pinned
+// host memory or device memory; row max -1 where none is set).  acc:
+// kPrepAcc device words, 0 before the first call and after every call.
+constexpr int kPrepAcc = 5;
+void launch_prep_mask(const uint8_t* mask, int mh, int mw, int mch, uint8_t* m01, int* acc,
+                      int* box, cudaStream_t st);
 // Writes mask, both state buffers and grad of the crop in the planar padded
 // layout (interior only: the halo keeps what it holds).
 void launch_prep_grid(const PrepArgs& a, uint8_t* mask, float* xa, float* xb, float* g,

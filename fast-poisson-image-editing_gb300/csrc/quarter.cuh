@@ -1,0 +1,116 @@
+// The quartered Jacobi sweep on register-resident strips, shared by the
+// resident kernel (grid_res.cu) and the pipelined one (grid_pipe.cu).
+//
+// A pixel's next value is ((((g + up) + down) + left) + right) / 4 in the
+// numpy order.  Scaling by 1/4 commutes with rounding, so with g' = g / 4 it
+// is fma(right, 1/4, fma(left, 1/4, fma(down, 1/4, fma(up, 1/4, g')))): the
+// same bits in four FFMAs instead of four additions and a multiplication.  An
+// unmasked pixel keeps its value by one maximum instead of a select on mask
+// bits: its g' is -inf, so the sum is -inf, and L, the value to keep, wins; a
+// masked pixel's L is a NaN, which a maximum ignores.  (Measured per 128x128
+// region and sweep, 8 warps: 690 cycles fully masked, 830-900 with the
+// maximum; the packed FADD2 sweep 725, with its selects 1,220.  A packed FADD2
+// takes two issue slots, so pairing rows gains nothing and costs register
+// moves; a multiplier register per pixel instead of the maximum, 880.)
+//
+// Where the scaling is exact.  A quartered partial sum is inexact only below
+// 2^-126, an unquartered one overflows only above 2^127, and -inf + inf is no
+// number.  The kernels therefore
+//  (1) read a mark (`wild`) that a reset sets for inputs that are not finite,
+//      above 2^40, or (gradients) nonzero below 2^-38, and with it take
+//      slow_sweep, the reference's order of operations, throughout.  Bounded
+//      inputs stay bounded: a sweep adds at most max|g| / 4.
+//  (2) look for nonzero values below a limit every few sweeps, and take slow
+//      sweeps where there are any.  Without any below 2^-e, and with the
+//      gradient's 2^-38, all values are multiples of 2^-(max(e, 38) + 23);
+//      every sweep makes that at most four times finer, so for n sweeps
+//      partial sums are multiples of 2^-(max(e, 38) + 23 + 2n), exact while
+//      that is at least 2^-126.
+#pragma once
+
+#include "common.cuh"
+
+namespace fpie {
+
+constexpr unsigned kMasked = 0x7fffffffu;   // L of a masked pixel (a NaN)
+constexpr unsigned kNegInf = 0xff800000u;   // g' of an unmasked pixel
+
+// 2 * |bits| - 1 of v, so that zeros wrap to the top: compare with tiny_limit.
+__device__ __forceinline__ unsigned tiny_key(float v) { return 2u * __float_as_uint(v) - 1u; }
+constexpr unsigned tiny_limit(int e) { return 2u * ((127u - e) << 23) - 1u; }  // of 2^-e
+
+// One in-place sweep of the strip P (R rows x 4 columns per thread, region rows
+// w * R on; a strip is LW lanes, half a warp where LW = 16), edge rows through shared memory, columns by shuffles.  FWD visits
+// rows downwards, !FWD upwards, each keeping the old row it just replaced: a
+// forward and a backward sweep leave every row in its registers.
+template <int R, int NS, int LW, bool FULL, bool FWD>
+__device__ __forceinline__ void quarter_sweep(float (&P)[R][4], const float (&Gq)[R][4],
+                                          const float (&L)[FULL ? 1 : R][4], int par, int lane, int w,
+                                          float4 (&edge)[2][2][NS][LW]) {
+  edge[par][0][w][lane] = make_float4(P[0][0], P[0][1], P[0][2], P[0][3]);
+  edge[par][1][w][lane] = make_float4(P[R - 1][0], P[R - 1][1], P[R - 1][2], P[R - 1][3]);
+  __syncthreads();
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  const float4 a4 = w > 0 ? edge[par][1][w - 1][lane] : zero;
+  const float4 b4 = w < NS - 1 ? edge[par][0][w + 1][lane] : zero;
+  const float a[4] = {a4.x, a4.y, a4.z, a4.w}, b[4] = {b4.x, b4.y, b4.z, b4.w};
+  float keep[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) keep[j] = FWD ? a[j] : b[j];
+#pragma unroll
+  for (int q = 0; q < R; ++q) {
+    const int i = FWD ? q : R - 1 - q;
+    const float cur[4] = {P[i][0], P[i][1], P[i][2], P[i][3]};
+    const float lf = __shfl_up_sync(0xffffffffu, cur[3], 1, LW);
+    const float rt = __shfl_down_sync(0xffffffffu, cur[0], 1, LW);
+    float t[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      t[j] = __fmaf_rn(FWD ? keep[j] : (i > 0 ? P[i > 0 ? i - 1 : 0][j] : a[j]), 0.25f, Gq[i][j]);
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      t[j] = __fmaf_rn(FWD ? (i < R - 1 ? P[i < R - 1 ? i + 1 : i][j] : b[j]) : keep[j], 0.25f, t[j]);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) t[j] = __fmaf_rn(j > 0 ? cur[j > 0 ? j - 1 : 0] : lf, 0.25f, t[j]);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      keep[j] = cur[j];
+      const float o = __fmaf_rn(j < 3 ? cur[j < 3 ? j + 1 : 0] : rt, 0.25f, t[j]);
+      P[i][j] = FULL ? o : fmaxf(o, L[FULL ? 0 : i][j]);
+    }
+  }
+}
+
+// The same sweep in the reference's order of operations, for values outside
+// the quartered form's range: gs * G is the gradient (gs 4, or 1 where G is
+// not quartered), `on(i, j)` tells the masked pixels.
+template <int R, int NS, int LW, typename On>
+__device__ __forceinline__ void slow_sweep(float (&P)[R][4], const float (&G)[R][4], On on,
+                                           float gs, int lane, int w,
+                                           float4 (&edge)[2][2][NS][LW]) {
+  edge[0][0][w][lane] = make_float4(P[0][0], P[0][1], P[0][2], P[0][3]);
+  edge[0][1][w][lane] = make_float4(P[R - 1][0], P[R - 1][1], P[R - 1][2], P[R - 1][3]);
+  __syncthreads();
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  const float4 a4 = w > 0 ? edge[0][1][w - 1][lane] : zero;
+  const float4 b4 = w < NS - 1 ? edge[0][0][w + 1][lane] : zero;
+  const float b[4] = {b4.x, b4.y, b4.z, b4.w};
+  float keep[4] = {a4.x, a4.y, a4.z, a4.w};
+#pragma unroll
+  for (int i = 0; i < R; ++i) {
+    const float cur[4] = {P[i][0], P[i][1], P[i][2], P[i][3]};
+    const float lf = __shfl_up_sync(0xffffffffu, cur[3], 1, LW);
+    const float rt = __shfl_down_sync(0xffffffffu, cur[0], 1, LW);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float o = jacobi5(__fmul_rn(G[i][j], gs), keep[j],
+                              i < R - 1 ? P[i < R - 1 ? i + 1 : i][j] : b[j],
+                              j > 0 ? cur[j > 0 ? j - 1 : 0] : lf, j < 3 ? cur[j < 3 ? j + 1 : 0] : rt);
+      keep[j] = cur[j];
+      if (on(i, j)) P[i][j] = o;
+    }
+  }
+  __syncthreads();  // the edge rows are read before the next sweep writes them
+}
+
+}  // namespace fpie

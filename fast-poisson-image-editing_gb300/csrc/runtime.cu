@@ -54,6 +54,14 @@ int stride_blocks(long long total, int threads, int per_sm) {
   return (int)std::max<long long>(1, std::min<long long>(want, (long long)n * per_sm));
 }
 
+int rows_per_thread(const GridGeom& g) {
+  const long long groups = (long long)g.n * ((g.m + 3) / 4);
+  const long long threads = (long long)stride_blocks(1LL << 40, 256, 8) * 256;  // 8 blocks per SM
+  int r = 1;
+  while (r < 8 && groups > threads * 2 * r) r *= 2;
+  return r;
+}
+
 cudaMemPool_t scratch_pool() {
   static std::mutex mu;
   static cudaMemPool_t pools[64] = {};
