@@ -326,7 +326,7 @@ struct BatchJob {
   uint8_t* mask = nullptr;
   uint8_t* img = nullptr;
   double* parts = nullptr;  // per-block partials: 6 doubles each (norms need 6)
-  float* err = nullptr;
+  float* err = nullptr;     // [3], then the word count() points at
   double* norm = nullptr;   // [max|r| x3, sum|r| x3] of the last norms() call
   void* e[2] = {nullptr, nullptr};  // mixed forms only
   float* r = nullptr;               // mixed forms only
@@ -334,6 +334,7 @@ struct BatchJob {
   int sweeps_total = 0, sweeps_done = 0;
   bool live = false;
   size_t bytes = 0;
+  unsigned* count() const { return reinterpret_cast<unsigned*>(err + 3); }
 };
 
 __global__ void batch_pack_kernel(GridGeom G, const int32_t* __restrict__ mk,
@@ -868,7 +869,7 @@ struct Batch {
   }
 
   // Queues the FP64 residual norms of the listed jobs' current states (one
-  // refine launch + one reduction per job) and one copy of all of them into
+  // launch per job) and one copy of all of them into
   // a pinned array; norms_wait() waits for that copy only.
   void norms_async(const int* ids, int count) {
     FPIE_REQUIRE((ids || count == 0) && count >= 0, FPIE_ERR_ARG, "bad arguments");
@@ -887,11 +888,10 @@ struct Batch {
       double* d = reinterpret_cast<double*>(dn.bytes());
       for (int k = 0; k < count; ++k) {
         BatchJob& j = job(ids[k]);
-        launch_refine(FPIE_FP32, j.L.sweep_grid, j.L.sweep_block, j.G, j.mask, j.g, j.x[j.cur],
-                      nullptr, nullptr, nullptr, j.parts, stream);
-        launch_norms_finalize(j.parts, j.L.nparts, d + 6 * (size_t)k, stream);
+        launch_norms(j.L, j.G, j.mask, j.g, j.x[j.cur], j.parts, j.count(), d + 6 * (size_t)k,
+                     stream);
         FPIE_CUDA(cudaGetLastError());
-        launches += 2;
+        ++launches;
       }
       FPIE_CUDA(cudaMemcpyAsync(h_norms, d, 6 * sizeof(double) * (size_t)count,
                                 cudaMemcpyDeviceToHost, stream));
@@ -908,19 +908,17 @@ struct Batch {
     norms_count = -1;
   }
 
-  // FP64 residual norms of the listed jobs' current states (one refine
-  // launch + one reduction per job), copied to out[6 * k ...].
+  // FP64 residual norms of the listed jobs' current states (one launch
+  // per job), copied to out[6 * k ...].
   void norms(const int* ids, int count, double* out) {
     FPIE_REQUIRE(ids && out && count >= 0, FPIE_ERR_ARG, "bad arguments");
     wait();
     std::vector<double> h(6 * (size_t)std::max(count, 1));
     for (int k = 0; k < count; ++k) {
       BatchJob& j = job(ids[k]);
-      launch_refine(FPIE_FP32, j.L.sweep_grid, j.L.sweep_block, j.G, j.mask, j.g, j.x[j.cur],
-                    nullptr, nullptr, nullptr, j.parts, stream);
-      launch_norms_finalize(j.parts, j.L.nparts, j.norm, stream);
+      launch_norms(j.L, j.G, j.mask, j.g, j.x[j.cur], j.parts, j.count(), j.norm, stream);
       FPIE_CUDA(cudaGetLastError());
-      launches += 2;
+      ++launches;
       FPIE_CUDA(cudaMemcpyAsync(h.data() + 6 * (size_t)k, j.norm, 6 * sizeof(double),
                                 cudaMemcpyDeviceToHost, stream));
     }
@@ -931,7 +929,7 @@ struct Batch {
   void finish(int id) {
     BatchJob& j = job(id);
     launch_grid_finish(j.L, j.G, j.mask, j.g, j.x[j.cur], j.img, j.parts,
-                       reinterpret_cast<unsigned*>(j.err + 3), j.err, stream);
+                       j.count(), j.err, stream);
     FPIE_CUDA(cudaGetLastError());
     ++launches;
   }

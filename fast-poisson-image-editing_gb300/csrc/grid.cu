@@ -310,8 +310,7 @@ struct GridSolverImpl : Solver {
   void* e[2] = {nullptr, nullptr};    // correction, FP16 or BF16 planes
   float* r = nullptr;                 // FP32 residual planes
   double* d_part6 = nullptr;          // per-block max|r|, sum|r| (double)
-  double* d_norm = nullptr;           // [max x3, sum x3]
-  double* h_norm = nullptr;           // pinned copy
+  double* h_norm = nullptr;           // pinned: [max x3, sum x3]
   uint8_t* mflags = nullptr;
   int mflags_cap = 0, mtiles_x = 0, mtiles = 0;
   bool mflags_ok = false;
@@ -353,11 +352,10 @@ struct GridSolverImpl : Solver {
     cudaFree(e[1]);
     cudaFree(r);
     cudaFree(d_part6);
-    cudaFree(d_norm);
     cudaFree(mflags);
     e[0] = e[1] = nullptr;
     r = nullptr;
-    d_part6 = d_norm = nullptr;
+    d_part6 = nullptr;
     mflags = nullptr;
     mflags_cap = 0;
     mflags_ok = false;
@@ -900,7 +898,6 @@ struct GridSolverImpl : Solver {
       FPIE_CUDA(cudaMalloc(&e[1], eb));
       FPIE_CUDA(cudaMalloc(&r, (size_t)G.plane * 3 * sizeof(float)));
       FPIE_CUDA(cudaMalloc(&d_part6, (size_t)L.nparts * 6 * sizeof(double)));
-      FPIE_CUDA(cudaMalloc(&d_norm, 6 * sizeof(double)));
       FPIE_CUDA(cudaMemsetAsync(e[0], 0, eb, stream));
       FPIE_CUDA(cudaMemsetAsync(e[1], 0, eb, stream));
       FPIE_CUDA(cudaMemsetAsync(r, 0, (size_t)G.plane * 3 * sizeof(float), stream));
@@ -929,13 +926,6 @@ struct GridSolverImpl : Solver {
       mflags_ok = false;
     }
     mvariant = v;
-  }
-
-  // FP64 norms of the residual of x[cur] (no fold) into d_norm.
-  void refine_norms(cudaStream_t st, float* rout) {
-    launch_refine(precision, L.sweep_grid, L.sweep_block, G, mask, g, x[cur], nullptr,
-                  nullptr, rout, d_part6, st);
-    launch_norms_finalize(d_part6, L.nparts, d_norm, st);
   }
 
   // Pending correction: the last cycle's e (in e[e_last]) not yet added to x.
@@ -970,7 +960,7 @@ struct GridSolverImpl : Solver {
   void mixed_flush(cudaStream_t st) {
     if (!e_pending) return;
     launch_refine(precision, L.sweep_grid, L.sweep_block, G, mask, g, x[cur], e[e_last],
-                  x[cur ^ 1], nullptr, nullptr, st);
+                  x[cur ^ 1], nullptr, st);
     cur ^= 1;
     e_pending = false;
   }
@@ -1112,12 +1102,10 @@ struct GridSolverImpl : Solver {
     FPIE_REQUIRE(ready, FPIE_ERR_STATE, "no state before reset");
     if (!d_part6) {
       FPIE_CUDA(cudaMalloc(&d_part6, (size_t)L.nparts * 6 * sizeof(double)));
-      FPIE_CUDA(cudaMalloc(&d_norm, 6 * sizeof(double)));
     }
     if (!h_norm) FPIE_CUDA(cudaMallocHost(&h_norm, 6 * sizeof(double)));
-    refine_norms(stream, nullptr);
-    post_launch(this, 2);
-    FPIE_CUDA(cudaMemcpyAsync(h_norm, d_norm, 6 * sizeof(double), cudaMemcpyDeviceToHost, stream));
+    launch_norms(L, G, mask, g, x[cur], d_part6, finish_count(), h_norm, stream);
+    post_launch(this);
     FPIE_CUDA(cudaStreamSynchronize(stream));
     std::memcpy(out, h_norm, 6 * sizeof(double));
   }

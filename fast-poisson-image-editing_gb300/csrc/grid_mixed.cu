@@ -30,54 +30,16 @@ __device__ __forceinline__ float4 ld4_any(const TS* p) {
   return make_float4(to_f(p[0]), to_f(p[1]), to_f(p[2]), to_f(p[3]));
 }
 
-// Block-wide max and sum of three doubles each; valid in thread 0.
-__device__ __forceinline__ void block_maxsum3(double (&mx)[3], double (&sm)[3]) {
-  __shared__ double sh[6][32];
-  const int tid = threadIdx.x + threadIdx.y * blockDim.x;
-  const int lane = tid & 31, warp = tid >> 5, nwarps = (blockDim.x * blockDim.y) >> 5;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      mx[c] = fmax(mx[c], __shfl_down_sync(0xffffffffu, mx[c], o));
-      sm[c] += __shfl_down_sync(0xffffffffu, sm[c], o);
-    }
-  if (lane == 0)
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      sh[c][warp] = mx[c];
-      sh[3 + c][warp] = sm[c];
-    }
-  __syncthreads();
-  if (warp == 0) {
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      mx[c] = lane < nwarps ? sh[c][lane] : 0.0;
-      sm[c] = lane < nwarps ? sh[3 + c][lane] : 0.0;
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        mx[c] = fmax(mx[c], __shfl_down_sync(0xffffffffu, mx[c], o));
-        sm[c] += __shfl_down_sync(0xffffffffu, sm[c], o);
-      }
-  }
-}
-
 // Thread = 4 adjacent pixels of one row, all channels (the one-sweep
 // kernel's geometry).  e == nullptr: no fold (x is already current);
-// r == nullptr: the residual is only reduced, not stored; parts == nullptr:
-// no norm partials (the refinement cycles do not need them).
+// r == nullptr: the residual is not stored.
 template <typename TS>
 __global__ void __launch_bounds__(256)
 grid_refine_kernel(GridGeom G, const uint8_t* __restrict__ mask, const float* __restrict__ g,
                    const float* __restrict__ xin, const TS* __restrict__ e,
-                   float* __restrict__ xout, float* __restrict__ r,
-                   double* __restrict__ parts) {
+                   float* __restrict__ xout, float* __restrict__ r) {
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
   const int i = blockIdx.y * blockDim.y + threadIdx.y;
-  double mx[3] = {0.0, 0.0, 0.0}, sm[3] = {0.0, 0.0, 0.0};
   if (i < G.n && 4 * q < G.m) {
     const long long p = G.at(i, 4 * q);
     const uint32_t mk = *reinterpret_cast<const uint32_t*>(mask + p);
@@ -95,7 +57,7 @@ grid_refine_kernel(GridGeom G, const uint8_t* __restrict__ mask, const float* __
         rt = __fadd_rn(rt, to_f(e[o + 4]));
         if (mk) *reinterpret_cast<float4*>(xout + o) = ce;
       }
-      if (mk || r) {
+      if (r) {
         const float gv[4] = {__ldg(g + o), __ldg(g + o + 1), __ldg(g + o + 2), __ldg(g + o + 3)};
         const float xv[6] = {lf, ce.x, ce.y, ce.z, ce.w, rt};
         const float uv[4] = {up.x, up.y, up.z, up.w}, dv[4] = {dn.x, dn.y, dn.z, dn.w};
@@ -103,61 +65,152 @@ grid_refine_kernel(GridGeom G, const uint8_t* __restrict__ mask, const float* __
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
           const bool on = (mk >> (8 * k)) & 0xffu;
-          const float v = on ? -grid_res(xv[k + 1], gv[k], uv[k], dv[k], xv[k], xv[k + 2]) : 0.0f;
-          rr[k] = v;
-          mx[c] = fmax(mx[c], (double)fabsf(v));
-          sm[c] += (double)fabsf(v);
+          rr[k] = on ? -grid_res(xv[k + 1], gv[k], uv[k], dv[k], xv[k], xv[k + 2]) : 0.0f;
         }
-        if (r) *reinterpret_cast<float4*>(r + o) = make_float4(rr[0], rr[1], rr[2], rr[3]);
+        *reinterpret_cast<float4*>(r + o) = make_float4(rr[0], rr[1], rr[2], rr[3]);
       }
-    }
-  }
-  if (parts == nullptr) return;  // uniform: a kernel argument
-  block_maxsum3(mx, sm);
-  if (threadIdx.x == 0 && threadIdx.y == 0) {
-    const long long b = blockIdx.y * (long long)gridDim.x + blockIdx.x;
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      parts[6 * b + c] = mx[c];
-      parts[6 * b + 3 + c] = sm[c];
     }
   }
 }
 
+// ---- residual norms ------------------------------------------------------------
+// A sum of floats as hi + mid + lo, exact to about 2^-70 of it: more than a sum
+// of doubles keeps, without FP64 adds (two per SM and cycle).  Values above
+// 2^90, whose float sum could overflow where a double's does not, are added in
+// double.
+struct Sum3 {
+  float hi = 0.f, mid = 0.f, lo = 0.f;
+  double big = 0.0;
+};
+__device__ __forceinline__ float two_sum(float a, float b, float& err) {
+  const float t = __fadd_rn(a, b), c = __fsub_rn(t, a);
+  err = __fadd_rn(__fsub_rn(a, __fsub_rn(t, c)), __fsub_rn(b, c));
+  return t;
+}
+__device__ __forceinline__ void sum3_add(Sum3& s, float v) {
+  float e, f;
+  s.hi = two_sum(s.hi, v, e);
+  s.mid = two_sum(s.mid, e, f);
+  s.lo = __fadd_rn(s.lo, f);
+}
+
+// max |r| and sum |r| per channel of the state x, out[0..2] and out[3..5]; the
+// last block to arrive reduces the blocks' partials (6 doubles each) in a fixed
+// order.  One launch: with a second one for the blocks and FP64 reductions a
+// check of a 152x152 grid took 14 us.
 __global__ void __launch_bounds__(256)
-norms_finalize_kernel(const double* __restrict__ parts, int nparts, double* __restrict__ out) {
-  double mx[3] = {0.0, 0.0, 0.0}, sm[3] = {0.0, 0.0, 0.0};
-  for (int k = threadIdx.x; k < nparts; k += blockDim.x)
+grid_norms_kernel(GridGeom G, const uint8_t* __restrict__ mask, const float* __restrict__ g,
+                  const float* __restrict__ x, double* __restrict__ parts,
+                  unsigned* __restrict__ count, double* __restrict__ out, int rows) {
+  const int q = blockIdx.x * blockDim.x + threadIdx.x;
+  const int i0 = (blockIdx.y * blockDim.y + threadIdx.y) * rows;
+  const int i1 = 4 * q < G.m ? min(i0 + rows, G.n) : i0;
+  float mx[3] = {0.f, 0.f, 0.f};
+  Sum3 sm[3];
+  for (int i = i0; i < i1; ++i) {
+    const long long p = G.at(i, 4 * q);
+    const uint32_t mk = __ldg(reinterpret_cast<const uint32_t*>(mask + p));
+    if (!mk) continue;
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-      mx[c] = fmax(mx[c], parts[6 * k + c]);
-      sm[c] += parts[6 * k + 3 + c];
-    }
-  block_maxsum3(mx, sm);
-  if (threadIdx.x == 0)
+      const float* xc = x + c * G.plane + p;
+      const float4 ce = ld4(xc), up = ld4(xc - G.pitch), dn = ld4(xc + G.pitch);
+      const float4 gg = ld4(g + c * G.plane + p);
+      const float xv[6] = {__ldg(xc - 1), ce.x, ce.y, ce.z, ce.w, __ldg(xc + 4)};
+      const float uv[4] = {up.x, up.y, up.z, up.w}, dv[4] = {dn.x, dn.y, dn.z, dn.w};
+      const float gv[4] = {gg.x, gg.y, gg.z, gg.w};
 #pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      out[c] = mx[c];
-      out[3 + c] = sm[c];
+      for (int k = 0; k < 4; ++k)
+        if ((mk >> (8 * k)) & 0xffu) {
+          const float v = fabsf(grid_res(xv[k + 1], gv[k], uv[k], dv[k], xv[k], xv[k + 2]));
+          mx[c] = fmaxf(mx[c], v);
+          if (v > 0x1p90f)
+            sm[c].big += (double)v;
+          else
+            sum3_add(sm[c], v);
+        }
     }
+  }
+  __shared__ float shm[3][8];
+  __shared__ double shs[3][8];
+  __shared__ bool last;
+  const int tid = threadIdx.x + threadIdx.y * blockDim.x, lane = tid & 31, warp = tid >> 5;
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    // Not negative and no NaN (a maximum drops them): bits order as values do.
+    const float m = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(mx[c])));
+    const bool big = __any_sync(0xffffffffu, sm[c].big != 0.0);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const float h = __shfl_down_sync(0xffffffffu, sm[c].hi, o);
+      const float d = __shfl_down_sync(0xffffffffu, sm[c].mid, o);
+      const float l = __shfl_down_sync(0xffffffffu, sm[c].lo, o);
+      sum3_add(sm[c], h);
+      float e;
+      sm[c].mid = two_sum(sm[c].mid, d, e);
+      sm[c].lo = __fadd_rn(sm[c].lo, __fadd_rn(l, e));
+      if (big) sm[c].big += __shfl_down_sync(0xffffffffu, sm[c].big, o);
+    }
+    if (lane == 0) {
+      shm[c][warp] = m;
+      shs[c][warp] = isfinite(sm[c].hi)
+                         ? (((double)sm[c].hi + (double)sm[c].mid) + (double)sm[c].lo) + sm[c].big
+                         : (double)sm[c].hi;
+    }
+  }
+  __syncthreads();
+  const unsigned block = blockIdx.y * gridDim.x + blockIdx.x, blocks = gridDim.x * gridDim.y;
+  if (tid < 3) {
+    float m = 0.f;
+    double t = 0.0;
+    for (int w = 0; w < 8; ++w) {
+      m = fmaxf(m, shm[tid][w]);
+      t += shs[tid][w];
+    }
+    parts[6 * (size_t)block + tid] = (double)m;
+    parts[6 * (size_t)block + 3 + tid] = t;
+    __threadfence();
+  }
+  __syncthreads();
+  if (tid == 0) last = atomicAdd(count, 1u) == blocks - 1;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  // Warp 0 per column of the partials: lanes stride over the blocks.
+  if (warp < 6) {
+    double v = 0.0;
+    for (unsigned k = lane; k < blocks; k += 32) {
+      const double u = __ldcg(parts + 6 * (size_t)k + warp);
+      v = warp < 3 ? fmax(v, u) : v + u;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const double u = __shfl_down_sync(0xffffffffu, v, o);
+      v = warp < 3 ? fmax(v, u) : v + u;
+    }
+    if (lane == 0) out[warp] = v;
+  }
+  if (tid == 0) *count = 0;
 }
 
 void launch_refine(int precision, dim3 grid, dim3 block, const GridGeom& G, const uint8_t* mask,
                    const float* g, const float* xin, const void* e, float* xout, float* r,
-                   double* parts, cudaStream_t st) {
+                   cudaStream_t st) {
   if (precision == FPIE_MIXED_BF16)
     grid_refine_kernel<__nv_bfloat16><<<grid, block, 0, st>>>(
-        G, mask, g, xin, static_cast<const __nv_bfloat16*>(e), xout, r, parts);
+        G, mask, g, xin, static_cast<const __nv_bfloat16*>(e), xout, r);
   else if (precision == FPIE_MIXED_FP16)
     grid_refine_kernel<__half><<<grid, block, 0, st>>>(G, mask, g, xin,
-                                                       static_cast<const __half*>(e), xout, r, parts);
+                                                       static_cast<const __half*>(e), xout, r);
   else
     grid_refine_kernel<float><<<grid, block, 0, st>>>(G, mask, g, xin,
-                                                      static_cast<const float*>(e), xout, r, parts);
+                                                      static_cast<const float*>(e), xout, r);
 }
 
-void launch_norms_finalize(const double* parts, int nparts, double* out, cudaStream_t st) {
-  norms_finalize_kernel<<<1, 256, 0, st>>>(parts, nparts, out);
+void launch_norms(const GridLaunch& L, const GridGeom& G, const uint8_t* mask, const float* g,
+                  const float* x, double* parts, unsigned* count, double* out, cudaStream_t st) {
+  grid_norms_kernel<<<L.finish_grid, L.finish_block, 0, st>>>(G, mask, g, x, parts, count, out,
+                                                              L.finish_rows);
 }
 
 }  // namespace fpie

@@ -119,3 +119,51 @@ def test_finish_sums_that_overflow_or_are_no_number():
     o = np_jacobi.GridJacobi(mask, tgt, grad)
     with np.errstate(all="ignore"):
         np.testing.assert_array_equal(err, o.err64().astype(np.float32))
+
+
+@pytest.mark.parametrize("shape", [(1, 1), (5, 3), (9, 130), (40, 259), (333, 517), (1700, 2100)])
+def test_norms_any_shape(shape):
+    """max |r| exactly, sum |r| to 1e-14 of the float64 sum (its terms are
+    float32 values, summed without FP64 rounding to 2^-52)."""
+    from fpie_gb300 import backend
+
+    n, m = shape
+    rng = np.random.default_rng(n * 7 + m)
+    mask = (rng.random((n, m)) < 0.8).astype(np.int32)
+    tgt = rng.uniform(-50, 300, (n, m, 3)).astype(np.float32)
+    grad = rng.uniform(-30, 30, (n, m, 3)).astype(np.float32)
+    s = backend.GridSolver(8, 8)
+    s.reset(mask.size, mask, tgt, grad)
+    for _ in range(2):
+        r = np.abs(_residual(mask, tgt, grad)).astype(np.float64)
+        mx, sm = s.residual_norms()
+        np.testing.assert_array_equal(mx, r.max((0, 1)))
+        np.testing.assert_allclose(sm, [np.sum(np.sort(r[..., c].ravel())) for c in range(3)], rtol=1e-14)
+
+
+def _residual(mask, x, g):
+    """The oracle's float32 residual, numpy order, 0 outside the mask."""
+    p = np.pad(x, ((1, 1), (1, 1), (0, 0)))
+    four = np.float32(4)
+    r = four * x - g
+    for nb in (p[:-2, 1:-1], p[2:, 1:-1], p[1:-1, :-2], p[1:-1, 2:]):
+        r = r - nb
+    r[mask == 0] = 0
+    return r
+
+
+@pytest.mark.parametrize("scale", [1e36, 1e-42])
+def test_norms_of_huge_and_tiny_residuals(scale):
+    from fpie_gb300 import backend
+
+    rng = np.random.default_rng(1)
+    mask = np.ones((50, 70), np.int32)
+    tgt = (rng.uniform(-1, 1, (50, 70, 3)) * scale).astype(np.float32)
+    tgt[:, :35] *= np.float32(1e-20) if scale > 1 else np.float32(1)
+    grad = np.zeros_like(tgt)
+    s = backend.GridSolver(8, 8)
+    s.reset(mask.size, mask, tgt, grad)
+    r = np.abs(_residual(mask, tgt, grad)).astype(np.float64)
+    mx, sm = s.residual_norms()
+    np.testing.assert_array_equal(mx, r.max((0, 1)))
+    np.testing.assert_allclose(sm, r.sum((0, 1)), rtol=1e-13)
