@@ -1122,9 +1122,9 @@ def batch_jobs(n_jobs: int = 256, seed: int = 7, mix=None):
 
 def batch_study(jobs, precision: str = "fp32", sequential: bool = True) -> dict:
     """All jobs in one persistent launch (BatchSolver.run to completion) vs
-    one GridSolver per job back to back.  The autotuner (64 real sweeps of
-    every job per candidate) runs on a first batch of the same jobs and is
-    timed on its own; the timed batch is pinned to the tuned kernel."""
+    one GridSolver per job back to back.  A first batch of the same jobs
+    warms up and names the kernel that the engine chooses for them; it is
+    timed on its own, and the timed batch is pinned to that kernel."""
     import torch
 
     from fpie_gb300 import backend
@@ -1137,7 +1137,7 @@ def batch_study(jobs, precision: str = "fp32", sequential: bool = True) -> dict:
         tune.add(mc, t, g, it)
     torch.cuda.synchronize()
     t0 = time.perf_counter()
-    tune.run(256)  # 3 candidates x 64 sweeps + 64 more
+    tune.run(256)
     torch.cuda.synchronize()
     tune_s = time.perf_counter() - t0
     kernel = tune.kernel

@@ -306,6 +306,7 @@ static const std::vector<BatchVariant>& batch_variants() {
       make_bv<16, 8, 16>("p16w8k16"),
       make_bv<8, 16, 16>("p8w16k16"),
       make_bv<16, 8, 8>("p16w8k8"),
+      make_bv<8, 8, 16>("p8w8k16"),
   };
   return v;
 }
@@ -362,7 +363,7 @@ struct Batch {
   std::vector<BatchJob> jobs;
   size_t budget = 0, used = 0;
   int variant = 0;
-  bool tuned = false, pinned = false;
+  bool pinned = false;
   long long launches = 0;
   long long spin_limit = 1LL << 25;  // x ~128 ns sleeps: a few seconds at most
   int sms = 0;
@@ -674,9 +675,8 @@ struct Batch {
   bool prepared[8][3] = {};
 
   // Runs `sweeps[id]` more sweeps of the listed jobs in one persistent launch
-  // of variant v; returns the device milliseconds (measured with events).
-  float launch(const std::vector<int>& ids, const std::vector<int>& sw, int vi, bool time_it,
-               bool async = false) {
+  // of variant v.
+  void launch(const std::vector<int>& ids, const std::vector<int>& sw, int vi, bool async) {
     const BatchVariant& v = batch_variants()[vi];
     std::vector<BJobDev> dj;
     std::vector<int2> tiles;
@@ -720,7 +720,6 @@ struct Batch {
       act[z] = a;
       lo[z + 1] = lo[z] + ct[a];
     }
-    float ms = 0.f;
     if (nlevels > 0 && lo[nlevels] > 0) {
       // One device block for the queue tables (freed after the launch).
       const size_t b_jobs = sizeof(BJobDev) * nj, b_order = sizeof(int) * nj,
@@ -769,17 +768,10 @@ struct Batch {
       FPIE_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, v.kernel[precision],
                                                               v.warps * 32, dyn));
       const int grid = std::max(1, occ) * sms;
-      cudaEvent_t e0 = nullptr, e1 = nullptr;
-      if (time_it) {
-        FPIE_CUDA(cudaEventCreate(&e0));
-        FPIE_CUDA(cudaEventCreate(&e1));
-        FPIE_CUDA(cudaEventRecord(e0, stream));
-      }
       v.launch[precision](grid, q, stream);
       FPIE_CUDA(cudaGetLastError());
       ++launches;
-      if (time_it) FPIE_CUDA(cudaEventRecord(e1, stream));
-      if (async && !time_it) {
+      if (async) {
         // The flag is read by wait(); the queue tables are freed after the
         // copy in stream order.  The jobs' bookkeeping below still applies.
         if (!h_errs) FPIE_CUDA(cudaMallocHost(&h_errs, kMaxPending * sizeof(int)));
@@ -792,11 +784,6 @@ struct Batch {
         int herr = 0;
         FPIE_CUDA(cudaMemcpyAsync(&herr, q.error, sizeof(int), cudaMemcpyDeviceToHost, stream));
         FPIE_CUDA(cudaStreamSynchronize(stream));
-        if (time_it) {
-          FPIE_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-          cudaEventDestroy(e0);
-          cudaEventDestroy(e1);
-        }
         FPIE_REQUIRE(herr == 0, FPIE_ERR_TIMEOUT,
                      "batch kernel: a dependency wait exceeded its spin limit");
       }
@@ -810,7 +797,6 @@ struct Batch {
       }
       j.sweeps_done += sw[k];
     }
-    return ms;
   }
 
   std::vector<int> live_ids() const {
@@ -820,41 +806,40 @@ struct Batch {
     return ids;
   }
 
-  // Advances every live job by min(limit, its remaining sweeps); limit < 0
-  // means "to completion".  Tunes the kernel on the first call with enough
-  // work (each candidate runs 64 real sweeps of every job).
-  void run(int limit, bool async = false) {
-    std::vector<int> ids = live_ids();
-    auto remaining = [&](int id) {
-      const int rem = jobs[id].sweeps_total - jobs[id].sweeps_done;
-      return limit < 0 ? rem : std::min(rem, limit);
-    };
-    int budget_sweeps = limit;
-    if (!tuned && !pinned) {
-      const int ncand = (int)batch_variants().size();
-      int minrem = 1 << 30;
-      for (int id : ids) minrem = std::min(minrem, remaining(id));
-      if (!ids.empty() && minrem >= 64 * (ncand + 1)) {
-        int best = 0;
-        float best_ms = 1e30f;
-        for (int v = 0; v < ncand; ++v) {
-          std::vector<int> sw(ids.size(), 64);
-          const float ms = launch(ids, sw, v, true);
-          if (ms < best_ms) { best_ms = ms; best = v; }
-        }
-        variant = best;
-        tuned = true;
-        if (budget_sweeps >= 0) budget_sweeps -= 64 * ncand;
-      }
+  // Which variant runs the listed jobs, unless one was named.  A launch is
+  // bound either by the chain of levels of its longest job (an item's latency
+  // per level: 13 us for "p16w8k16", 8.6 us for "p8w8k16", whose warps hold
+  // half the rows) or by the SMs' throughput, where the small regions' wider
+  // aprons cost more (2.7 region pixels per pixel of a tile instead of 1.8).
+  // Measured with up to 48 uneven jobs, us per launch, items per level of
+  // "p8w8k16" in brackets, FP32: [78] 1,634 against 2,375, [231] 2,037
+  // against 2,348, [279] 2,192 against 2,419, [333] 2,520 against 2,265,
+  // [429] 3,233 against 2,473; FP16 [78] 1,701 against 2,685, [333] 2,635
+  // against 2,533: the line lies at two items per SM.
+  int pick(const std::vector<int>& ids) {
+    const size_t small = 3;  // "p8w8k16" in batch_variants()
+    long long items = 0;
+    for (int id : ids) {
+      BatchJob& j = jobs[id];
+      if (j.tiles_of.size() != batch_variants().size()) tile_lists(j);
+      items += 3LL * (long long)j.tiles_of[small].size();
     }
+    return items <= 2LL * sms ? (int)small : 0;
+  }
+
+  // Advances every live job by min(limit, its remaining sweeps); limit < 0
+  // means "to completion".
+  void run(int limit, bool async = false) {
     std::vector<int> sw;
     std::vector<int> run_ids;
-    for (int id : ids) {
+    for (int id : live_ids()) {
       int rem = jobs[id].sweeps_total - jobs[id].sweeps_done;
-      if (budget_sweeps >= 0) rem = std::min(rem, std::max(0, budget_sweeps));
+      if (limit >= 0) rem = std::min(rem, limit);
       if (rem > 0) { run_ids.push_back(id); sw.push_back(rem); }
     }
-    if (!run_ids.empty()) launch(run_ids, sw, variant, false, async);
+    if (run_ids.empty()) return;
+    if (!pinned) variant = pick(run_ids);
+    launch(run_ids, sw, variant, async);
   }
 
   // Waits for everything queued on the batch's stream and checks the error
@@ -1096,7 +1081,6 @@ int fpie_batch_set_kernel(fpie_batch* b, const char* name) {
     FPIE_REQUIRE(name != nullptr, FPIE_ERR_ARG, "null kernel name");
     if (std::string(name) == "auto") {
       h->pinned = false;
-      h->tuned = false;
       return;
     }
     for (size_t k = 0; k < batch_variants().size(); ++k)

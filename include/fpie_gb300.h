@@ -322,9 +322,8 @@ int fpie_grid_step_noalloc(int n, int m, const int32_t* mask, float* x,
  * a grid problem in the GridSolver layouts plus its own sweep count.
  * fpie_batch_run advances every job by min(max_sweeps, its remaining
  * sweeps) (max_sweeps < 0: to completion) in one persistent kernel whose
- * CTAs pull (job, tile, channel, level) items from a queue; the first run
- * with enough work autotunes the tile shape and temporal depth on real
- * sweeps.  A job's result is bit-identical to a GridSolver run of the same
+ * CTAs pull (job, tile, channel, level) items from a queue; the tile shape
+ * follows from the number of items the run has for each SM.  A job's result is bit-identical to a GridSolver run of the same
  * sweeps.  Dependency waits inside the kernel are bounded: past the spin
  * limit the call returns FPIE_ERR_TIMEOUT and the jobs' states are
  * undefined (remove and re-add them). */
@@ -360,9 +359,8 @@ int fpie_batch_add_images(fpie_batch* b, const uint8_t* src, int src_h, int src_
                           int tgt_row, int tgt_col, int gradient, int iterations, int* job_id,
                           int* box);
 int fpie_batch_run(fpie_batch* b, int max_sweeps);
-/* fpie_batch_run without waiting for the launch (the first run with enough
- * work still tunes synchronously); fpie_batch_wait waits for all queued work
- * and reports a dependency wait that exceeded its limit (FPIE_ERR_TIMEOUT).
+/* fpie_batch_run without waiting for the launch; fpie_batch_wait waits for all
+ * queued work and reports a dependency wait that exceeded its limit (FPIE_ERR_TIMEOUT).
  * Jobs added or removed meanwhile take effect in stream order. */
 int fpie_batch_run_async(fpie_batch* b, int max_sweeps);
 int fpie_batch_wait(fpie_batch* b);
