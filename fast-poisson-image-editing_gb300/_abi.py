@@ -47,6 +47,8 @@ _PROTOS: dict[str, tuple] = {
     "fpie_grid_create": ([_I, _I, ctypes.POINTER(_P)], _I),
     "fpie_grid_reset": ([_P, _I, _I, _I, _P, _P, _P], _I),
     "fpie_grid_step": ([_P, _I, _P, _P], _I),
+    "fpie_grid_step_into": ([_P, _I, _P, ctypes.c_longlong, _P], _I),
+    "fpie_equ_step_into": ([_P, _I, _P, _P, _I, _P, _I, _I, _P, ctypes.POINTER(_I)], _I),
     "fpie_sync": ([_P], _I),
     "fpie_destroy": ([_P], _I),
     "fpie_set_stream": ([_P, _P], _I),
@@ -71,6 +73,7 @@ _PROTOS: dict[str, tuple] = {
     "fpie_equ_reset_images": ([_P, _P, _I, _I, _P, _I, _I, _I, _P, _I, _I, _I, _I, _I, _I, _I,
                                _I, _P, ctypes.POINTER(_I)], _I),
     "fpie_equ_get_index": ([_P, _P, _P], _I),
+    "fpie_equ_get_index64": ([_P, _P, _P], _I),
     "fpie_equ_get_inputs": ([_P, _P, _P], _I),
     "fpie_equ_set_kernel": ([_P, ctypes.c_char_p], _I),
     "fpie_equ_kernel": ([_P, ctypes.c_char_p, _I], _I),

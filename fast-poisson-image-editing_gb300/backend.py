@@ -43,6 +43,12 @@ def _as(a, dtype, shape=None, name="array") -> np.ndarray:
     return out
 
 
+def _is_rgb(a) -> bool:
+    """Whether a is an image that native code may store into as uint8[h][w][3]."""
+    return (type(a) is np.ndarray and a.dtype == np.uint8 and a.ndim == 3 and a.shape[2] == 3
+            and a.flags.c_contiguous and a.flags.writeable)
+
+
 def _image_args(src, mask, tgt, gradient):
     """Pointers, shapes and codes for the *_reset_images calls (numpy or CUDA tensors)."""
     mode = {"src": 0, "avg": 1, "max": 2}.get(gradient)
@@ -206,6 +212,24 @@ class EquSolver(_Solver):
         _abi.call("fpie_equ_step", self._h, int(iteration), _ptr(x), _ptr(err))
         return x, err
 
+    def step_into(self, iteration: int, image: np.ndarray, index) -> np.ndarray:
+        """step() with the unknowns 1..N-1 stored into ``image`` at ``index``
+        = (rows, cols), as ``image[index] = x[1:]`` does; returns err."""
+        if _is_rgb(image) and isinstance(index, tuple) and len(index) == 2 and self.N > 1 and all(
+                type(a) is np.ndarray and a.dtype == np.int64 and a.shape == (self.N - 1,)
+                and a.flags.c_contiguous for a in index):
+            err = np.empty(3, np.float32)
+            stored = ctypes.c_int(0)
+            _abi.call("fpie_equ_step_into", self._h, int(iteration), _ptr(index[0]),
+                      _ptr(index[1]), self.N - 1, _ptr(image), image.shape[0], image.shape[1],
+                      _ptr(err), ctypes.byref(stored))
+            if stored.value:
+                return err
+            iteration = 0  # the sweeps are done; numpy judges the coordinates
+        x, err = self.step(iteration)
+        image[index] = x[1:]
+        return err
+
     def reset_images(self, src, mask, tgt, mask_on_src: tuple[int, int],
                      mask_on_tgt: tuple[int, int], gradient: str = "max"):
         """Build ids/A/X/B on the GPU from uint8 images (EquProcessor.reset semantics).
@@ -220,11 +244,11 @@ class EquSolver(_Solver):
                   ctypes.byref(n_out))
         del keep
         self.N = n_out.value
-        rows = np.empty(self.N - 1, np.int32)
-        cols = np.empty(self.N - 1, np.int32)
+        rows = np.empty(self.N - 1, np.int64)
+        cols = np.empty(self.N - 1, np.int64)
         if self.N > 1:
-            _abi.call("fpie_equ_get_index", self._h, _ptr(rows), _ptr(cols))
-        return self.N, tuple(box), (rows.astype(np.int64), cols.astype(np.int64))
+            _abi.call("fpie_equ_get_index64", self._h, _ptr(rows), _ptr(cols))
+        return self.N, tuple(box), (rows, cols)
 
     def set_kernel(self, name: str) -> None:
         """"auto" (grid kernels for 4-neighbour raster systems, else gather),
@@ -291,6 +315,21 @@ class GridSolver(_Solver):
         err = np.empty(3, np.float32)
         _abi.call("fpie_grid_step", self._h, int(iteration), _ptr(img), _ptr(err))
         return img, err
+
+    def step_into(self, iteration: int, image: np.ndarray, box) -> np.ndarray:
+        """step() with the picture stored into ``image`` at ``box`` = (row0,
+        row1, col0, col1), as ``image[row0:row1, col0:col1] = img`` does;
+        returns err."""
+        r0, r1, c0, c1 = box
+        if (_is_rgb(image) and 0 <= r0 < r1 <= image.shape[0] and 0 <= c0 < c1 <= image.shape[1]
+                and self.shape == (r1 - r0, c1 - c0)):
+            err = np.empty(3, np.float32)
+            _abi.call("fpie_grid_step_into", self._h, int(iteration),
+                      _ptr(image) + 3 * (r0 * image.shape[1] + c0), 3 * image.shape[1], _ptr(err))
+            return err
+        img, err = self.step(iteration)
+        image[r0:r1, c0:c1] = img
+        return err
 
     def set_kernel(self, name: str) -> None:
         """Pin the sweep kernel ("auto", "sweep1", or a variant like "p16w8k16")."""

@@ -45,6 +45,17 @@ __global__ void equ_pack_kernel(EquGeom E, const float* __restrict__ X,
   }
 }
 
+// Index arrays in the width numpy indexes with.
+__global__ void equ_widen_kernel(size_t n, const int* __restrict__ rows,
+                                 const int* __restrict__ cols, int64_t* __restrict__ wr,
+                                 int64_t* __restrict__ wc) {
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
+       i += (size_t)gridDim.x * blockDim.x) {
+    wr[i] = rows[i];
+    wc[i] = cols[i];
+  }
+}
+
 // Counts A entries outside [0, N) so no sweep ever gathers out of bounds.
 __global__ void equ_check_kernel(EquGeom E, const int4* __restrict__ A,
                                  unsigned int* __restrict__ bad) {
@@ -713,8 +724,22 @@ struct EquSolverImpl : Solver {
     choose_mode(nullptr);
   }
 
-  int* d_rows = nullptr;  // target coordinates of unknowns 1..N-1 (GPU reset)
+  // Target coordinates of unknowns 1..N-1 (GPU reset), in arrays that only
+  // grow: freeing and allocating them on each reset synchronised the device.
+  int* d_rows = nullptr;
   int* d_cols = nullptr;
+  int idx_cap = 0;
+
+  void ensure_index(int unknowns) {
+    if (unknowns <= idx_cap && d_rows) return;
+    cudaFree(d_rows);
+    cudaFree(d_cols);
+    d_rows = d_cols = nullptr;
+    idx_cap = 0;
+    FPIE_CUDA(cudaMalloc(&d_rows, sizeof(int) * (size_t)std::max(unknowns, 1)));
+    FPIE_CUDA(cudaMalloc(&d_cols, sizeof(int) * (size_t)std::max(unknowns, 1)));
+    idx_cap = std::max(unknowns, 1);
+  }
 
   // GPU-side counterpart of EquProcessor.reset (fpie/process.py:192-271):
   // ids, A, X, B and the unknowns' target coordinates from the uint8 images.
@@ -775,11 +800,7 @@ struct EquSolverImpl : Solver {
     if (rb) n_mid = tallies[1] + 1;
     const int N = unknowns + 1;
     allocate(N);
-    cudaFree(d_rows);
-    cudaFree(d_cols);
-    d_rows = d_cols = nullptr;
-    FPIE_CUDA(cudaMalloc(&d_rows, sizeof(int) * std::max(unknowns, 1)));
-    FPIE_CUDA(cudaMalloc(&d_cols, sizeof(int) * std::max(unknowns, 1)));
+    ensure_index(unknowns);
     FPIE_CUDA(cudaMemsetAsync(A, 0, sizeof(int4) * N, stream));
     FPIE_CUDA(cudaMemsetAsync(x[0], 0, (size_t)E.np * 3 * sizeof(float), stream));
     FPIE_CUDA(cudaMemsetAsync(x[1], 0, (size_t)E.np * 3 * sizeof(float), stream));
@@ -805,9 +826,29 @@ struct EquSolverImpl : Solver {
     return N;
   }
 
-  void get_index(int32_t* rows, int32_t* cols) {
+  void check_index(const void* rows, const void* cols) const {
     FPIE_REQUIRE(rows && cols, FPIE_ERR_ARG, "null output array");
-    FPIE_REQUIRE(ready && d_rows, FPIE_ERR_STATE, "no index: the solver was not reset from images");
+    FPIE_REQUIRE(ready && d_rows && E.N - 1 <= idx_cap, FPIE_ERR_STATE,
+                 "no index: the solver was not reset from images");
+  }
+
+  // Widened on the device: 5 MB of 64-bit indices copied out take 39 us,
+  // widening 640,000 32-bit ones on the host took 190 (400 through numpy).
+  void get_index64(int64_t* rows, int64_t* cols) {
+    check_index(rows, cols);
+    const size_t n = (size_t)(E.N - 1);
+    if (!n) return;
+    AsyncScratch wide(2 * n * sizeof(int64_t), stream);
+    int64_t* w = reinterpret_cast<int64_t*>(wide.bytes());
+    equ_widen_kernel<<<conv_blocks((long long)n), 256, 0, stream>>>(n, d_rows, d_cols, w, w + n);
+    post_launch(this);
+    FPIE_CUDA(cudaMemcpyAsync(rows, w, n * sizeof(int64_t), cudaMemcpyDeviceToHost, stream));
+    FPIE_CUDA(cudaMemcpyAsync(cols, w + n, n * sizeof(int64_t), cudaMemcpyDeviceToHost, stream));
+    FPIE_CUDA(cudaStreamSynchronize(stream));
+  }
+
+  void get_index(int32_t* rows, int32_t* cols) {
+    check_index(rows, cols);
     FPIE_CUDA(cudaMemcpyAsync(rows, d_rows, sizeof(int) * (E.N - 1), cudaMemcpyDeviceToHost, stream));
     FPIE_CUDA(cudaMemcpyAsync(cols, d_cols, sizeof(int) * (E.N - 1), cudaMemcpyDeviceToHost, stream));
     FPIE_CUDA(cudaStreamSynchronize(stream));
@@ -933,6 +974,38 @@ struct EquSolverImpl : Solver {
     std::memcpy(err_out, h_err, 3 * sizeof(float));
   }
 
+  std::vector<uint8_t> h_x;  // step_into: the unknowns' bytes on the host
+
+  // step_host with unknown k stored at pixel (rows[k-1], cols[k-1]) of the
+  // image dst.  The coordinates are the caller's, so they are checked (while
+  // the GPU sweeps); where one lies outside the image nothing is stored and
+  // false is returned, the sweeps done.
+  bool step_into(int iteration, const int64_t* rows, const int64_t* cols, int count, uint8_t* dst,
+                 int h, int w, float* err_out) {
+    FPIE_REQUIRE(rows && cols && dst && err_out, FPIE_ERR_ARG, "null array");
+    if (!ready) {
+      err_out[0] = err_out[1] = err_out[2] = 0.0f;
+      return false;
+    }
+    FPIE_REQUIRE(count == E.N - 1, FPIE_ERR_ARG, "one pixel per unknown");
+    run_sweeps(iteration);
+    finish(d_img, d_err);
+    uint64_t out = 0;
+    for (int k = 0; k < count; ++k)
+      out |= (uint64_t)((uint64_t)rows[k] >= (uint64_t)h) | (uint64_t)((uint64_t)cols[k] >= (uint64_t)w);
+    h_x.resize((size_t)E.N * 3);
+    FPIE_CUDA(cudaMemcpyAsync(h_x.data(), d_img, (size_t)E.N * 3, cudaMemcpyDeviceToHost, stream));
+    FPIE_CUDA(cudaMemcpyAsync(h_err, d_err, 3 * sizeof(float), cudaMemcpyDeviceToHost, stream));
+    FPIE_CUDA(cudaStreamSynchronize(stream));
+    check_async();
+    std::memcpy(err_out, h_err, 3 * sizeof(float));
+    if (out) return false;
+    const uint8_t* px = h_x.data() + 3;
+    for (int k = 0; k < count; ++k)
+      std::memcpy(dst + 3 * ((size_t)rows[k] * (size_t)w + (size_t)cols[k]), px + 3 * (size_t)k, 3);
+    return true;
+  }
+
   void get_state(float* out) {
     FPIE_REQUIRE(out, FPIE_ERR_ARG, "null output array");
     FPIE_REQUIRE(ready, FPIE_ERR_STATE, "no state before reset");
@@ -1020,6 +1093,18 @@ int fpie_equ_reset_images(fpie_solver* s, const uint8_t* src, int src_h, int src
 
 int fpie_equ_get_index(fpie_solver* s, int32_t* rows, int32_t* cols) {
   return guarded([&] { equ_of(s)->get_index(rows, cols); });
+}
+
+int fpie_equ_get_index64(fpie_solver* s, int64_t* rows, int64_t* cols) {
+  return guarded([&] { equ_of(s)->get_index64(rows, cols); });
+}
+
+int fpie_equ_step_into(fpie_solver* s, int iteration, const int64_t* rows, const int64_t* cols,
+                       int count, uint8_t* dst, int h, int w, float* err_out, int* stored) {
+  return guarded([&] {
+    const bool done = equ_of(s)->step_into(iteration, rows, cols, count, dst, h, w, err_out);
+    if (stored) *stored = done ? 1 : 0;
+  });
 }
 
 int fpie_equ_get_inputs(fpie_solver* s, int32_t* A, float* B) {

@@ -1237,6 +1237,27 @@ struct GridSolverImpl : Solver {
     std::memcpy(err_out, h_err, 3 * sizeof(float));
   }
 
+  // step_host with row i of the picture stored at dst + i * pitch, one 2-D
+  // copy: 810 KB into an image take 13 us, a contiguous array and a host copy
+  // of its rows 58.  dst keeps its bytes when a kernel gave up waiting.
+  void step_into(int iteration, uint8_t* dst, long long pitch, float* err_out) {
+    FPIE_REQUIRE(dst && err_out, FPIE_ERR_ARG, "null output array");
+    if (!ready) {
+      err_out[0] = err_out[1] = err_out[2] = 0.0f;
+      return;
+    }
+    FPIE_REQUIRE(pitch >= 3LL * G.m, FPIE_ERR_ARG, "rows of the picture overlap");
+    run_sweeps(iteration);
+    finish(d_img, d_err);
+    FPIE_CUDA(cudaMemcpyAsync(h_err, d_err, 4 * sizeof(float), cudaMemcpyDeviceToHost, stream));
+    FPIE_CUDA(cudaStreamSynchronize(stream));
+    raise_waits();
+    FPIE_CUDA(cudaMemcpy2DAsync(dst, (size_t)pitch, d_img, (size_t)G.m * 3, (size_t)G.m * 3,
+                                (size_t)G.n, cudaMemcpyDeviceToHost, stream));
+    FPIE_CUDA(cudaStreamSynchronize(stream));
+    std::memcpy(err_out, h_err, 3 * sizeof(float));
+  }
+
   void get_state(float* out) {
     FPIE_REQUIRE(out, FPIE_ERR_ARG, "null output array");
     FPIE_REQUIRE(ready, FPIE_ERR_STATE, "no state before reset");
@@ -1273,6 +1294,11 @@ int fpie_grid_reset(fpie_solver* s, int N, int n, int m, const int32_t* mask,
 int fpie_grid_step(fpie_solver* s, int iteration, uint8_t* img_out,
                    float* err_out) {
   return guarded([&] { grid_of(s)->step_host(iteration, img_out, err_out); });
+}
+
+int fpie_grid_step_into(fpie_solver* s, int iteration, uint8_t* dst, long long pitch,
+                        float* err_out) {
+  return guarded([&] { grid_of(s)->step_into(iteration, dst, pitch, err_out); });
 }
 
 int fpie_grid_reset_device(fpie_solver* s, int n, int m, const int32_t* mask,

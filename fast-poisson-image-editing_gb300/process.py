@@ -145,8 +145,7 @@ class EquProcessor(BaseProcessor):
         return system.N
 
     def step(self, iteration: int):
-        x, err = self.core.step(iteration)
-        self.tgt[self.tgt_index] = x[1:]
+        err = self.core.step_into(iteration, self.tgt, self.tgt_index)
         return self.tgt, err
 
 
@@ -176,6 +175,5 @@ class GridProcessor(BaseProcessor):
         return n
 
     def step(self, iteration: int):
-        img, err = self.core.step(iteration)
-        self.tgt[self.x0:self.x1, self.y0:self.y1] = img
+        err = self.core.step_into(iteration, self.tgt, (self.x0, self.x1, self.y0, self.y1))
         return self.tgt, err

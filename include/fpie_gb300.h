@@ -108,6 +108,12 @@ int fpie_equ_reset_placed(fpie_solver* s, int N, const int32_t* A, const float* 
  * err_out[3]. */
 int fpie_equ_step(fpie_solver* s, int iteration, uint8_t* x_out,
                   float* err_out);
+/* fpie_equ_step with unknown k = 1..count stored at pixel (rows[k-1],
+ * cols[k-1]) of the host image dst, uint8[h][w][3]; count must be N - 1.  A
+ * coordinate outside the image: the sweeps run, *stored is 0 and dst keeps
+ * its bytes (fpie_equ_step of 0 sweeps then gives the result). */
+int fpie_equ_step_into(fpie_solver* s, int iteration, const int64_t* rows, const int64_t* cols,
+                       int count, uint8_t* dst, int h, int w, float* err_out, int* stored);
 
 /* ---- GridSolver: fpie/core/base_solver.h:77-152, fpie/core/cuda/grid.cu -- */
 
@@ -127,6 +133,11 @@ int fpie_grid_reset(fpie_solver* s, int N, int n, int m, const int32_t* mask,
  * uint8[n][m][3]. */
 int fpie_grid_step(fpie_solver* s, int iteration, uint8_t* img_out,
                    float* err_out);
+/* fpie_grid_step with row i of the picture stored at dst + i * pitch bytes
+ * (pitch >= 3 m): the crop of a larger host image.  dst keeps its bytes when
+ * the call fails. */
+int fpie_grid_step_into(fpie_solver* s, int iteration, uint8_t* dst, long long pitch,
+                        float* err_out);
 
 /* ---- shared ------------------------------------------------------------ */
 
@@ -192,6 +203,8 @@ int fpie_equ_reset_images(fpie_solver* s, const uint8_t* src, int src_h, int src
 /* Target-image coordinates of unknowns 1..N-1 after fpie_equ_reset_images
  * (the processor's tgt_index, fpie/process.py:269): rows, cols int32[N-1]. */
 int fpie_equ_get_index(fpie_solver* s, int32_t* rows, int32_t* cols);
+/* The same as 64-bit integers. */
+int fpie_equ_get_index64(fpie_solver* s, int64_t* rows, int64_t* cols);
 
 /* Copies the equation inputs the solver holds: A int32[N][4], B
  * float32[N][3]. */
