@@ -7,12 +7,13 @@
 // (a 194x194 grid: 5.6 us per 8-sweep launch, of which ~1.6 us are sweeps):
 // launch, region load and store, tail.  Here that is one exchange, and
 // regions are cut as small as lets every SM hold one.  Per sweep: 194x194
-// 0.295 us (0.71 before), 251x389 0.403 (0.83), 176x1457 0.564 (0.83).
+// 0.298 us (0.71 as launches of 8 sweeps), 251x389 0.407 (0.83), 176x1457
+// 0.540 (0.83).
 //
 // The update is quarter.cuh's.  Each CTA looks for values below 2^-60 every
-// 16 sweeps; one that finds some takes slow sweeps until its next look and
-// marks the packets it sends, and a CTA that receives a marked packet does the
-// same.
+// 16 sweeps, before an exchange if there is one; one that finds some takes slow
+// sweeps until its next look and marks the packets it sends, and a CTA that
+// receives a marked packet does the same.
 //
 // Exchange.  A packet is 8 bytes {value, epoch} in one 64-bit store, two per
 // 16-byte access, at the pixel's place in a plane of packets: the reader
@@ -195,7 +196,7 @@ __global__ void __launch_bounds__(W * 32, 1) grid_res_kernel(ResArgs A) {
     using Out = Ring<K, TH, TW>;  // this tile's outermost K pixels
     using In = Ring<K, H, WD>;   // the apron
     constexpr int NU = (In::pairs + NT - 1) / NT, NO = (Out::pairs + NT - 1) / NT;
-    constexpr int NB = NU < 4 ? NU : R >= 12 ? 4 : NU < 9 ? NU : (NU + 1) / 2;  // polled at a time
+    constexpr int NB = R >= 16 ? 4 : NU < 9 ? NU : (NU + 1) / 2;  // polled at a time
     static_assert(NU <= 32, "one bit per pair");
     unsigned need = 0;
     for (int q = 0; q < NU; ++q) {
@@ -215,7 +216,19 @@ __global__ void __launch_bounds__(W * 32, 1) grid_res_kernel(ResArgs A) {
     }
     bool slow = wild;
     for (int done = 0; done < A.sweeps; done += A.period) {
-      if (done > 0 && A.tiles > 1) {
+      // The look for tiny values.  What the apron holds next is looked at by
+      // its senders, who mark it.
+      const auto least = [&] {
+        unsigned v = 0xffffffffu;
+#pragma unroll
+        for (int i = 0; i < R; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) v = min(v, tiny_key(P[i][j]));
+        return v < tiny_limit(kTiny);
+      };
+      if (done == 0 || A.tiles == 1) {
+        slow = __syncthreads_or(least()) || s_wild;
+      } else {
         const int tid = fresh_tid(), ln = tid % LW, st = tid / LW, p = done / K;
         float* const strip = halo + (st * R) * WD + 4 * ln;
         // Warps that hold rows of the ring or of the apron above or below
@@ -230,7 +243,10 @@ __global__ void __launch_bounds__(W * 32, 1) grid_res_kernel(ResArgs A) {
             *reinterpret_cast<float4*>(strip + WD * i) =
                 make_float4(P[i][0], P[i][1], P[i][2], P[i][3]);
         }
-        __syncthreads();
+        if (done % kCheck == 0)
+          slow = __syncthreads_or(least()) || s_wild;
+        else
+          __syncthreads();
         const unsigned want = (s_base + 1 + p) << 1, e = want | (slow ? 1u : 0u);
         const int tl = blockIdx.x / 3, tr = tl / A.tiles_x;
         unsigned long long* out = A.packets + ((p & 1) * 3 + (int)(blockIdx.x - 3 * tl)) * G.plane +
@@ -272,7 +288,7 @@ __global__ void __launch_bounds__(W * 32, 1) grid_res_kernel(ResArgs A) {
             }
           }
         }
-        slow = __syncthreads_or(marks & 1u) || (slow && done % kCheck != 0) || s_wild;
+        slow = __syncthreads_or(marks & 1u) || slow;
         if (s_stop) break;
         // The apron into the strips: whole strips at the sides, and in the
         // first and last warps (whose other pixels were staged above).
@@ -287,22 +303,15 @@ __global__ void __launch_bounds__(W * 32, 1) grid_res_kernel(ResArgs A) {
           }
         }
       }
-      if (done % kCheck == 0) {
-        unsigned least = 0xffffffffu;
-#pragma unroll
-        for (int i = 0; i < R; ++i)
-#pragma unroll
-          for (int j = 0; j < 4; ++j) least = min(least, tiny_key(P[i][j]));
-        const bool tiny = __syncthreads_or(least < tiny_limit(kTiny));
-        slow = tiny || s_wild || (A.tiles > 1 && slow);
-      }
       const int ks = min(A.period, A.sweeps - done);
       int s = 0;
-      if (!slow) {
+      if (!slow && ks >= 2) {
+        post_edges<R, NS, LW>(P, 0, lane, w, edge);
+        __syncthreads();
 #pragma unroll 1
         for (; s + 2 <= ks; s += 2) {
-          quarter_sweep<R, NS, LW, false, true>(P, Gq, L, 0, lane, w, edge);
-          quarter_sweep<R, NS, LW, false, false>(P, Gq, L, 1, lane, w, edge);
+          quarter_sweep<R, NS, LW, true>(P, Gq, L, 0, lane, w, edge);
+          quarter_sweep<R, NS, LW, false>(P, Gq, L, 1, lane, w, edge);
         }
       }
       // An odd last sweep takes this path too (the same values).
@@ -352,18 +361,18 @@ ResKernel res_make(float many, float one) {
 }
 
 // Depth 8 where a grid fits one tile; with many, a deep apron is cheaper than
-// more exchanges (8 rows x 64 columns: 0.295 us at 16, 0.37 at 8).
+// more exchanges (8 rows x 64 columns: 0.295 us at 16, 0.367 at 8).
 const std::vector<ResKernel>& res_kernels() {
   static const std::vector<ResKernel> v = {
-      res_make<6, 4, 16, 8>(0.332f, 0.143f),    // tiles of 32 x 48
-      res_make<8, 4, 16, 8>(0.370f, 0.165f),    // 48 x 48
-      res_make<8, 8, 32, 8>(0.501f, 0.278f),    // 48 x 112
-      res_make<6, 4, 16, 16>(0.257f, 0.253f),   // 16 x 32
-      res_make<8, 4, 16, 16>(0.296f, 0.222f),   // 32 x 32
-      res_make<8, 8, 16, 16>(0.403f, 0.365f),   // 96 x 32
-      res_make<8, 8, 32, 16>(0.424f, 0.272f),   // 32 x 96
-      res_make<12, 8, 32, 16>(0.564f, 0.382f),  // 64 x 96
-      res_make<16, 8, 32, 16>(0.740f, 0.508f),  // 96 x 96
+      res_make<6, 4, 16, 8>(0.323f, 0.132f),    // tiles of 32 x 48
+      res_make<8, 4, 16, 8>(0.367f, 0.159f),    // 48 x 48
+      res_make<8, 8, 32, 8>(0.488f, 0.263f),    // 48 x 112
+      res_make<6, 4, 16, 16>(0.249f, 0.207f),   // 16 x 32
+      res_make<8, 4, 16, 16>(0.295f, 0.210f),   // 32 x 32
+      res_make<8, 8, 16, 16>(0.403f, 0.351f),   // 96 x 32
+      res_make<8, 8, 32, 16>(0.404f, 0.260f),   // 32 x 96
+      res_make<12, 8, 32, 16>(0.538f, 0.370f),  // 64 x 96
+      res_make<16, 8, 32, 16>(0.715f, 0.492f),  // 96 x 96
   };
   return v;
 }
@@ -422,8 +431,8 @@ ResShape res_named(const char* name, int n, int m) {
 
 // The shape with the least measured time whose tiles fit, one (tile, channel)
 // per SM.  Measured against the tile kernel the tuner picked before, us per
-// sweep: 152x152 0.257 (0.80), 194x194 0.295 (0.71), 251x389 0.403 (0.83),
-// 176x1457 0.564 (0.83).
+// sweep: 152x152 0.249 (0.80), 194x194 0.298 (0.71), 251x389 0.407 (0.83),
+// 176x1457 0.540 (0.83).
 ResShape res_pick(int n, int m) {
   ResShape best{0, 0, 0, 0};
   if ((long long)n * m > (1LL << 21)) return best;  // far more tiles than SMs

@@ -1,5 +1,5 @@
-// The quartered Jacobi sweep on register-resident strips, shared by the
-// resident kernel (grid_res.cu) and the pipelined one (grid_pipe.cu).
+// The quartered Jacobi sweep on register-resident strips, for the resident
+// kernel (grid_res.cu).
 //
 // A pixel's next value is ((((g + up) + down) + left) + right) / 4 in the
 // numpy order.  Scaling by 1/4 commutes with rounding, so with g' = g / 4 it
@@ -39,46 +39,71 @@ constexpr unsigned kNegInf = 0xff800000u;   // g' of an unmasked pixel
 __device__ __forceinline__ unsigned tiny_key(float v) { return 2u * __float_as_uint(v) - 1u; }
 constexpr unsigned tiny_limit(int e) { return 2u * ((127u - e) << 23) - 1u; }  // of 2^-e
 
-// One in-place sweep of the strip P (R rows x 4 columns per thread, region rows
-// w * R on; a strip is LW lanes, half a warp where LW = 16), edge rows through shared memory, columns by shuffles.  FWD visits
-// rows downwards, !FWD upwards, each keeping the old row it just replaced: a
-// forward and a backward sweep leave every row in its registers.
-template <int R, int NS, int LW, bool FULL, bool FWD>
-__device__ __forceinline__ void quarter_sweep(float (&P)[R][4], const float (&Gq)[R][4],
-                                          const float (&L)[FULL ? 1 : R][4], int par, int lane, int w,
-                                          float4 (&edge)[2][2][NS][LW]) {
+// The edge rows of a strip, for its neighbours' next sweep.
+template <int R, int NS, int LW>
+__device__ __forceinline__ void post_edges(const float (&P)[R][4], int par, int lane, int w,
+                                           float4 (&edge)[2][2][NS][LW]) {
   edge[par][0][w][lane] = make_float4(P[0][0], P[0][1], P[0][2], P[0][3]);
   edge[par][1][w][lane] = make_float4(P[R - 1][0], P[R - 1][1], P[R - 1][2], P[R - 1][3]);
-  __syncthreads();
+}
+
+// One in-place sweep of the strip P (R rows x 4 columns per thread, region rows
+// w * R on; a strip is LW lanes, half a warp where LW = 16), edge rows through
+// shared memory, columns by shuffles.  On entry edge[par] holds the strips'
+// edge rows (post_edges and a barrier before the first sweep), on return
+// edge[par ^ 1] the new ones, and all strips have read the old.  FWD visits
+// rows downwards, !FWD upwards, each keeping the old row it just replaced: a
+// forward and a backward sweep leave every row in its registers.  Rows are
+// visited in a circle that passes the edge rows in the middle, so that the
+// neighbours' rows are loaded behind the first rows' work and the new edge
+// rows stored before the last rows' (fully masked region of 8 rows, 4 warps:
+// 302 cycles a sweep against 318 from the top row down; through an mbarrier
+// with arrival and wait apart, 424).
+template <int R, int NS, int LW, bool FWD>
+__device__ __forceinline__ void quarter_sweep(float (&P)[R][4], const float (&Gq)[R][4],
+                                              const float (&L)[R][4], int par, int lane, int w,
+                                              float4 (&edge)[2][2][NS][LW]) {
   const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
   const float4 a4 = w > 0 ? edge[par][1][w - 1][lane] : zero;
   const float4 b4 = w < NS - 1 ? edge[par][0][w + 1][lane] : zero;
   const float a[4] = {a4.x, a4.y, a4.z, a4.w}, b[4] = {b4.x, b4.y, b4.z, b4.w};
-  float keep[4];
+  constexpr int F = FWD ? 2 : R - 3;  // the first row visited
+  float keep[4], first[4];            // the old rows just replaced, and F
 #pragma unroll
-  for (int j = 0; j < 4; ++j) keep[j] = FWD ? a[j] : b[j];
+  for (int j = 0; j < 4; ++j) first[j] = P[F][j];
 #pragma unroll
-  for (int q = 0; q < R; ++q) {
-    const int i = FWD ? q : R - 1 - q;
+  for (int k = 0; k < R; ++k) {
+    const int i = FWD ? (F + k) % R : (F - k + R) % R;
     const float cur[4] = {P[i][0], P[i][1], P[i][2], P[i][3]};
     const float lf = __shfl_up_sync(0xffffffffu, cur[3], 1, LW);
     const float rt = __shfl_down_sync(0xffffffffu, cur[0], 1, LW);
     float t[4];
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
-      t[j] = __fmaf_rn(FWD ? keep[j] : (i > 0 ? P[i > 0 ? i - 1 : 0][j] : a[j]), 0.25f, Gq[i][j]);
+    for (int j = 0; j < 4; ++j) {
+      const float up = i == 0                 ? a[j]
+                       : FWD && k > 0         ? keep[j]
+                       : !FWD && k == R - 1   ? first[j]
+                                              : P[i > 0 ? i - 1 : 0][j];
+      t[j] = __fmaf_rn(up, 0.25f, Gq[i][j]);
+    }
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
-      t[j] = __fmaf_rn(FWD ? (i < R - 1 ? P[i < R - 1 ? i + 1 : i][j] : b[j]) : keep[j], 0.25f, t[j]);
+    for (int j = 0; j < 4; ++j) {
+      const float down = i == R - 1             ? b[j]
+                         : !FWD && k > 0        ? keep[j]
+                         : FWD && k == R - 1    ? first[j]
+                                                : P[i < R - 1 ? i + 1 : i][j];
+      t[j] = __fmaf_rn(down, 0.25f, t[j]);
+    }
 #pragma unroll
     for (int j = 0; j < 4; ++j) t[j] = __fmaf_rn(j > 0 ? cur[j > 0 ? j - 1 : 0] : lf, 0.25f, t[j]);
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       keep[j] = cur[j];
-      const float o = __fmaf_rn(j < 3 ? cur[j < 3 ? j + 1 : 0] : rt, 0.25f, t[j]);
-      P[i][j] = FULL ? o : fmaxf(o, L[FULL ? 0 : i][j]);
+      P[i][j] = fmaxf(__fmaf_rn(j < 3 ? cur[j < 3 ? j + 1 : 0] : rt, 0.25f, t[j]), L[i][j]);
     }
+    if (i == (FWD ? 0 : R - 1)) post_edges<R, NS, LW>(P, par ^ 1, lane, w, edge);
   }
+  __syncthreads();
 }
 
 // The same sweep in the reference's order of operations, for values outside
@@ -88,8 +113,7 @@ template <int R, int NS, int LW, typename On>
 __device__ __forceinline__ void slow_sweep(float (&P)[R][4], const float (&G)[R][4], On on,
                                            float gs, int lane, int w,
                                            float4 (&edge)[2][2][NS][LW]) {
-  edge[0][0][w][lane] = make_float4(P[0][0], P[0][1], P[0][2], P[0][3]);
-  edge[0][1][w][lane] = make_float4(P[R - 1][0], P[R - 1][1], P[R - 1][2], P[R - 1][3]);
+  post_edges<R, NS, LW>(P, 0, lane, w, edge);
   __syncthreads();
   const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
   const float4 a4 = w > 0 ? edge[0][1][w - 1][lane] : zero;
