@@ -7,19 +7,23 @@
 // (a 194x194 grid: 5.6 us per 8-sweep launch, of which ~1.6 us are sweeps):
 // launch, region load and store, tail.  Here that is one exchange, and
 // regions are cut as small as lets every SM hold one.  Per sweep: 194x194
-// 0.298 us (0.71 as launches of 8 sweeps), 251x389 0.407 (0.83), 176x1457
-// 0.540 (0.83).
+// 0.266 us (0.71 as launches of 8 sweeps), 251x389 0.385 (0.83), 176x1457
+// 0.523 (0.83).
 //
 // The update is quarter.cuh's.  Each CTA looks for values below 2^-60 every
 // 16 sweeps, before an exchange if there is one; one that finds some takes slow
 // sweeps until its next look and marks the packets it sends, and a CTA that
 // receives a marked packet does the same.
 //
-// Exchange.  A packet is 8 bytes {value, epoch} in one 64-bit store, two per
-// 16-byte access, at the pixel's place in a plane of packets: the reader
-// polls the packet itself, so data and readiness arrive together (measured
-// one way: 690 cycles, against 1,490 with release and acquire), without a
-// fence, a flag or a barrier on the sender's side.  Two buffers alternate.
+// Exchange.  A packet is 16 bytes, three values and an epoch, in one 128-bit
+// store: the reader polls the packet itself, so data and readiness arrive
+// together (one way 450-850 cycles as the poll falls, against 1,490 with
+// release and acquire), without a fence, a flag or a barrier on the sender's
+// side.  What bounds an exchange is the volume, all CTAs' packets at once:
+// with two values and two epochs in 16 bytes, 194x194 took 0.296 us per sweep
+// instead of 0.266 and 660x660 0.716 instead of 0.645.  A tile's packets lie
+// together, ordered by the parts of its ring
+// that different neighbours read.  Two buffers alternate.
 // Overwriting one is safe: a CTA sends exchange p only after it received
 // every neighbour's exchange p - 1, which that neighbour sent after reading
 // exchange p - 2.  Epochs grow from launch to launch (the last CTA to leave
@@ -48,7 +52,7 @@ struct ResArgs {
   const float* g;
   const float* xin;
   float* xout;
-  unsigned long long* packets;  // [2][3][plane]
+  uint4* packets;  // [2][CTA][packets of a tile]
   unsigned* act;                // [tiles * 3] activity words
   unsigned* ctl;                // [0] epoch base, [1] CTAs that left
   const unsigned* wild;
@@ -61,20 +65,24 @@ struct ResArgs {
 constexpr int kCheck = 16;            // sweeps between range checks
 constexpr int kTiny = 60;     // and their limit, 2^-60: exact for 16 sweeps (quarter.cuh)
 
-__device__ __forceinline__ void st_packets(unsigned long long* p, float a, float b, unsigned e) {
-  const unsigned long long hi = (unsigned long long)e << 32;
-  asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};"
-               :
-               : "l"(p), "l"(hi | __float_as_uint(a)), "l"(hi | __float_as_uint(b))
-               : "memory");
+// 128-bit relaxed accesses are single transactions.
+__device__ __forceinline__ void st_packet(uint4* p, float a, float b, float c, unsigned e) {
+  const unsigned long long lo = __float_as_uint(a) | (unsigned long long)__float_as_uint(b) << 32,
+                           hi = __float_as_uint(c) | (unsigned long long)e << 32;
+  asm volatile(
+      "{ .reg .b128 t; mov.b128 t, {%1, %2}; st.relaxed.gpu.global.b128 [%0], t; }"
+      :
+      : "l"(p), "l"(lo), "l"(hi)
+      : "memory");
 }
 
-__device__ __forceinline__ ulonglong2 ld_packets(const unsigned long long* p) {
+__device__ __forceinline__ ulonglong2 ld_packet(const uint4* p) {
   ulonglong2 v;
-  asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];"
-               : "=l"(v.x), "=l"(v.y)
-               : "l"(p)
-               : "memory");
+  asm volatile(
+      "{ .reg .b128 t; ld.relaxed.gpu.global.b128 t, [%2]; mov.b128 {%0, %1}, t; }"
+      : "=l"(v.x), "=l"(v.y)
+      : "l"(p)
+      : "memory");
   return v;
 }
 
@@ -86,28 +94,50 @@ __device__ __forceinline__ int fresh_tid() {
   return t;
 }
 
-// Pixel pairs of a ring `K` wide inside a region of RH x RW pixels starting
-// at (r0, r0): whole rows at the top and bottom, K columns on either side of
-// the rows between.
-template <int K, int RH, int RW>
+// The ring of a TH x TW tile, its K outermost pixels, cut into the blocks that
+// different neighbours read: three bands of rows (one where TH is K) by three
+// of columns, without the middle.  A block's pixels, row by row, fill packets
+// of three; the last one repeats the last pixel.
+template <int K, int TH, int TW>
 struct Ring {
-  static constexpr int rows = K * RW / 2, side = (RH - 2 * K) * (K / 2);
-  static constexpr int pairs = 2 * rows + 2 * side;
-  // Row and column (relative to the ring's corner) of pair u.
-  static __device__ __forceinline__ void at(int u, int& r, int& c) {
-    if (u < 2 * rows) {
-      const bool low = u >= rows;
-      const int v = low ? u - rows : u;
-      r = v / (RW / 2);
-      c = 2 * (v - r * (RW / 2));
-      if (low) r += RH - K;
-    } else {
-      int v = u - 2 * rows;
-      const bool right = v >= side;
-      if (right) v -= side;
-      r = K + v / (K / 2);
-      c = 2 * (v % (K / 2)) + (right ? RW - K : 0);
+  static constexpr int bands = TH == K ? 1 : 3, last = bands - 1;
+  static_assert((TH == K || TH >= 2 * K) && TW >= 2 * K, "bands");
+  static constexpr int row0(int i) { return i == 0 ? 0 : i == 1 ? K : TH - K; }
+  static constexpr int rows(int i) { return i == 1 ? TH - 2 * K : K; }
+  static constexpr int col0(int j) { return j == 0 ? 0 : j == 1 ? K : TW - K; }
+  static constexpr int cols(int j) { return j == 1 ? TW - 2 * K : K; }
+  static constexpr int count(int i, int j) {  // packets of a block
+    return i == 1 && j == 1 ? 0 : (rows(i) * cols(j) + 2) / 3;
+  }
+  static constexpr int first(int i, int j) {
+    int n = 0;
+    for (int k = 0; k < 3 * i + j; ++k) n += count(k / 3, k % 3);
+    return n;
+  }
+  static constexpr int packets = first(bands - 1, 3);
+  // The block rows [i0, i1) and columns [j0, j1) that the tile to the south
+  // (dy 1), north (-1), east (dx 1) or west of this one reads.
+  static constexpr int i0(int dy) { return dy > 0 ? last : 0; }
+  static constexpr int i1(int dy) { return dy < 0 ? 1 : bands; }
+  static constexpr int j0(int dx) { return dx > 0 ? 2 : 0; }
+  static constexpr int j1(int dx) { return dx < 0 ? 1 : 3; }
+  static constexpr int apron() {  // packets that a tile reads
+    int n = 0;
+    for (int k = 0; k < 9; ++k)
+      for (int i = i0(k / 3 - 1); i < i1(k / 3 - 1) && k != 4; ++i)
+        for (int j = j0(k % 3 - 1); j < j1(k % 3 - 1); ++j) n += count(i, j);
+    return n;
+  }
+  // Places in a region with rows `pitch` apart, of the three pixels of packet u of
+  // block (i, j) of the tile (dy, dx) away; 16 bits each.
+  static __device__ __forceinline__ uint2 places(int i, int j, int u, int dy, int dx, int pitch) {
+    unsigned at[3];
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+      const int l = min(3 * u + q, rows(i) * cols(j) - 1), r = l / cols(j);
+      at[q] = (K + dy * TH + row0(i) + r) * pitch + K + dx * TW + col0(j) + l - r * cols(j);
     }
+    return make_uint2(at[0] | at[1] << 16, at[2]);
   }
 };
 
@@ -118,19 +148,23 @@ __global__ void __launch_bounds__(W * 32, 1) grid_res_kernel(ResArgs A) {
   __shared__ int s_stop;
   __shared__ unsigned s_base, s_nb;
   __shared__ int s_wild;
-  // [H][WD]: the apron (received, or constant) and the tile's ring (to send).
+  // [H][HP]: the apron (received, or constant) and the tile's ring (to send).
+  // Rows K words further apart than their width put a side block's pixels,
+  // K a row, into consecutive banks.
+  constexpr int HP = WD + K;
   extern __shared__ __align__(16) float halo[];
-  // Per pair of pixels to send (then: to receive) its place in a plane of
-  // packets and in halo[], relative to the region's first pixel.
-  int2* const t_out = reinterpret_cast<int2*>(halo + H * WD);
-  int2* const t_in = t_out + Ring<K, H - 2 * K, WD - 2 * K>::pairs;
-  // Per thread: its apron pairs that a neighbour sends.
-  unsigned* const t_need = reinterpret_cast<unsigned*>(t_in + Ring<K, H, WD>::pairs);
+  // Places in halo[] of the packets to send and to receive, and where the
+  // latter lie (-1: no tile that sends).
+  using Out = Ring<K, H - 2 * K, WD - 2 * K>;
+  constexpr int NP = Out::packets, NI = Out::apron();
+  uint2* const t_out = reinterpret_cast<uint2*>(halo + H * HP);
+  uint2* const t_in = t_out + NP;
+  int* const t_from = reinterpret_cast<int*>(t_in + NI);
   const GridGeom& G = A.G;
   const int lane = threadIdx.x % LW, w = threadIdx.x / LW;  // place in the strip, strip
   constexpr int KL = K / 4;  // apron lanes
   constexpr int TH = H - 2 * K, TW = WD - 2 * K;
-  static_assert(TH >= K && TW >= K && K % 4 == 0 && K <= kCheck && kCheck % K == 0, "rings and aprons");
+  static_assert(H * HP <= 65536 && K % 4 == 0 && K <= kCheck && kCheck % K == 0, "places and periods");
   const int tile = blockIdx.x / 3, c = blockIdx.x - 3 * tile;
   const int ty = tile / A.tiles_x, tx = tile - ty * A.tiles_x;
   const long long org = G.at(ty * TH - K, tx * TW - K);  // the region's first pixel
@@ -162,7 +196,7 @@ __global__ void __launch_bounds__(W * 32, 1) grid_res_kernel(ResArgs A) {
       Gq[i][j] = on ? (wild ? gv[j] : __fmul_rn(gv[j], 0.25f)) : __uint_as_float(kNegInf);
     }
     // Apron pixels nobody sends keep these values.
-    if (r < K || r >= H - K || !core_lane) *reinterpret_cast<float4*>(halo + r * WD + 4 * lane) = x4;
+    if (r < K || r >= H - K || !core_lane) *reinterpret_cast<float4*>(halo + r * HP + 4 * lane) = x4;
   }
   const bool active = __syncthreads_or(mine);
   const unsigned ebase = s_base;
@@ -193,26 +227,33 @@ __global__ void __launch_bounds__(W * 32, 1) grid_res_kernel(ResArgs A) {
   __syncthreads();
   if (active && !s_stop) {
     const unsigned nb = s_nb;
-    using Out = Ring<K, TH, TW>;  // this tile's outermost K pixels
-    using In = Ring<K, H, WD>;   // the apron
-    constexpr int NU = (In::pairs + NT - 1) / NT, NO = (Out::pairs + NT - 1) / NT;
-    constexpr int NB = R >= 16 ? 4 : NU < 9 ? NU : (NU + 1) / 2;  // polled at a time
-    static_assert(NU <= 32, "one bit per pair");
-    unsigned need = 0;
-    for (int q = 0; q < NU; ++q) {
-      const int u = threadIdx.x + q * NT;
-      if (u >= In::pairs) break;
-      int r, cc;
-      In::at(u, r, cc);
-      const int k = (r < K ? 0 : r >= H - K ? 6 : 3) + (cc < K ? 0 : cc >= WD - K ? 2 : 1);
-      if ((nb >> k) & 1u) need |= 1u << q;
-      t_in[u] = make_int2(r * G.pitch + cc, r * WD + cc);
-    }
-    t_need[threadIdx.x] = need;
-    for (int u = threadIdx.x; u < Out::pairs; u += NT) {
-      int r, cc;
-      Out::at(u, r, cc);
-      t_out[u] = make_int2((r + K) * G.pitch + cc + K, (r + K) * WD + cc + K);
+    constexpr int NU = (NI + NT - 1) / NT, NO = (NP + NT - 1) / NT;
+    constexpr int NB = R < 16 || NU < 6 ? NU : (NU + 1) / 2;  // polled at a time
+    if (A.tiles > 1) {
+#pragma unroll
+      for (int i = 0; i < Out::bands; ++i)
+#pragma unroll
+        for (int j = 0; j < 3; ++j)
+          for (int u = threadIdx.x; u < Out::count(i, j); u += NT)
+            t_out[Out::first(i, j) + u] = Out::places(i, j, u, 0, 0, HP);
+      int n = 0;
+#pragma unroll
+      for (int k = 0; k < 9; ++k) {
+        const int dy = k / 3 - 1, dx = k % 3 - 1;
+        if (k == 4) continue;
+        // The neighbour at (dy, dx) is read where it faces this tile.
+        const int from = (nb >> k) & 1u ? (((int)blockIdx.x + 3 * (dy * A.tiles_x + dx)) * NP) : -1;
+#pragma unroll
+        for (int i = Out::i0(-dy); i < Out::i1(-dy); ++i)
+#pragma unroll
+          for (int j = Out::j0(-dx); j < Out::j1(-dx); ++j) {
+            for (int u = threadIdx.x; u < Out::count(i, j); u += NT) {
+              t_in[n + u] = Out::places(i, j, u, dy, dx, HP);
+              t_from[n + u] = from < 0 ? -1 : from + Out::first(i, j) + u;
+            }
+            n += Out::count(i, j);
+          }
+      }
     }
     bool slow = wild;
     for (int done = 0; done < A.sweeps; done += A.period) {
@@ -230,17 +271,15 @@ __global__ void __launch_bounds__(W * 32, 1) grid_res_kernel(ResArgs A) {
         slow = __syncthreads_or(least()) || s_wild;
       } else {
         const int tid = fresh_tid(), ln = tid % LW, st = tid / LW, p = done / K;
-        float* const strip = halo + (st * R) * WD + 4 * ln;
-        // Warps that hold rows of the ring or of the apron above or below
-        // stage (and reload) their whole strip.
-        const bool apron_strip = st * R < K || (st + 1) * R > H - K;
-        const bool ring_strip = st * R < 2 * K || (st + 1) * R > H - 2 * K;
+        float* const strip = halo + (st * R) * HP + 4 * ln;
         // Send the ring (state after `done` sweeps), through shared memory:
         // from registers it would be R rows of mostly idle stores.
-        if (ring_strip || ln < 2 * KL || ln >= LW - 2 * KL) {
+        const bool side_out = ln < 2 * KL || ln >= LW - 2 * KL, side_in = ln < KL || ln >= LW - KL;
 #pragma unroll
-          for (int i = 0; i < R; ++i)
-            *reinterpret_cast<float4*>(strip + WD * i) =
+        for (int i = 0; i < R; ++i) {
+          const int r = st * R + i;
+          if (side_out || r < 2 * K || r >= H - 2 * K)
+            *reinterpret_cast<float4*>(strip + HP * i) =
                 make_float4(P[i][0], P[i][1], P[i][2], P[i][3]);
         }
         if (done % kCheck == 0)
@@ -249,35 +288,42 @@ __global__ void __launch_bounds__(W * 32, 1) grid_res_kernel(ResArgs A) {
           __syncthreads();
         const unsigned want = (s_base + 1 + p) << 1, e = want | (slow ? 1u : 0u);
         const int tl = blockIdx.x / 3, tr = tl / A.tiles_x;
-        unsigned long long* out = A.packets + ((p & 1) * 3 + (int)(blockIdx.x - 3 * tl)) * G.plane +
-                                  G.at(tr * TH - K, (tl - tr * A.tiles_x) * TW - K);
+        uint4* const buf = A.packets + (size_t)((p & 1) * gridDim.x) * NP;
 #pragma unroll
         for (int q = 0; q < NO; ++q)
-          if ((q + 1) * NT <= Out::pairs || tid + q * NT < Out::pairs) {
-            const int2 t = t_out[tid + q * NT];
-            const float2 v = *reinterpret_cast<const float2*>(halo + t.y);
-            st_packets(out + t.x, v.x, v.y, e);
+          if ((q + 1) * NT <= NP || tid + q * NT < NP) {
+            const uint2 t = t_out[tid + q * NT];
+            st_packet(buf + (size_t)blockIdx.x * NP + tid + q * NT, halo[t.x & 0xffffu],
+                      halo[t.x >> 16], halo[t.y], e);
           }
         // Receive the neighbours' rings into the apron.
         unsigned marks = 0;
 #pragma unroll 1
         for (int q0 = 0; q0 < NU; q0 += NB) {
-          unsigned pend = (t_need[tid] >> q0) & ((1u << NB) - 1u);
-          const int2* t = t_in + tid + q0 * NT;
+          const uint2* t = t_in + tid + q0 * NT;
+          int from[NB];
+          unsigned pend = 0;
+#pragma unroll
+          for (int q = 0; q < NB; ++q) {
+            from[q] = tid + (q0 + q) * NT < NI ? t_from[tid + (q0 + q) * NT] : -1;
+            if (from[q] >= 0) pend |= 1u << q;
+          }
           for (long long spins = 0; pend; ++spins) {
             ulonglong2 v[NB];
 #pragma unroll
             for (int q = 0; q < NB; ++q)
-              if ((pend >> q) & 1u) v[q] = ld_packets(out + t[q * NT].x);
+              if ((pend >> q) & 1u) v[q] = ld_packet(buf + from[q]);
 #pragma unroll
             for (int q = 0; q < NB; ++q)
               if ((pend >> q) & 1u) {
-                const unsigned ea = (unsigned)(v[q].x >> 32), eb = (unsigned)(v[q].y >> 32);
-                if (((ea ^ want) | (eb ^ want)) <= 1u) {
+                const unsigned ev = (unsigned)(v[q].y >> 32);
+                if ((ev ^ want) <= 1u) {
                   pend &= ~(1u << q);
-                  marks |= ea | eb;
-                  *reinterpret_cast<float2*>(halo + t[q * NT].y) =
-                      make_float2(__uint_as_float((unsigned)v[q].x), __uint_as_float((unsigned)v[q].y));
+                  marks |= ev;
+                  const uint2 at = t[q * NT];
+                  halo[at.x & 0xffffu] = __uint_as_float((unsigned)v[q].x);
+                  halo[at.x >> 16] = __uint_as_float((unsigned)(v[q].x >> 32));
+                  halo[at.y] = __uint_as_float((unsigned)v[q].y);
                 }
               }
             if (pend && (spins >= A.spin_limit || ((spins & 63) == 63 && *(volatile int*)A.error))) {
@@ -290,12 +336,12 @@ __global__ void __launch_bounds__(W * 32, 1) grid_res_kernel(ResArgs A) {
         }
         slow = __syncthreads_or(marks & 1u) || slow;
         if (s_stop) break;
-        // The apron into the strips: whole strips at the sides, and in the
-        // first and last warps (whose other pixels were staged above).
-        if (apron_strip || ln < KL || ln >= LW - KL) {
+        // The apron into the strips.
 #pragma unroll
-          for (int i = 0; i < R; ++i) {
-            const float4 v = *reinterpret_cast<const float4*>(strip + WD * i);
+        for (int i = 0; i < R; ++i) {
+          const int r = st * R + i;
+          if (side_in || r < K || r >= H - K) {
+            const float4 v = *reinterpret_cast<const float4*>(strip + HP * i);
             P[i][0] = v.x;
             P[i][1] = v.y;
             P[i][2] = v.z;
@@ -361,18 +407,18 @@ ResKernel res_make(float many, float one) {
 }
 
 // Depth 8 where a grid fits one tile; with many, a deep apron is cheaper than
-// more exchanges (8 rows x 64 columns: 0.295 us at 16, 0.367 at 8).
+// more exchanges (8 rows x 64 columns: 0.266 us at 16, 0.345 at 8).
 const std::vector<ResKernel>& res_kernels() {
   static const std::vector<ResKernel> v = {
-      res_make<6, 4, 16, 8>(0.323f, 0.132f),    // tiles of 32 x 48
-      res_make<8, 4, 16, 8>(0.367f, 0.159f),    // 48 x 48
-      res_make<8, 8, 32, 8>(0.488f, 0.263f),    // 48 x 112
-      res_make<6, 4, 16, 16>(0.249f, 0.207f),   // 16 x 32
-      res_make<8, 4, 16, 16>(0.295f, 0.210f),   // 32 x 32
-      res_make<8, 8, 16, 16>(0.403f, 0.351f),   // 96 x 32
-      res_make<8, 8, 32, 16>(0.404f, 0.260f),   // 32 x 96
-      res_make<12, 8, 32, 16>(0.538f, 0.370f),  // 64 x 96
-      res_make<16, 8, 32, 16>(0.715f, 0.492f),  // 96 x 96
+      res_make<6, 4, 16, 8>(0.310f, 0.130f),    // tiles of 32 x 48
+      res_make<8, 4, 16, 8>(0.345f, 0.160f),    // 48 x 48
+      res_make<8, 8, 32, 8>(0.461f, 0.260f),    // 48 x 112
+      res_make<6, 4, 16, 16>(0.220f, 0.200f),   // 16 x 32
+      res_make<8, 4, 16, 16>(0.266f, 0.214f),   // 32 x 32
+      res_make<8, 8, 16, 16>(0.383f, 0.344f),   // 96 x 32
+      res_make<8, 8, 32, 16>(0.385f, 0.265f),   // 32 x 96
+      res_make<12, 8, 32, 16>(0.523f, 0.374f),  // 64 x 96
+      res_make<16, 8, 32, 16>(0.645f, 0.495f),  // 96 x 96
   };
   return v;
 }
@@ -383,11 +429,22 @@ const ResKernel* res_kernel(const ResShape& s) {
   return nullptr;
 }
 
-// halo[] and the two tables.
+// Packets of a tile, and of its apron (Ring's counts).
+int res_ring(const ResShape& s, bool apron) {
+  const int h = s.tile_h(), w = s.tile_w(), k = s.depth;
+  const auto n = [](int px) { return (px + 2) / 3; };
+  const int corner = n(k * k), row = n(k * (w - 2 * k));
+  const bool one = h == k;  // a single band of rows
+  const int col = one ? 0 : n((h - 2 * k) * k), corners = one ? 2 : 4, sides = one ? 1 : 2;
+  if (!apron) return corners * corner + sides * row + 2 * col;
+  // North and south, west and east, and the corners.
+  return 2 * (2 * corner + row) + 2 * (corners / 2 * corner + col) + 4 * corner;
+}
+
+// halo[] and the tables.
 size_t res_smem(const ResShape& s) {
-  const size_t h = s.region_h(), w = s.width, k = s.depth;
-  const size_t in = w * k + (h - 2 * k) * k, out = (w - 2 * k) * k + (h - 4 * k) * k;
-  return h * w * sizeof(float) + (in + out) * sizeof(int2) + s.warps * 32 * sizeof(unsigned);
+  return (size_t)s.region_h() * (s.width + s.depth) * sizeof(float) + res_ring(s, false) * sizeof(uint2) +
+         res_ring(s, true) * (sizeof(uint2) + sizeof(int));
 }
 
 // SMs of the current device; the kernels' shared-memory limit is raised on
@@ -431,8 +488,8 @@ ResShape res_named(const char* name, int n, int m) {
 
 // The shape with the least measured time whose tiles fit, one (tile, channel)
 // per SM.  Measured against the tile kernel the tuner picked before, us per
-// sweep: 152x152 0.249 (0.80), 194x194 0.298 (0.71), 251x389 0.407 (0.83),
-// 176x1457 0.540 (0.83).
+// sweep: 152x152 0.220 (0.80), 194x194 0.266 (0.71), 251x389 0.385 (0.83),
+// 176x1457 0.523 (0.83).
 ResShape res_pick(int n, int m) {
   ResShape best{0, 0, 0, 0};
   if ((long long)n * m > (1LL << 21)) return best;  // far more tiles than SMs
@@ -450,9 +507,16 @@ ResShape res_pick(int n, int m) {
   return best;
 }
 
-// Packets of three channels, two buffers, then an activity word per SM.
+// The activity words, and two buffers of packets of the shape that needs most.
 size_t res_exchange_bytes(const GridGeom& G) {
-  return (size_t)G.plane * 6 * sizeof(unsigned long long) + 4096;
+  size_t most = 0;
+  if ((long long)G.n * G.m <= (1LL << 21))
+    for (const ResKernel& k : res_kernels()) {
+      const int tiles = res_tiles(k.shape, G.n, G.m);
+      if (tiles > 1 && 3 * tiles <= res_sms())
+        most = std::max(most, (size_t)2 * 3 * tiles * res_ring(k.shape, false) * sizeof(uint4));
+    }
+  return most + 4096;
 }
 
 void launch_res(const GridGeom& G, const ResShape& s, const uint8_t* mask, const float* g,
@@ -465,8 +529,9 @@ void launch_res(const GridGeom& G, const ResShape& s, const uint8_t* mask, const
   const int tiles = res_tiles(s, G.n, G.m);
   FPIE_REQUIRE(3 * tiles <= res_sms() && 3 * tiles <= 1024, FPIE_ERR_STATE,
                "resident kernel: more tiles than SMs");
-  unsigned long long* packets = static_cast<unsigned long long*>(exchange);
-  unsigned* act = reinterpret_cast<unsigned*>(packets + 6 * G.plane);
+  // The activity words first: their place does not depend on the shape.
+  unsigned* act = static_cast<unsigned*>(exchange);
+  uint4* packets = reinterpret_cast<uint4*>(static_cast<char*>(exchange) + 4096);
   ResArgs a{G,    mask,       g,       xin,
             xout, packets,    act,     ctl,
             wild, error,      std::min(spin_limit, 1LL << 23),

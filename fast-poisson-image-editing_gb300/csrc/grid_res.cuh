@@ -29,9 +29,9 @@ ResShape res_pick(int n, int m);
 ResShape res_named(const char* name, int n, int m);
 bool res_is_name(const char* name);
 
-// Device memory of an exchange over geometry G: the packets of every pixel
-// (two buffers, 8 bytes per pixel and channel) and the activity words;
-// must be zero before the first launch.  ctl: kResCtl words, zero before the
+// Device memory of an exchange over geometry G: two buffers of packets for
+// any shape that fits, and the activity words; must be zero before the first
+// launch.  ctl: kResCtl words, zero before the
 // first launch.
 size_t res_exchange_bytes(const GridGeom& G);
 constexpr int kResCtl = 4;
