@@ -141,9 +141,11 @@ def kernel_shape(kernel: str, sweeps: int):
     grid sweep kernel, from its name: "sweep1"; "p<R>w<W>k<K>[t]" (K sweeps
     per launch); "p16w8k16d" / "p16w8k12d" (and their "dp" forms) /
     "rb16w8k8d" (dependency flow: the whole step in one launch, a pass per
-    level)."""
+    level); "p<R>w<W>x<width>k<K>r" (resident: one launch, one pass)."""
     if kernel == "sweep1":
         return 1, sweeps, 1
+    if kernel.endswith("r"):
+        return sweeps, 1, 1
     depth = int(re.search(r"k(\d+)", kernel).group(1))
     if re.search(r"k\d+dp?$", kernel):
         return sweeps, 1, -(-sweeps // depth)
@@ -155,15 +157,16 @@ FP32_OPS_PER_UPDATE = 15  # per pixel update: 4 additions + 1 multiplication, 3 
 
 def apron_factor(kernel: str) -> float:
     """Region pixels a temporally blocked kernel sweeps per tile pixel it
-    writes: regions are W*R rows x 128 columns, tiles lose K pixels (2K for
-    red-black levels) on every side; 1 for the one-sweep kernel."""
-    m = re.match(r"(rb|p)(\d+)w(\d+)k(\d+)", kernel)
+    writes: regions are W*R rows x 128 columns (or as wide as named, with as
+    many pixels), tiles lose K pixels (2K for red-black levels) on every side;
+    1 for the one-sweep kernel."""
+    m = re.match(r"(rb|p)(\d+)w(\d+)(?:x(\d+))?k(\d+)", kernel)
     if not m:
         return 1.0
-    r, w, k = (int(v) for v in m.groups()[1:])
+    r, w, width, k = (int(v or 128) for v in m.groups()[1:])
     k = 2 * k if m.group(1) == "rb" else k
-    rows = r * w
-    return rows * 128 / ((rows - 2 * k) * (128 - 2 * k))
+    rows = r * w * 128 // width
+    return rows * width / ((rows - 2 * k) * (width - 2 * k))
 
 
 def fp32_peaks(stream_handle: int) -> dict:
@@ -1012,7 +1015,7 @@ def run_gb300(args):
         out_img2, _ = img_solver.step(sweeps)
     e2e_img_dt = (time.perf_counter() - t0) / e2e_steps
 
-    kernel = s.kernel
+    kernel = s.resident or s.kernel
     per_launch, launches_per_step, passes = kernel_shape(kernel, sweeps)
     avg_launch_s = sweep_ms / 1e3 / (args.steps * launches_per_step)
     peaks = fp32_peaks(stream.cuda_stream)

@@ -407,7 +407,8 @@ ResKernel res_make(float many, float one) {
 }
 
 // Depth 8 where a grid fits one tile; with many, a deep apron is cheaper than
-// more exchanges (8 rows x 64 columns: 0.266 us at 16, 0.345 at 8).
+// more exchanges (8 rows x 64 columns: 0.266 us at 16, 0.345 at 8).  Depth 4
+// for the largest tiles, where deeper ones would not fit on the SMs.
 const std::vector<ResKernel>& res_kernels() {
   static const std::vector<ResKernel> v = {
       res_make<6, 4, 16, 8>(0.310f, 0.130f),    // tiles of 32 x 48
@@ -419,6 +420,7 @@ const std::vector<ResKernel>& res_kernels() {
       res_make<8, 8, 32, 16>(0.385f, 0.265f),   // 32 x 96
       res_make<12, 8, 32, 16>(0.523f, 0.374f),  // 64 x 96
       res_make<16, 8, 32, 16>(0.645f, 0.495f),  // 96 x 96
+      res_make<16, 8, 32, 4>(0.925f, 0.500f),   // 120 x 120
   };
   return v;
 }
@@ -489,7 +491,10 @@ ResShape res_named(const char* name, int n, int m) {
 // The shape with the least measured time whose tiles fit, one (tile, channel)
 // per SM.  Measured against the tile kernel the tuner picked before, us per
 // sweep: 152x152 0.220 (0.80), 194x194 0.266 (0.71), 251x389 0.385 (0.83),
-// 176x1457 0.523 (0.83).
+// 176x1457 0.523 (0.83).  The depth-4 shape runs at 0.92-0.94 at any size,
+// the flow kernel according to its 96x96 tiles: with 64 of them or fewer
+// (680x680 to 760x760, 600x840) at 0.89-0.96, with more (803x803, 600x1080,
+// 240x2400) at 0.95-1.15; so it is taken above 64.
 ResShape res_pick(int n, int m) {
   ResShape best{0, 0, 0, 0};
   if ((long long)n * m > (1LL << 21)) return best;  // far more tiles than SMs
@@ -498,6 +503,7 @@ ResShape res_pick(int n, int m) {
   for (const ResKernel& k : res_kernels()) {
     const int tiles = res_tiles(k.shape, n, m);
     if (3 * tiles > sms) continue;
+    if (k.shape.depth == 4 && ((n + 95) / 96) * ((m + 95) / 96) <= 64) continue;
     const float t = tiles > 1 ? k.many : k.one;
     if (t < least) {
       least = t;

@@ -22,6 +22,7 @@ SHAPES = {  # name: (tile rows, tile columns)
     "p6w4x64k8r": (32, 48), "p8w4x64k8r": (48, 48), "p8w8x128k8r": (48, 112),
     "p6w4x64k16r": (16, 32), "p8w4x64k16r": (32, 32), "p8w8x64k16r": (96, 32),
     "p8w8x128k16r": (32, 96), "p12w8x128k16r": (64, 96), "p16w8x128k16r": (96, 96),
+    "p16w8x128k4r": (120, 120),
 }
 
 
@@ -68,6 +69,18 @@ def test_rule_picks_a_resident_kernel(size):
     s.reset(mask.size, mask, tgt, grad)
     assert s.resident in SHAPES
     _compare(s, cjacobi.CGrid(mask, tgt, grad), (33, 100))
+
+
+@pytest.mark.parametrize("size,deep4", [((768, 768), False), ((769, 673), True), ((840, 840), True),
+                                        ((841, 840), False), ((97, 2592), False), ((193, 2305), True)])
+def test_depth_4_above_64_tiles_of_the_flow_kernel(size, deep4):
+    from fpie_gb300 import backend
+
+    mask, tgt, grad = _inputs(*size, 5)
+    s = backend.GridSolver(8, 8)
+    s.reset(mask.size, mask, tgt, grad)
+    assert (s.resident == "p16w8x128k4r") == deep4
+    _compare(s, cjacobi.CGrid(mask, tgt, grad), (33,))
 
 
 def test_inactive_tiles_and_new_masks():
