@@ -420,9 +420,11 @@ struct GridSolverImpl : Solver {
       flags_ok = false;  // the new mask may activate other tiles
       mflags_ok = false;
       ft_ok = false;
+      untuned_sweeps = 0;
       return;
     }
     release();
+    untuned_sweeps = 0;
     if (!pinned) tuned = false;
     G = make_geom(n, m);
     L = grid_launch(G);
@@ -607,6 +609,22 @@ struct GridSolverImpl : Solver {
     for (size_t k = 0; k < tb_variants().size(); ++k)
       if (std::string(tb_variants()[k].name) == "p16w8k16") return (int)k;
     return 0;
+  }
+
+  // Steps too short to tune on.  The flow kernel's tables cost 25 us (902x902)
+  // to 65 us (1800x1800) after a reset, its sweeps less than the launches';
+  // us for 100, 200, 400 sweeps from a reset, launches against flow: disk of
+  // 902x902 175/177, 325/286, 628/511; box of 1100x1100 230/238, 428/405,
+  // 835/743; box of 1800x1800 522/553, 991/1008, 1943/1935; 500x2500 262/255,
+  // 490/436, 952/806 (so from 256 sweeps on).  On larger grids the launches are as fast (2300x2300
+  // 2528/2556) or faster (2900x2900 3865/3945).
+  static constexpr int kFlowFrom = 256;
+  static constexpr long long kFlowPixels = 1800LL * 1800;
+  int untuned_sweeps = 0;  // since the reset, up to kFlowFrom
+  int untuned_variant(int iters) const {
+    return iters >= kFlowFrom - untuned_sweeps && (long long)G.n * G.m <= kFlowPixels
+               ? kFlow12
+               : default_variant();
   }
 
   int depth() const {
@@ -871,6 +889,8 @@ struct GridSolverImpl : Solver {
     FPIE_REQUIRE(res_pin.empty() || red_black, FPIE_ERR_ARG,
                  "the grid's tiles do not fit on the device: no '" + res_pin + "' sweeps");
     if (!tuned && !pinned) iters -= autotune(iters);
+    if (!tuned && !pinned && !red_black) select_variant(untuned_variant(iters));
+    untuned_sweeps += std::min(iters, kFlowFrom - untuned_sweeps);
     if (is_flow(variant)) {
       if (iters > 0) run_flow(iters);
       return;
