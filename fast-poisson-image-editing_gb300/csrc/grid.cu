@@ -603,28 +603,29 @@ struct GridSolverImpl : Solver {
   int flags_cap = 0, tiles_x = 0, tiles = 0;
   bool flags_ok = false;
 
-  // The kernel used before (or without) autotuning: the packed 16-row,
-  // 8-warp, 16-sweep variant, fastest on both benchmark shapes measured.
-  static int default_variant() {
+  static int tb_named(const char* name) {
     for (size_t k = 0; k < tb_variants().size(); ++k)
-      if (std::string(tb_variants()[k].name) == "p16w8k16") return (int)k;
+      if (std::string(tb_variants()[k].name) == name) return (int)k;
     return 0;
   }
+
+  // The kernel before any step.
+  static int default_variant() { return tb_named("p16w8k16"); }
 
   // Steps too short to tune on.  The flow kernel's tables cost 25 us (902x902)
   // to 65 us (1800x1800) after a reset, its sweeps less than the launches';
   // us for 100, 200, 400 sweeps from a reset, launches against flow: disk of
   // 902x902 175/177, 325/286, 628/511; box of 1100x1100 230/238, 428/405,
   // 835/743; box of 1800x1800 522/553, 991/1008, 1943/1935; 500x2500 262/255,
-  // 490/436, 952/806 (so from 256 sweeps on).  On larger grids the launches are as fast (2300x2300
-  // 2528/2556) or faster (2900x2900 3865/3945).
+  // 490/436, 952/806 (so from 256 sweeps on).  On larger grids launches of
+  // tall regions are faster (grid_tbp.cu; 2300x2300 disk 2,420/2,556, 2900x2900
+  // 3,550/3,945).
   static constexpr int kFlowFrom = 256;
   static constexpr long long kFlowPixels = 1800LL * 1800;
   int untuned_sweeps = 0;  // since the reset, up to kFlowFrom
   int untuned_variant(int iters) const {
-    return iters >= kFlowFrom - untuned_sweeps && (long long)G.n * G.m <= kFlowPixels
-               ? kFlow12
-               : default_variant();
+    if ((long long)G.n * G.m > kFlowPixels) return tb_named("p22w8k16");
+    return iters >= kFlowFrom - untuned_sweeps ? kFlow12 : default_variant();
   }
 
   int depth() const {
@@ -805,7 +806,7 @@ struct GridSolverImpl : Solver {
     // kernel below (two depths).  sweep1 (one sweep per launch, the baseline) and the TMA
     // kernel stay available by name but were never the fastest on a
     // measured shape; timing them would only lengthen the first step.
-    static const char* const kTuned[] = {"p16w8k16", "p8w16k16", "p16w8k8", "p8w8k8"};
+    static const char* const kTuned[] = {"p16w8k16", "p8w16k16", "p22w8k16", "p8w8k8"};
     std::vector<int> cands;
     for (int v = 0; v < (int)tb_variants().size(); ++v) {
       const TbVariant& tv = tb_variants()[v];

@@ -194,6 +194,12 @@ const std::vector<MixedVariant>& mixed_variants() {
 void append_packed_variants(std::vector<TbVariant>& v) {
   v.push_back(make_packed<16, 8, 8>("p16w8k8"));
   v.push_back(make_packed<16, 8, 16>("p16w8k16"));
+  // Tall regions (176 rows) for large grids: 1.63 region pixels per pixel of
+  // a tile instead of 1.78, and per sweep fewer loads, stores and barriers.
+  // us per sweep, against p16w8k16: 1950x1950 box 5.61 (5.65), disk 4.76
+  // (4.89); 2300x2300 6.73 (7.31), 6.04 (6.25); 3603x3603 disk 12.72 (14.05).
+  // 24 rows a thread spill (13.47); 20 rows 13.19.
+  v.push_back(make_packed<22, 8, 16>("p22w8k16"));
   // Short regions (64 rows) for small grids: twice the tiles of the 128-row
   // variants, so a small paste keeps more SMs busy.
   v.push_back(make_packed<8, 8, 8>("p8w8k8"));

@@ -1,6 +1,7 @@
 """Steps too short for the autotuner: launches at first, the flow kernel once
-256 sweeps have been asked for since the reset; the oracle's states, bit for
-bit, through the change and after a new reset."""
+256 sweeps have been asked for since the reset, and launches of tall regions on
+grids of more than 1800x1800; the oracle's states, bit for bit, through the
+change and after a new reset."""
 
 from __future__ import annotations
 
@@ -29,14 +30,29 @@ def test_kernel_by_the_sweeps_since_the_reset(size, flow):
     from fpie_gb300 import backend
 
     s = backend.GridSolver(8, 8)
-    late = "p16w8k12d" if flow else "p16w8k16"
+    early, late = ("p16w8k16", "p16w8k12d") if flow else ("p22w8k16", "p22w8k16")
     for seed in (1, 2):
         mask, tgt, grad = _inputs(*size, seed)
         s.reset(mask.size, mask, tgt, grad)
         assert s.resident == ""
         o = cjacobi.CGrid(mask, tgt, grad)
-        for k, kernel in ((100, "p16w8k16"), (155, "p16w8k16"), (1, late), (13, late)):
+        for k, kernel in ((100, early), (155, early), (1, late), (13, late)):
             s.step(k)
             o.sweep(k)
             assert s.kernel == kernel
             np.testing.assert_array_equal(s.state(), o.x)
+
+
+@pytest.mark.parametrize("size", [(1, 1), (143, 95), (144, 96), (145, 97), (300, 210)])
+def test_tall_regions_at_their_edges(size):
+    from fpie_gb300 import backend
+
+    mask, tgt, grad = _inputs(*size, 3)
+    s = backend.GridSolver(8, 8)
+    s.set_kernel("p22w8k16")
+    s.reset(mask.size, mask, tgt, grad)
+    o = cjacobi.CGrid(mask, tgt, grad)
+    for k in (1, 15, 16, 64, 37):
+        s.step(k)
+        o.sweep(k)
+        np.testing.assert_array_equal(s.state(), o.x)
