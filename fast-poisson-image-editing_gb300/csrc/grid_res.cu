@@ -62,7 +62,6 @@ struct ResArgs {
   // within tol.  NULL: none.
   const double* maxima;
   double tol;
-  int period;  // sweeps between exchanges (K, or 16 for a single tile)
   int tiles_x, tiles, sweeps;
 };
 
@@ -153,7 +152,10 @@ __device__ __forceinline__ bool res_beyond(const double* maxima, double tol) {
   return (a < m ? m : a) > tol;
 }
 
-template <int R, int W, int LW, int K>
+// WHOLE: the region holds the whole grid.  It needs no apron but a lane on
+// each side, whose zeros are what a grid's border sees beyond it, and no
+// exchange.
+template <int R, int W, int LW, int K, bool WHOLE>
 __global__ void __launch_bounds__(W * 32, 1) grid_res_kernel(ResArgs A) {
   constexpr int NT = W * 32, NS = NT / LW, H = R * NS, WD = 4 * LW;  // strips, region rows and columns
   __shared__ float4 edge[2][2][NS][LW];
@@ -179,7 +181,9 @@ __global__ void __launch_bounds__(W * 32, 1) grid_res_kernel(ResArgs A) {
   static_assert(H * HP <= 65536 && K % 4 == 0 && K <= kCheck && kCheck % K == 0, "places and periods");
   const int tile = blockIdx.x / 3, c = blockIdx.x - 3 * tile;
   const int ty = tile / A.tiles_x, tx = tile - ty * A.tiles_x;
-  const long long org = G.at(ty * TH - K, tx * TW - K);  // the region's first pixel
+  constexpr int ap = WHOLE ? 0 : K, al = WHOLE ? 1 : KL;
+  constexpr int period = WHOLE ? kCheck : K;  // sweeps between exchanges
+  const long long org = G.at(ty * TH - ap, tx * TW - 4 * al);  // the region's first pixel
   const long long base = org + (long long)(w * R) * G.pitch + 4 * lane;
   const long long co = c * G.plane;
   if (threadIdx.x == 0) {
@@ -191,7 +195,7 @@ __global__ void __launch_bounds__(W * 32, 1) grid_res_kernel(ResArgs A) {
   const bool wild = *A.wild != 0;
   float P[R][4], Gq[R][4], L[R][4];
   bool mine = false;  // a masked pixel in the tile interior
-  const bool core_lane = lane >= KL && lane < LW - KL;
+  const bool core_lane = lane >= al && lane < LW - al;
 #pragma unroll
   for (int i = 0; i < R; ++i) {
     const long long p = base + (long long)i * G.pitch;
@@ -199,7 +203,7 @@ __global__ void __launch_bounds__(W * 32, 1) grid_res_kernel(ResArgs A) {
     const float4 g4 = ld4(A.g + co + p);
     const uint32_t mk = __ldg(reinterpret_cast<const unsigned*>(A.mask + p));
     const int r = w * R + i;
-    mine = mine || (mk != 0 && core_lane && r >= K && r < H - K);
+    mine = mine || (mk != 0 && core_lane && r >= ap && r < H - ap);
     const float x[4] = {x4.x, x4.y, x4.z, x4.w}, gv[4] = {g4.x, g4.y, g4.z, g4.w};
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -209,6 +213,7 @@ __global__ void __launch_bounds__(W * 32, 1) grid_res_kernel(ResArgs A) {
       Gq[i][j] = on ? (wild ? gv[j] : __fmul_rn(gv[j], 0.25f)) : __uint_as_float(kNegInf);
     }
     // Apron pixels nobody sends keep these values.
+    if (WHOLE) continue;
     if (r < K || r >= H - K || !core_lane) *reinterpret_cast<float4*>(halo + r * HP + 4 * lane) = x4;
   }
   const bool active = __syncthreads_or(mine);
@@ -220,7 +225,7 @@ __global__ void __launch_bounds__(W * 32, 1) grid_res_kernel(ResArgs A) {
   if (threadIdx.x < 32) {
     const int ny = ty + (int)threadIdx.x / 3 - 1, nx = tx + (int)threadIdx.x % 3 - 1;
     bool on = false;
-    if (active && threadIdx.x < 9 && threadIdx.x != 4 && ny >= 0 && nx >= 0 && nx < A.tiles_x &&
+    if (!WHOLE && active && threadIdx.x < 9 && threadIdx.x != 4 && ny >= 0 && nx >= 0 && nx < A.tiles_x &&
         ny * A.tiles_x + nx < A.tiles) {
       const volatile unsigned* q = A.act + 3 * (ny * A.tiles_x + nx) + c;
       unsigned v = *q;
@@ -243,7 +248,7 @@ __global__ void __launch_bounds__(W * 32, 1) grid_res_kernel(ResArgs A) {
     const unsigned nb = s_nb;
     constexpr int NU = (NI + NT - 1) / NT, NO = (NP + NT - 1) / NT;
     constexpr int NB = R < 16 || NU < 6 ? NU : (NU + 1) / 2;  // polled at a time
-    if (A.tiles > 1) {
+    if constexpr (!WHOLE) {
 #pragma unroll
       for (int i = 0; i < Out::bands; ++i)
 #pragma unroll
@@ -270,7 +275,7 @@ __global__ void __launch_bounds__(W * 32, 1) grid_res_kernel(ResArgs A) {
       }
     }
     bool slow = wild;
-    for (int done = 0; done < A.sweeps; done += A.period) {
+    for (int done = 0; done < A.sweeps; done += period) {
       // The look for tiny values.  What the apron holds next is looked at by
       // its senders, who mark it.
       const auto least = [&] {
@@ -281,9 +286,9 @@ __global__ void __launch_bounds__(W * 32, 1) grid_res_kernel(ResArgs A) {
           for (int j = 0; j < 4; ++j) v = min(v, tiny_key(P[i][j]));
         return v < tiny_limit(kTiny);
       };
-      if (done == 0 || A.tiles == 1) {
+      if (WHOLE || done == 0) {
         slow = __syncthreads_or(least()) || s_wild;
-      } else {
+      } else if constexpr (!WHOLE) {
         const int tid = fresh_tid(), ln = tid % LW, st = tid / LW, p = done / K;
         float* const strip = halo + (st * R) * HP + 4 * ln;
         // Send the ring (state after `done` sweeps), through shared memory:
@@ -301,7 +306,6 @@ __global__ void __launch_bounds__(W * 32, 1) grid_res_kernel(ResArgs A) {
         else
           __syncthreads();
         const unsigned want = (s_base + 1 + p) << 1, e = want | (slow ? 1u : 0u);
-        const int tl = blockIdx.x / 3, tr = tl / A.tiles_x;
         uint4* const buf = A.packets + (size_t)((p & 1) * gridDim.x) * NP;
 #pragma unroll
         for (int q = 0; q < NO; ++q)
@@ -363,7 +367,7 @@ __global__ void __launch_bounds__(W * 32, 1) grid_res_kernel(ResArgs A) {
           }
         }
       }
-      const int ks = min(A.period, A.sweeps - done);
+      const int ks = min(period, A.sweeps - done);
       int s = 0;
       if (!slow && ks >= 2) {
         post_edges<R, NS, LW>(P, 0, lane, w, edge);
@@ -382,14 +386,14 @@ __global__ void __launch_bounds__(W * 32, 1) grid_res_kernel(ResArgs A) {
             s_wild ? 1.f : 4.f, lane, w, edge);
     }
     const int tid = fresh_tid(), ln = tid % LW, st = tid / LW;
-    if (ln >= KL && ln < LW - KL) {
+    if (ln >= al && ln < LW - al) {
       const int tl = blockIdx.x / 3, tr = tl / A.tiles_x;
       float* const o = A.xout + (int)(blockIdx.x - 3 * tl) * G.plane +
-                       G.at(tr * TH - K + st * R, (tl - tr * A.tiles_x) * TW - K + 4 * ln);
+                       G.at(tr * TH - ap + st * R, (tl - tr * A.tiles_x) * TW - 4 * al + 4 * ln);
 #pragma unroll
       for (int i = 0; i < R; ++i) {
         const int r = st * R + i;
-        if (r >= K && r < H - K)
+        if (r >= ap && r < H - ap)
           *reinterpret_cast<float4*>(o + (long long)i * G.pitch) =
               make_float4(P[i][0], P[i][1], P[i][2], P[i][3]);
       }
@@ -401,7 +405,7 @@ __global__ void __launch_bounds__(W * 32, 1) grid_res_kernel(ResArgs A) {
     __threadfence();
     if (atomicAdd(A.ctl + 1, 1u) == gridDim.x - 1) {
       A.ctl[1] = 0;
-      A.ctl[0] = s_base + 2u + (unsigned)((A.sweeps + A.period - 1) / A.period);
+      A.ctl[0] = s_base + 2u + (unsigned)((A.sweeps + period - 1) / period);
     }
   }
 }
@@ -412,29 +416,33 @@ struct ResKernel {
   // the whole grid in one tile (no exchange).  Neither depends on the grid:
   // every CTA does the same work, whatever their number.
   float many, one;
-  const void* kernel;
+  const void *kernel, *whole;
 };
 
 template <int R, int W, int LW, int K>
 ResKernel res_make(float many, float one) {
-  return {{R, W, 4 * LW, K}, many, one, (const void*)grid_res_kernel<R, W, LW, K>};
+  return {{R, W, 4 * LW, K},
+          many,
+          one,
+          (const void*)grid_res_kernel<R, W, LW, K, false>,
+          (const void*)grid_res_kernel<R, W, LW, 8, true>};
 }
 
-// Depth 8 where a grid fits one tile; with many, a deep apron is cheaper than
+// Depth 8 or 16 where a grid fits one region; with many tiles, a deep apron is cheaper than
 // more exchanges (8 rows x 64 columns: 0.266 us at 16, 0.345 at 8).  Depth 4
 // for the largest tiles, where deeper ones would not fit on the SMs.
 const std::vector<ResKernel>& res_kernels() {
   static const std::vector<ResKernel> v = {
-      res_make<6, 4, 16, 8>(0.310f, 0.130f),    // tiles of 32 x 48
-      res_make<8, 4, 16, 8>(0.345f, 0.160f),    // 48 x 48
-      res_make<8, 8, 32, 8>(0.461f, 0.260f),    // 48 x 112
-      res_make<6, 4, 16, 16>(0.220f, 0.200f),   // 16 x 32
-      res_make<8, 4, 16, 16>(0.266f, 0.214f),   // 32 x 32
-      res_make<8, 8, 16, 16>(0.383f, 0.344f),   // 96 x 32
-      res_make<8, 8, 32, 16>(0.385f, 0.265f),   // 32 x 96
-      res_make<12, 8, 32, 16>(0.523f, 0.374f),  // 64 x 96
-      res_make<16, 8, 32, 16>(0.645f, 0.495f),  // 96 x 96
-      res_make<16, 8, 32, 4>(0.925f, 0.500f),   // 120 x 120
+      res_make<6, 4, 16, 8>(0.310f, 0.128f),    // tiles of 32 x 48
+      res_make<8, 4, 16, 8>(0.345f, 0.161f),    // 48 x 48
+      res_make<8, 8, 32, 8>(0.461f, 0.267f),    // 48 x 112
+      res_make<6, 4, 16, 16>(0.220f, 0.128f),   // 16 x 32
+      res_make<8, 4, 16, 16>(0.266f, 0.161f),   // 32 x 32
+      res_make<8, 8, 16, 16>(0.383f, 0.275f),   // 96 x 32
+      res_make<8, 8, 32, 16>(0.385f, 0.267f),   // 32 x 96
+      res_make<12, 8, 32, 16>(0.523f, 0.376f),  // 64 x 96
+      res_make<16, 8, 32, 16>(0.645f, 0.488f),  // 96 x 96
+      res_make<16, 8, 32, 4>(0.925f, 0.490f),   // 120 x 120
   };
   return v;
 }
@@ -479,7 +487,11 @@ int res_sms() {
   return sms;
 }
 
+// One where the grid fits a region: its rows, its columns but a lane on each
+// side (48x64 with an apron of 8 would be tiles of 32x48; 38x38 then takes
+// 0.128 us per sweep instead of 0.161, 64x56 0.160 instead of 0.208).
 int res_tiles(const ResShape& s, int n, int m) {
+  if (n <= s.region_h() && m <= s.width - 8) return 1;
   return ((n + s.tile_h() - 1) / s.tile_h()) * ((m + s.tile_w() - 1) / s.tile_w());
 }
 
@@ -545,8 +557,8 @@ void launch_res(const GridGeom& G, const ResShape& s, const uint8_t* mask, const
                 cudaStream_t st, const double* maxima, double tol) {
   const ResKernel* k = res_kernel(s);
   FPIE_REQUIRE(k != nullptr, FPIE_ERR_STATE, "no such resident kernel");
-  const int tiles_x = (G.m + s.tile_w() - 1) / s.tile_w();
   const int tiles = res_tiles(s, G.n, G.m);
+  const int tiles_x = tiles == 1 ? 1 : (G.m + s.tile_w() - 1) / s.tile_w();
   FPIE_REQUIRE(3 * tiles <= res_sms() && 3 * tiles <= 1024, FPIE_ERR_STATE,
                "resident kernel: more tiles than SMs");
   // The activity words first: their place does not depend on the shape.
@@ -555,10 +567,10 @@ void launch_res(const GridGeom& G, const ResShape& s, const uint8_t* mask, const
   ResArgs a{G,    mask,       g,       xin,
             xout, packets,    act,     ctl,
             wild, error,      std::min(spin_limit, 1LL << 23), maxima, tol,
-            tiles > 1 ? s.depth : kCheck, tiles_x, tiles, sweeps};
+            tiles_x, tiles, sweeps};
   void* args[] = {&a};
-  FPIE_CUDA(cudaLaunchCooperativeKernel(k->kernel, dim3(3 * tiles), dim3(s.warps * 32), args,
-                                        res_smem(s), st));
+  FPIE_CUDA(cudaLaunchCooperativeKernel(tiles > 1 ? k->kernel : k->whole, dim3(3 * tiles),
+                                        dim3(s.warps * 32), args, tiles > 1 ? res_smem(s) : 0, st));
 }
 
 }  // namespace fpie

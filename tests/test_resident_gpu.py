@@ -60,6 +60,24 @@ def test_tile_edges(kernel, extra):
         _compare(s, cjacobi.CGrid(mask, tgt, grad), (1, 16, 7, 8, 100))
 
 
+@pytest.mark.parametrize("kernel", sorted(SHAPES))
+@pytest.mark.parametrize("less", [(0, 0), (1, 3), (0, -1), (-1, 0)])
+def test_a_region_that_holds_the_grid(kernel, less):
+    """Grids as large as a region (all its rows, its columns but a lane on each
+    side), with masked pixels on their borders; and one row or column more."""
+    from fpie_gb300 import backend
+
+    th, tw = SHAPES[kernel]
+    depth = int(kernel.split("k")[1][:-1])
+    mask, tgt, grad = _inputs(th + 2 * depth - less[0], tw + 2 * depth - 8 - less[1], 9)
+    mask[0, ::2] = mask[-1, 1::2] = 1
+    mask[::3, 0] = mask[1::3, -1] = 1
+    s = backend.GridSolver(8, 8)
+    s.set_kernel(kernel)
+    s.reset(mask.size, mask, tgt, grad)
+    _compare(s, cjacobi.CGrid(mask, tgt, grad), (1, 16, 33, 64))
+
+
 @pytest.mark.parametrize("size", [(32, 48), (33, 48), (48, 49), (160, 320), (161, 320), (672, 672)])
 def test_rule_picks_a_resident_kernel(size):
     from fpie_gb300 import backend
