@@ -411,35 +411,22 @@ struct Batch {
   void alloc(BatchJob& j) {
     const size_t pb = (size_t)j.G.plane * sizeof(float), eb = (size_t)j.G.plane * 3 * 2;
     const bool mixed = precision != FPIE_FP32;
-    struct Part {
-      void** p;
-      size_t bytes;
-    };
     // The cleared ones first; err holds the finish kernel's count behind it.
-    const Part parts[] = {{(void**)&j.x[0], 3 * pb},
-                          {(void**)&j.x[1], 3 * pb},
-                          {(void**)&j.g, 3 * pb},
-                          {(void**)&j.mask, (size_t)j.G.plane},
-                          {(void**)&j.err, 4 * sizeof(float)},
-                          {&j.e[0], mixed ? eb : 0},
-                          {&j.e[1], mixed ? eb : 0},
-                          {(void**)&j.r, mixed ? 3 * pb : 0},
-                          {(void**)&j.img, (size_t)j.n * j.m * 3},
-                          {(void**)&j.parts, (size_t)j.L.nparts * 6 * sizeof(double)},
-                          {(void**)&j.norm, 6 * sizeof(double)}};
-    constexpr int cleared = 8;
-    size_t total = 0, clear = 0;
-    for (const Part& p : parts) {
-      if (&p == parts + cleared) clear = total;
-      total += (p.bytes + 255) / 256 * 256;
-    }
-    FPIE_CUDA(cudaMallocFromPoolAsync(&j.block, total, scratch_pool(), stream));
-    size_t off = 0;
-    for (const Part& p : parts) {
-      if (p.bytes) *p.p = static_cast<char*>(j.block) + off;
-      off += (p.bytes + 255) / 256 * 256;
-    }
-    FPIE_CUDA(cudaMemsetAsync(j.block, 0, clear, stream));
+    const DevicePart parts[] = {{&j.x[0], 3 * pb},
+                                {&j.x[1], 3 * pb},
+                                {&j.g, 3 * pb},
+                                {&j.mask, (size_t)j.G.plane},
+                                {&j.err, 4 * sizeof(float)},
+                                {&j.e[0], mixed ? eb : 0},
+                                {&j.e[1], mixed ? eb : 0},
+                                {&j.r, mixed ? 3 * pb : 0},
+                                {&j.img, (size_t)j.n * j.m * 3},
+                                {&j.parts, (size_t)j.L.nparts * 6 * sizeof(double)},
+                                {&j.norm, 6 * sizeof(double)}};
+    const DeviceLayout l = device_layout(parts, 11, 8);
+    FPIE_CUDA(cudaMallocFromPoolAsync(&j.block, l.total, scratch_pool(), stream));
+    device_place(parts, 11, j.block);
+    FPIE_CUDA(cudaMemsetAsync(j.block, 0, l.clear, stream));
   }
 
   int precision = FPIE_FP32;

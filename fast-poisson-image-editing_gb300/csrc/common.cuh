@@ -79,6 +79,31 @@ struct AsyncScratch {
   char* bytes() const { return static_cast<char*>(ptr); }
 };
 
+// Arrays that live in one device block, each 256-byte aligned; the first
+// `cleared` of them are zeroed together.  An array of no bytes stays NULL.
+struct DevicePart {
+  void* pointer;  // where the array's pointer is
+  size_t bytes;
+};
+struct DeviceLayout {
+  size_t total = 0, clear = 0;
+};
+inline DeviceLayout device_layout(const DevicePart* parts, int count, int cleared) {
+  DeviceLayout l;
+  for (int k = 0; k < count; ++k) {
+    l.total += (parts[k].bytes + 255) / 256 * 256;
+    if (k < cleared) l.clear = l.total;
+  }
+  return l;
+}
+inline void device_place(const DevicePart* parts, int count, void* block) {
+  char* at = static_cast<char*>(block);
+  for (int k = 0; k < count; ++k) {
+    if (parts[k].bytes) *static_cast<void**>(parts[k].pointer) = at;
+    at += (parts[k].bytes + 255) / 256 * 256;
+  }
+}
+
 // ---- grid geometry ----------------------------------------------------------
 // The grid state lives in HBM as three planar float32 channel planes with a
 // zero halo of kPad rows above and kPad columns left of the crop, and

@@ -322,6 +322,8 @@ struct EquSolverImpl : Solver {
   int block = 256;
   bool ready = false;
   EquGeom E{0, 0};
+  void* arena = nullptr;    // the arrays that a system's size needs, A to d_part
+  size_t system_bytes = 0;  // of A, x and b, its first
   int4* A = nullptr;
   float* x[2] = {nullptr, nullptr};
   float* b = nullptr;
@@ -455,13 +457,8 @@ struct EquSolverImpl : Solver {
   void release() {
     cudaStreamSynchronize(stream);  // NULL (legacy default stream) included
     drop_graphs();
-    cudaFree(A);
-    cudaFree(x[0]);
-    cudaFree(x[1]);
-    cudaFree(b);
-    cudaFree(d_img);
-    cudaFree(d_part);
-    cudaFree(d_err);
+    cudaFree(arena);
+    arena = nullptr;
     A = nullptr;
     x[0] = x[1] = b = nullptr;
     d_img = nullptr;
@@ -672,17 +669,18 @@ struct EquSolverImpl : Solver {
     E.np = ((long long)N + 31) / 32 * 32;
     nparts = (N + 255) / 256;
     const size_t pb = (size_t)E.np * 3 * sizeof(float);
-    FPIE_CUDA(cudaMalloc(&A, (size_t)N * sizeof(int4)));
-    FPIE_CUDA(cudaMalloc(&x[0], pb));
-    FPIE_CUDA(cudaMalloc(&x[1], pb));
-    FPIE_CUDA(cudaMalloc(&b, pb));
-    FPIE_CUDA(cudaMalloc(&d_img, (size_t)N * 3));
-    FPIE_CUDA(cudaMalloc(&d_part, (size_t)nparts * 3 * sizeof(double)));
-    FPIE_CUDA(cudaMalloc(&d_err, 4 * sizeof(float)));  // and the finish kernel's count
-    FPIE_CUDA(cudaMemsetAsync(d_err, 0, 4 * sizeof(float), stream));
-    FPIE_CUDA(cudaMemsetAsync(x[0], 0, pb, stream));
-    FPIE_CUDA(cudaMemsetAsync(x[1], 0, pb, stream));
-    FPIE_CUDA(cudaMemsetAsync(b, 0, pb, stream));
+    const DevicePart parts[] = {{&A, (size_t)N * sizeof(int4)},
+                                {&x[0], pb},
+                                {&x[1], pb},
+                                {&b, pb},
+                                {&d_err, 4 * sizeof(float)},  // and the finish kernel's count
+                                {&d_img, (size_t)N * 3},
+                                {&d_part, (size_t)nparts * 3 * sizeof(double)}};
+    const DeviceLayout l = device_layout(parts, 7, 5);
+    system_bytes = device_layout(parts, 4, 4).clear;
+    FPIE_CUDA(cudaMalloc(&arena, l.total));
+    device_place(parts, 7, arena);
+    FPIE_CUDA(cudaMemsetAsync(arena, 0, l.clear, stream));
     cur = 0;
   }
 
@@ -801,10 +799,7 @@ struct EquSolverImpl : Solver {
     const int N = unknowns + 1;
     allocate(N);
     ensure_index(unknowns);
-    FPIE_CUDA(cudaMemsetAsync(A, 0, sizeof(int4) * N, stream));
-    FPIE_CUDA(cudaMemsetAsync(x[0], 0, (size_t)E.np * 3 * sizeof(float), stream));
-    FPIE_CUDA(cudaMemsetAsync(x[1], 0, (size_t)E.np * 3 * sizeof(float), stream));
-    FPIE_CUDA(cudaMemsetAsync(b, 0, (size_t)E.np * 3 * sizeof(float), stream));
+    FPIE_CUDA(cudaMemsetAsync(arena, 0, system_bytes, stream));
     launch_equ_build(m01, mw, x0, y0, n, m, ids, dsrc, sw, s_row + x0, s_col + y0, dtgt, tw,
                      t_row + x0, t_col + y0, mode, E.np, A, x[0], x[1], b, d_rows, d_cols, stream);
     post_launch(this);

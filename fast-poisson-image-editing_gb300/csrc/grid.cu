@@ -159,6 +159,8 @@ struct GridSolverImpl : Solver {
   int N_user = 0;
   bool ready = false;
   GridGeom G{};
+  void* arena = nullptr;   // the arrays that a geometry needs, x to d_part
+  size_t plane_bytes = 0;  // of x, g and mask, its first
   float* x[2] = {nullptr, nullptr};
   float* g = nullptr;
   uint8_t* mask = nullptr;
@@ -368,14 +370,8 @@ struct GridSolverImpl : Solver {
   void release() {
     cudaStreamSynchronize(stream);  // NULL (legacy default stream) included
     drop_graphs();
-    cudaFree(x[0]);
-    cudaFree(x[1]);
-    cudaFree(g);
-    cudaFree(mask);
-    cudaFree(code);
-    cudaFree(d_img);
-    cudaFree(d_part);
-    cudaFree(d_err);
+    cudaFree(arena);
+    arena = nullptr;
     cudaFree(flags);
     flags = nullptr;
     flags_cap = 0;
@@ -433,25 +429,26 @@ struct GridSolverImpl : Solver {
     L = grid_launch(G);
     FPIE_REQUIRE(L.sweep_grid.y <= 65535, FPIE_ERR_ARG, "grid has too many rows");
     const size_t pb = (size_t)G.plane * sizeof(float);
-    FPIE_CUDA(cudaMalloc(&x[0], 3 * pb));
-    FPIE_CUDA(cudaMalloc(&x[1], 3 * pb));
-    FPIE_CUDA(cudaMalloc(&g, 3 * pb));
-    FPIE_CUDA(cudaMalloc(&mask, (size_t)G.plane));
-    FPIE_CUDA(cudaMalloc(&code, (size_t)G.plane));
-    FPIE_CUDA(cudaMalloc(&d_img, (size_t)n * m * 3));
-    FPIE_CUDA(cudaMalloc(&d_part, (size_t)L.nparts * 3 * sizeof(double)));
-    // One set of control words: err and the wait flag (read back together),
-    // the resident kernel's, the range mark, the finish kernel's count.
-    FPIE_CUDA(cudaMalloc(&d_err, (4 + kResCtl + 2) * sizeof(unsigned)));
-    FPIE_CUDA(cudaMemsetAsync(d_err, 0, (4 + kResCtl + 2) * sizeof(unsigned), stream));
+    // d_err: one set of control words: err and the wait flag (read back
+    // together), the resident kernel's, the range mark, the finish kernel's
+    // count.
+    const DevicePart parts[] = {{&x[0], 3 * pb},
+                                {&x[1], 3 * pb},
+                                {&g, 3 * pb},
+                                {&mask, (size_t)G.plane},
+                                {&d_err, (4 + kResCtl + 2) * sizeof(unsigned)},
+                                {&code, (size_t)G.plane},
+                                {&d_img, (size_t)n * m * 3},
+                                {&d_part, (size_t)L.nparts * 3 * sizeof(double)}};
+    const DeviceLayout l = device_layout(parts, 8, 5);
+    plane_bytes = device_layout(parts, 4, 4).clear;
+    FPIE_CUDA(cudaMalloc(&arena, l.total));
+    device_place(parts, 8, arena);
+    FPIE_CUDA(cudaMemsetAsync(arena, 0, l.clear, stream));
     d_wait_err = reinterpret_cast<int*>(d_err + 3);
     res_ctl = reinterpret_cast<unsigned*>(d_err + 4);
     maybe_wild = false;
     res = res_pin.empty() ? res_pick(n, m) : res_named(res_pin.c_str(), n, m);
-    FPIE_CUDA(cudaMemsetAsync(x[0], 0, 3 * pb, stream));
-    FPIE_CUDA(cudaMemsetAsync(x[1], 0, 3 * pb, stream));
-    FPIE_CUDA(cudaMemsetAsync(g, 0, 3 * pb, stream));
-    FPIE_CUDA(cudaMemsetAsync(mask, 0, (size_t)G.plane, stream));
     cur = 0;
   }
 
@@ -491,11 +488,7 @@ struct GridSolverImpl : Solver {
                       long long np) {
     allocate(n, m);
     N_user = n * m;
-    const size_t pb = (size_t)G.plane * 3 * sizeof(float);
-    FPIE_CUDA(cudaMemsetAsync(x[0], 0, pb, stream));
-    FPIE_CUDA(cudaMemsetAsync(x[1], 0, pb, stream));
-    FPIE_CUDA(cudaMemsetAsync(g, 0, pb, stream));
-    FPIE_CUDA(cudaMemsetAsync(mask, 0, (size_t)G.plane, stream));
+    FPIE_CUDA(cudaMemsetAsync(arena, 0, plane_bytes, stream));
     if (N > 1) {
       grid_from_equ_kernel<<<conv_blocks(N), 256, 0, stream>>>(G, N, pos, xe, be, np, mask, x[0],
                                                                x[1], g);
