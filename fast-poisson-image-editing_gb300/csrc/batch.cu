@@ -30,6 +30,7 @@
 #include "grid_mixed.cuh"
 #include "grid_tbp.cuh"
 #include "mixed_levels.cuh"
+#include "quarter.cuh"
 
 namespace fpie {
 
@@ -40,6 +41,7 @@ struct BJobDev {
   float* x[2];
   void* e[2];       // mixed forms: the correction (FP16 / BF16 planes)
   float* r;         // mixed forms: the FP32 residual planes
+  unsigned* odd;    // FP32: values outside the quartered sweep's range were seen
   int tiles_x;      // tiles per row of this job
   int ntiles;       // active tiles
   int tile_off;     // first entry of this job in the tile list
@@ -102,10 +104,70 @@ __device__ __noinline__ void batch_fold_item(const GridGeom& G, const uint8_t* m
                                                ks, lane, w, edge);
 }
 
+// An FP32 item by the quartered update (quarter.cuh), for jobs whose values
+// are in its range; whether this thread stored a nonzero value below 2^-60,
+// from which the next level (16 sweeps) would not be exact.  Most regions of
+// small jobs hold unmasked pixels, for which the packed update selects bit by
+// bit: 4 jobs of up to 400x400 took 1,627 us on 64-row regions, now 1,331, 24
+// of them on 128-row regions 2,452, now 2,330.
+constexpr int kTinyItem = 60;
+
+template <int R, int W, int K, bool FULL>
+__device__ __noinline__ bool batch_quarter_item(const GridGeom& G, const uint8_t* mask,
+                                                const float* gc, const float* xc, float* oc,
+                                                long long base, int ks, int lane, int w,
+                                                float4 (&edge)[2][2][W][32]) {
+  float P[R][4], Gq[R][4], L[FULL ? 1 : R][4];
+#pragma unroll
+  for (int i = 0; i < R; ++i) {
+    const long long p = base + (long long)i * G.pitch;
+    const float4 x4 = __ldcg(reinterpret_cast<const float4*>(xc + p));
+    const float4 g4 = ld4(gc + p);
+    const uint32_t mk = FULL ? 0u : __ldg(reinterpret_cast<const unsigned*>(mask + p));
+    const float x[4] = {x4.x, x4.y, x4.z, x4.w}, gv[4] = {g4.x, g4.y, g4.z, g4.w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const bool on = FULL || ((mk >> (8 * j)) & 0xffu);
+      P[i][j] = x[j];
+      if (!FULL) L[FULL ? 0 : i][j] = on ? __uint_as_float(kMasked) : x[j];
+      Gq[i][j] = on ? __fmul_rn(gv[j], 0.25f) : __uint_as_float(kNegInf);
+    }
+  }
+  int s = 0;
+  if (ks >= 2) {
+    post_edges<R, W, 32>(P, 0, lane, w, edge);
+    __syncthreads();
+#pragma unroll 1
+    for (; s + 2 <= ks; s += 2) {
+      quarter_sweep<R, W, 32, FULL, true>(P, Gq, L, 0, lane, w, edge);
+      quarter_sweep<R, W, 32, FULL, false>(P, Gq, L, 1, lane, w, edge);
+    }
+  }
+  if (s < ks)  // an odd last sweep
+    slow_sweep<R, W, 32>(
+        P, Gq, [&](int i, int j) { return FULL || __float_as_uint(L[FULL ? 0 : i][j]) == kMasked; },
+        4.f, lane, w, edge);
+  unsigned least = 0xffffffffu;
+  if (lane >= K / 4 && lane < 32 - K / 4) {
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      const int r = w * R + i;
+      if (r >= K && r < R * W - K) {
+        *reinterpret_cast<float4*>(oc + base + (long long)i * G.pitch) =
+            make_float4(P[i][0], P[i][1], P[i][2], P[i][3]);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) least = min(least, tiny_key(P[i][j]));
+      }
+    }
+  }
+  return least < tiny_limit(kTinyItem);
+}
+
 template <int R, int W, int K, typename TS>
 __global__ void __launch_bounds__(W * 32)
 batch_persistent_kernel(BQueue Q) {
   constexpr bool MIXED = !std::is_same<TS, float>::value;
+  constexpr bool QUARTER = !MIXED && W == 8;  // 16 warps: too few registers
   constexpr int TH = W * R - 2 * K;
   constexpr int TW = 128 - 2 * K;
   // The queue tables, in shared memory when they fit: decoding an item is
@@ -116,7 +178,7 @@ batch_persistent_kernel(BQueue Q) {
   __shared__ long long s_lo[kSL + 1], s_ct[kSJ + 1];
   __shared__ int s_act[kSL], s_order[kSJ];
   __shared__ long long s_idx;
-  __shared__ int s_stop;
+  __shared__ int s_stop, s_odd;
   __shared__ int2 s_tf;
   // The current item's job record, copied by warp 0 (one round trip) so
   // that the CTA does not chase it field by field through global memory --
@@ -175,7 +237,9 @@ batch_persistent_kernel(BQueue Q) {
       // Acquire loads: the read that sees the count orders the producers'
       // writes before everything this thread does next, and the CTA barrier
       // below carries that order to the other threads -- no separate fence.
-      while (ld_acquire_gpu(Q.done + j) < need) {
+      // The count's sign bit: an item of the last level was odd (below).
+      int v;
+      while (((v = ld_acquire_gpu(Q.done + j)) & 0x7fffffff) < need) {
         if (*(volatile int*)Q.error) { stop = 1; break; }
         if (++spins > Q.spin_limit) {
           atomicExch(Q.error, 1);
@@ -185,6 +249,7 @@ batch_persistent_kernel(BQueue Q) {
         __nanosleep(128);
       }
       s_stop = stop;
+      if (QUARTER) s_odd = z == 0 ? *(volatile unsigned*)J.odd != 0 : v < 0;
       // The next item is taken now, so that the atomic's round trip
       // overlaps this item's sweeps.  (A CTA then holds two items; the
       // lowest unfinished item is always one being worked on, since a held
@@ -199,12 +264,19 @@ batch_persistent_kernel(BQueue Q) {
     const long long base = J.G.at(ty * TH - K + w * R, tx * TW - K + 4 * lane);
     const long long co = c * J.G.plane;
     const float* gc = J.g + co;
+    bool odd = false;
+    unsigned* const odd_word = J.odd;
     if (!MIXED) {
       const int pin = (J.parity + z) & 1;
       const float* xc = J.x[pin] + co;
       float* oc = J.x[pin ^ 1] + co;
       const int ks = min(K, J.sweeps - z * K);
-      if (tf.y == 2)
+      odd = QUARTER && s_odd;
+      if (QUARTER && !odd) {
+        if constexpr (QUARTER)
+          odd = tf.y == 2 ? batch_quarter_item<R, W, K, true>(J.G, J.mask, gc, xc, oc, base, ks, lane, w, edge)
+                          : batch_quarter_item<R, W, K, false>(J.G, J.mask, gc, xc, oc, base, ks, lane, w, edge);
+      } else if (tf.y == 2)
         batch_sweep_item<R, W, K, true, float>(J.G, J.mask, gc, xc, oc, base, ks, lane, w, edge);
       else
         batch_sweep_item<R, W, K, false, float>(J.G, J.mask, gc, xc, oc, base, ks, lane, w, edge);
@@ -253,7 +325,11 @@ batch_persistent_kernel(BQueue Q) {
     // Release: the CTA barrier orders every thread's writes before the
     // release reduction, which makes them visible before the count.  Thread
     // 32 issues it, so that thread 0's next acquire does not queue behind it.
-    __syncthreads();
+    const bool any = QUARTER ? __syncthreads_or(odd) : (__syncthreads(), false);
+    if (QUARTER && any && threadIdx.x == 32) {  // for the next level, and the next launch
+      atomicOr(reinterpret_cast<unsigned*>(Q.done + j), 0x80000000u);
+      *(volatile unsigned*)odd_word = 1u;
+    }
     if (threadIdx.x == 32)
       asm volatile("red.release.gpu.global.add.s32 [%0], 1;" : : "l"(Q.done + j) : "memory");
   }
@@ -328,7 +404,7 @@ struct BatchJob {
   uint8_t* mask = nullptr;
   uint8_t* img = nullptr;
   double* parts = nullptr;  // per-block partials: 6 doubles each (norms need 6)
-  float* err = nullptr;     // [3], then the word count() points at
+  float* err = nullptr;     // [3], then the words count() and odd() point at
   double* norm = nullptr;   // [max|r| x3, sum|r| x3] of the last norms() call
   void* e[2] = {nullptr, nullptr};  // mixed forms only
   float* r = nullptr;               // mixed forms only
@@ -337,7 +413,23 @@ struct BatchJob {
   bool live = false;
   size_t bytes = 0;
   unsigned* count() const { return reinterpret_cast<unsigned*>(err + 3); }
+  unsigned* odd() const { return reinterpret_cast<unsigned*>(err + 4); }
 };
+
+// Sets *odd where a job's inputs are outside the quartered sweep's range:
+// values that are not finite, above 2^40 or nonzero below 2^-60, gradients of
+// masked pixels nonzero below 2^-38 (quarter.cuh).
+__global__ void batch_range_kernel(long long px, const int32_t* __restrict__ mk,
+                                   const float* __restrict__ t, const float* __restrict__ gr,
+                                   unsigned* odd) {
+  bool out = false;
+  for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < 3 * px;
+       k += (long long)gridDim.x * blockDim.x) {
+    out = out || !(fabsf(t[k]) <= 0x1p40f) || tiny_key(t[k]) < tiny_limit(kTinyItem);
+    if (mk[k / 3]) out = out || !(fabsf(gr[k]) <= 0x1p40f) || tiny_key(gr[k]) < tiny_limit(38);
+  }
+  if (out) *odd = 1u;
+}
 
 __global__ void batch_pack_kernel(GridGeom G, const int32_t* __restrict__ mk,
                                   const float* __restrict__ t, const float* __restrict__ gr,
@@ -416,7 +508,7 @@ struct Batch {
                                 {&j.x[1], 3 * pb},
                                 {&j.g, 3 * pb},
                                 {&j.mask, (size_t)j.G.plane},
-                                {&j.err, 4 * sizeof(float)},
+                                {&j.err, 5 * sizeof(float)},
                                 {&j.e[0], mixed ? eb : 0},
                                 {&j.e[1], mixed ? eb : 0},
                                 {&j.r, mixed ? 3 * pb : 0},
@@ -506,7 +598,11 @@ struct Batch {
           j.G, reinterpret_cast<int32_t*>(stage), reinterpret_cast<float*>(stage + px * 4),
           reinterpret_cast<float*>(stage + px * 16), j.mask, j.x[0], j.x[1], j.g);
       FPIE_CUDA(cudaGetLastError());
-      ++launches;
+      batch_range_kernel<<<blocks, 256, 0, stream>>>(
+          (long long)px, reinterpret_cast<int32_t*>(stage), reinterpret_cast<float*>(stage + px * 4),
+          reinterpret_cast<float*>(stage + px * 16), j.odd());
+      FPIE_CUDA(cudaGetLastError());
+      launches += 2;
       FPIE_CUDA(cudaStreamSynchronize(stream));  // the caller may reuse its arrays
     } catch (...) {
       free_job(j);
@@ -680,6 +776,7 @@ struct Batch {
       d.e[0] = j.e[0];
       d.e[1] = j.e[1];
       d.r = j.r;
+      d.odd = j.odd();
       d.tiles_x = tx;
       d.ntiles = (int)tl.size();
       d.tile_off = (int)tiles.size();
@@ -793,13 +890,13 @@ struct Batch {
 
   // Which variant runs the listed jobs, unless one was named.  A launch is
   // bound either by the chain of levels of its longest job (an item's latency
-  // per level: 13 us for "p16w8k16", 8.6 us for "p8w8k16", whose warps hold
+  // per level: 11.5 us for "p16w8k16", 7.2 us for "p8w8k16", whose warps hold
   // half the rows) or by the SMs' throughput, where the small regions' wider
   // aprons cost more (2.7 region pixels per pixel of a tile instead of 1.8).
   // Measured with up to 48 uneven jobs, us per launch, items per level of
-  // "p8w8k16" in brackets, FP32: [78] 1,634 against 2,375, [231] 2,037
-  // against 2,348, [279] 2,192 against 2,419, [333] 2,520 against 2,265,
-  // [429] 3,233 against 2,473; FP16 [78] 1,701 against 2,685, [333] 2,635
+  // "p8w8k16" in brackets, FP32: [78] 1,331 against 2,132, [231] 1,717
+  // against 2,126, [279] 1,876 against 2,210, [429] 2,689 against 2,330,
+  // [447] 2,725 against 2,591; FP16 [78] 1,701 against 2,685, [333] 2,635
   // against 2,533: the line lies at two items per SM.
   int pick(const std::vector<int>& ids) {
     const size_t small = 3;  // "p8w8k16" in batch_variants()

@@ -374,8 +374,8 @@ __global__ void __launch_bounds__(W * 32, 1) grid_res_kernel(ResArgs A) {
         __syncthreads();
 #pragma unroll 1
         for (; s + 2 <= ks; s += 2) {
-          quarter_sweep<R, NS, LW, true>(P, Gq, L, 0, lane, w, edge);
-          quarter_sweep<R, NS, LW, false>(P, Gq, L, 1, lane, w, edge);
+          quarter_sweep<R, NS, LW, false, true>(P, Gq, L, 0, lane, w, edge);
+          quarter_sweep<R, NS, LW, false, false>(P, Gq, L, 1, lane, w, edge);
         }
       }
       // An odd last sweep takes this path too (the same values).

@@ -1,5 +1,5 @@
 // The quartered Jacobi sweep on register-resident strips, for the resident
-// kernel (grid_res.cu).
+// kernel (grid_res.cu) and the batch (batch.cu).
 //
 // A pixel's next value is ((((g + up) + down) + left) + right) / 4 in the
 // numpy order.  Scaling by 1/4 commutes with rounding, so with g' = g / 4 it
@@ -59,10 +59,11 @@ __device__ __forceinline__ void post_edges(const float (&P)[R][4], int par, int 
 // rows stored before the last rows' (fully masked region of 8 rows, 4 warps:
 // 302 cycles a sweep against 318 from the top row down; through an mbarrier
 // with arrival and wait apart, 424).
-template <int R, int NS, int LW, bool FWD>
+// FULL: all of the region is masked.
+template <int R, int NS, int LW, bool FULL, bool FWD>
 __device__ __forceinline__ void quarter_sweep(float (&P)[R][4], const float (&Gq)[R][4],
-                                              const float (&L)[R][4], int par, int lane, int w,
-                                              float4 (&edge)[2][2][NS][LW]) {
+                                              const float (&L)[FULL ? 1 : R][4], int par, int lane,
+                                              int w, float4 (&edge)[2][2][NS][LW]) {
   const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
   const float4 a4 = w > 0 ? edge[par][1][w - 1][lane] : zero;
   const float4 b4 = w < NS - 1 ? edge[par][0][w + 1][lane] : zero;
@@ -99,7 +100,8 @@ __device__ __forceinline__ void quarter_sweep(float (&P)[R][4], const float (&Gq
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       keep[j] = cur[j];
-      P[i][j] = fmaxf(__fmaf_rn(j < 3 ? cur[j < 3 ? j + 1 : 0] : rt, 0.25f, t[j]), L[i][j]);
+      const float o = __fmaf_rn(j < 3 ? cur[j < 3 ? j + 1 : 0] : rt, 0.25f, t[j]);
+      P[i][j] = FULL ? o : fmaxf(o, L[FULL ? 0 : i][j]);
     }
     if (i == (FWD ? 0 : R - 1)) post_edges<R, NS, LW>(P, par ^ 1, lane, w, edge);
   }
