@@ -14,11 +14,9 @@
 //
 // Variants measured and removed (slower on every measured shape, kept out of
 // the library): the scalar one-value-per-lane "r" family (best r16w8k16:
-// 1.49 us/sweep on square800 against 1.32 for the packed p16w8k16), the
+// 1.49 us/sweep on square800 against 1.32 for the packed p16w8k16), and the
 // shallower and shared-grad packed ones (p8w12k8, p16w8k4, p12w12k8s,
-// p8w16k8s), and a one-launch kernel with tiles resident in registers for
-// the whole step (1.76 us/sweep: its per-period neighbour waits cost more
-// than the reloads they saved).
+// p8w16k8s).
 #include "common.cuh"
 #include "grid_tb.cuh"
 
