@@ -468,7 +468,7 @@ struct Batch {
   static constexpr int kMaxPending = 64;
   int* h_errs = nullptr;
   int n_pending = 0;
-  float* h_err = nullptr;  // a result's err, pinned: a copy to pageable memory waits by itself (36 us a result, now 29)
+  float* h_err = nullptr;  // a result's err, pinned: the finish kernel stores it
   // Asynchronous norms: one pinned array, filled by one copy per call.
   double* h_norms = nullptr;
   int h_norms_cap = 0, norms_count = -1;
@@ -993,10 +993,9 @@ struct Batch {
     std::memcpy(out, h.data(), 6 * sizeof(double) * (size_t)count);
   }
 
-  void finish(int id) {
+  void finish(int id, float* err) {
     BatchJob& j = job(id);
-    launch_grid_finish(j.L, j.G, j.mask, j.g, j.x[j.cur], j.img, j.parts,
-                       j.count(), j.err, stream);
+    launch_grid_finish(j.L, j.G, j.mask, j.g, j.x[j.cur], j.img, j.parts, j.count(), err, stream);
     FPIE_CUDA(cudaGetLastError());
     ++launches;
   }
@@ -1006,8 +1005,7 @@ struct Batch {
     if (n_pending) wait();
     BatchJob& j = job(id);
     if (!h_err) FPIE_CUDA(cudaMallocHost(&h_err, 3 * sizeof(float)));
-    finish(id);
-    FPIE_CUDA(cudaMemcpyAsync(h_err, j.err, 3 * sizeof(float), cudaMemcpyDeviceToHost, stream));
+    finish(id, h_err);
     FPIE_CUDA(cudaMemcpyAsync(img, j.img, (size_t)j.n * j.m * 3, cudaMemcpyDeviceToHost, stream));
     FPIE_CUDA(cudaStreamSynchronize(stream));
     std::memcpy(err, h_err, 3 * sizeof(float));

@@ -227,9 +227,12 @@ __device__ __forceinline__ double sum2_value(const Sum2& s) {
 // Block-wide sums of acc[3] to parts[3 * block ...], and by the last block to
 // arrive the total of all blocks' parts to err[3], in a fixed order.  256
 // threads; every thread of every block calls it.  count: a device word, 0
-// before the first launch; the last block clears it.
+// before the first launch; the last block clears it.  err may be pinned host
+// memory: then no copy follows (3-4 us of a step).  flag, unless NULL, goes to
+// err[3] with it.
 __device__ __forceinline__ void finish_sums(Sum2 (&acc)[3], unsigned block, unsigned blocks,
-                                            double* parts, unsigned* count, float* err) {
+                                            double* parts, unsigned* count, float* err,
+                                            const int* flag) {
   __shared__ double sh[3][8];
   __shared__ bool last;
   const int tid = threadIdx.x + threadIdx.y * blockDim.x, lane = tid & 31, warp = tid >> 5;
@@ -268,6 +271,7 @@ __device__ __forceinline__ void finish_sums(Sum2 (&acc)[3], unsigned block, unsi
     err[0] = (float)a;
     err[1] = (float)b;
     err[2] = (float)c;
+    if (flag) err[3] = __int_as_float(*(const volatile int*)flag);
     *count = 0;
   }
 }

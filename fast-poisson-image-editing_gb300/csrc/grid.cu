@@ -1269,9 +1269,9 @@ struct GridSolverImpl : Solver {
     }
   }
 
-  void finish(uint8_t* img, float* err) {
+  void finish(uint8_t* img, float* err, const int* flag = nullptr) {
     launch_grid_finish(L, G, mask, g, x[cur], img ? img : d_img, d_part, finish_count(),
-                       err ? err : d_err, stream);
+                       err ? err : d_err, stream, flag);
     post_launch(this);
   }
 
@@ -1282,13 +1282,11 @@ struct GridSolverImpl : Solver {
       return;
     }
     run_sweeps(iteration);
-    finish(d_img, d_err);
+    finish(d_img, h_err, d_wait_err);  // err and the wait flag behind it
     const size_t bytes = (size_t)G.n * G.m * 3;
     // Straight into the caller's (pageable) array: measured on GB300 5x
     // faster than a pinned staging buffer plus a host copy.
     FPIE_CUDA(cudaMemcpyAsync(img_out, d_img, bytes, cudaMemcpyDeviceToHost, stream));
-    // err and the wait flag behind it, in one copy.
-    FPIE_CUDA(cudaMemcpyAsync(h_err, d_err, 4 * sizeof(float), cudaMemcpyDeviceToHost, stream));
     FPIE_CUDA(cudaStreamSynchronize(stream));
     raise_waits();
     std::memcpy(err_out, h_err, 3 * sizeof(float));
@@ -1305,8 +1303,7 @@ struct GridSolverImpl : Solver {
     }
     FPIE_REQUIRE(pitch >= 3LL * G.m, FPIE_ERR_ARG, "rows of the picture overlap");
     run_sweeps(iteration);
-    finish(d_img, d_err);
-    FPIE_CUDA(cudaMemcpyAsync(h_err, d_err, 4 * sizeof(float), cudaMemcpyDeviceToHost, stream));
+    finish(d_img, h_err, d_wait_err);  // err and the wait flag behind it
     FPIE_CUDA(cudaStreamSynchronize(stream));
     raise_waits();
     FPIE_CUDA(cudaMemcpy2DAsync(dst, (size_t)pitch, d_img, (size_t)G.m * 3, (size_t)G.m * 3,
@@ -1459,6 +1456,15 @@ void grid_pin_kernel(Solver* s, const std::string& name) {
 }
 void grid_set_red_black(Solver* s, bool on) { static_cast<GridSolverImpl*>(s)->set_red_black(on); }
 std::string grid_kernel_of(Solver* s) { return static_cast<GridSolverImpl*>(s)->kernel_name(); }
+// The wait flag of the grid's kernels on the device, NULL without a grid; and
+// the error that a copy of it stands for.
+const int* grid_wait_flag(Solver* s) { return s ? static_cast<GridSolverImpl*>(s)->d_wait_err : nullptr; }
+void grid_raise(Solver* s, const float* flag) {
+  if (!s || !static_cast<GridSolverImpl*>(s)->d_wait_err) return;
+  GridSolverImpl* g = static_cast<GridSolverImpl*>(s);
+  std::memcpy(g->h_err + 3, flag, sizeof(float));
+  g->raise_waits();
+}
 void grid_set_spin(Solver* s, long long spins) {
   GridSolverImpl* h = static_cast<GridSolverImpl*>(s);
   if (spins != h->spin_limit) h->drop_graphs();

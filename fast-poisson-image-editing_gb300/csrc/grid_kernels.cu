@@ -78,7 +78,8 @@ __global__ void __launch_bounds__(kSweepBX * kSweepBY)
 grid_finish_kernel(GridGeom G, const uint8_t* __restrict__ mask,
                    const float* __restrict__ g, const float* __restrict__ x,
                    uint8_t* __restrict__ img, double* __restrict__ parts,
-                   unsigned* __restrict__ count, float* __restrict__ err, int rows) {
+                   unsigned* __restrict__ count, float* __restrict__ err,
+                   const int* flag, int rows) {
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
   const int i0 = (blockIdx.y * blockDim.y + threadIdx.y) * rows;
   Sum2 acc[3];
@@ -118,7 +119,8 @@ grid_finish_kernel(GridGeom G, const uint8_t* __restrict__ mask,
     const int q0 = q & ~31;  // the warp's first group
     store_run(img + ((long long)i * G.m + 4 * q0) * 3, w0, w1, w2, jn);
   }
-  finish_sums(acc, blockIdx.y * gridDim.x + blockIdx.x, gridDim.x * gridDim.y, parts, count, err);
+  finish_sums(acc, blockIdx.y * gridDim.x + blockIdx.x, gridDim.x * gridDim.y, parts, count, err,
+              flag);
 }
 
 GridLaunch grid_launch(const GridGeom& G) {
@@ -143,9 +145,9 @@ void launch_grid_sweep(const GridLaunch& L, const GridGeom& G,
 void launch_grid_finish(const GridLaunch& L, const GridGeom& G,
                         const uint8_t* mask, const float* g, const float* x,
                         uint8_t* img, double* parts, unsigned* count, float* err,
-                        cudaStream_t st) {
+                        cudaStream_t st, const int* flag) {
   grid_finish_kernel<<<L.finish_grid, L.finish_block, 0, st>>>(G, mask, g, x, img, parts, count,
-                                                               err, L.finish_rows);
+                                                               err, flag, L.finish_rows);
 }
 
 }  // namespace fpie

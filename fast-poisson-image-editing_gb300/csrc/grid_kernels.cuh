@@ -21,10 +21,11 @@ void launch_grid_sweep(const GridLaunch& L, const GridGeom& G,
 
 // The residual sums (err[3]; parts: nparts x 3 doubles of scratch, count: a
 // device word that is 0 between launches) and the clipped uint8 image in the
-// reference's interleaved [n][m][3] layout.
+// reference's interleaved [n][m][3] layout.  err may be pinned host memory;
+// flag, unless NULL, is copied to err[3].
 void launch_grid_finish(const GridLaunch& L, const GridGeom& G,
                         const uint8_t* mask, const float* g, const float* x,
                         uint8_t* img, double* parts, unsigned* count, float* err,
-                        cudaStream_t st);
+                        cudaStream_t st, const int* flag = nullptr);
 
 }  // namespace fpie
