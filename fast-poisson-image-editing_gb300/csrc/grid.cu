@@ -213,6 +213,7 @@ struct GridSolverImpl : Solver {
   int flow_cap = 0;             // tiles the arrays hold
   int ft_tiles_x = 0, ft_tiles = 0;
   int ft_k = 0;  // depth the tables were built for
+  bool ft_pin = false;  // with the code plane and the bodies
   bool ft_ok = false;
   int flow_grid = 0;
 
@@ -608,20 +609,22 @@ struct GridSolverImpl : Solver {
   // The kernel before any step.
   static int default_variant() { return tb_named("p16w8k16"); }
 
-  // Steps too short to tune on.  The flow kernel's tables cost 25 us (902x902)
-  // to 65 us (1800x1800) after a reset, its sweeps less than the launches';
-  // us for 100, 200, 400 sweeps from a reset, launches against flow: disk of
-  // 902x902 175/177, 325/286, 628/511; box of 1100x1100 230/238, 428/405,
-  // 835/743; box of 1800x1800 522/553, 991/1008, 1943/1935; 500x2500 262/255,
-  // 490/436, 952/806 (so from 256 sweeps on).  On larger grids launches of
-  // tall regions are faster (grid_tbp.cu; 2300x2300 disk 2,420/2,556, 2900x2900
-  // 3,550/3,945).
-  static constexpr int kFlowFrom = 256;
-  static constexpr long long kFlowPixels = 1800LL * 1800;
-  int untuned_sweeps = 0;  // since the reset, up to kFlowFrom
+  // Steps too short to tune on.  The flow kernel's tables cost 10-20 us after
+  // a reset, its sweeps less than the launches'; us for 64, 100, 200 sweeps
+  // from a reset, launches against flow: disk of 902x902 111/112, 175/149,
+  // 324/262; box of 1100x1100 146/151, 232/214, 429/380; disk of 1400x1400
+  // 192/202, 306/285, 571/516; 500x2500 164/161, 259/226, 487/406; box of
+  // 1800x1800 321/353, 520/522, 990/972.  On larger grids launches of tall
+  // regions are faster (grid_tbp.cu; 2300x2300 disk 2,420 for 400 sweeps
+  // against 2,556, 2900x2900 3,550 against 3,945).
+  static constexpr int kFlowFrom = 100, kFlowFromLarge = 200;
+  static constexpr long long kFlowLarge = 1500LL * 1500, kFlowPixels = 1800LL * 1800;
+  int untuned_sweeps = 0;  // since the reset, up to kFlowFromLarge
   int untuned_variant(int iters) const {
-    if ((long long)G.n * G.m > kFlowPixels) return tb_named("p22w8k16");
-    return iters >= kFlowFrom - untuned_sweeps ? kFlow12 : default_variant();
+    const long long px = (long long)G.n * G.m;
+    if (px > kFlowPixels) return tb_named("p22w8k16");
+    const int from = px > kFlowLarge ? kFlowFromLarge : kFlowFrom;
+    return untuned_sweeps >= from || iters >= from - untuned_sweeps ? kFlow12 : default_variant();
   }
 
   int depth() const {
@@ -674,7 +677,7 @@ struct GridSolverImpl : Solver {
   // Flags, active-tile list, records and counters of the flow tiling.
   void ensure_flow_tables() {
     const int kd = flow_k();
-    if (ft_ok && ft_k == kd) return;
+    if (ft_ok && ft_k == kd && (ft_pin || !flow_pin())) return;
     const int th = flow_tile_h(kd), tw = flow_tile_w(kd);
     ft_tiles_x = (G.m + tw - 1) / tw;
     ft_tiles = ft_tiles_x * ((G.n + th - 1) / th);
@@ -699,11 +702,13 @@ struct GridSolverImpl : Solver {
     post_launch(this);
     launch_tma_list(ft_flags, ft_tiles, ft_list, stream);
     post_launch(this);
-    launch_grid_code(G, mask, code, stream);
-    post_launch(this);
-    launch_flow_tables(G, code, kd, ft_list, ft_flags, ft_tiles_x, ft_tiles, flow_inv, flow_rec,
-                       stream);
-    post_launch(this, 3);
+    // The code plane and the bodies chosen from it take most of the time (20
+    // us of 25 on a 902x902 grid); only the pinned-boundary kernels read them.
+    ft_pin = flow_pin();
+    if (ft_pin) launch_grid_code(G, mask, code, stream);
+    launch_flow_tables(G, ft_pin ? code : nullptr, kd, ft_list, ft_flags, ft_tiles_x, ft_tiles,
+                       flow_inv, flow_rec, stream);
+    post_launch(this, ft_pin ? 4 : 2);
     ft_k = kd;
     ft_ok = true;
   }
@@ -887,7 +892,7 @@ struct GridSolverImpl : Solver {
                  "the grid's tiles do not fit on the device: no '" + res_pin + "' sweeps");
     if (!tuned && !pinned) iters -= autotune(iters);
     if (!tuned && !pinned && !red_black) select_variant(untuned_variant(iters));
-    untuned_sweeps += std::min(iters, kFlowFrom - untuned_sweeps);
+    untuned_sweeps += std::min(iters, kFlowFromLarge - untuned_sweeps);
     if (is_flow(variant)) {
       if (iters > 0) run_flow(iters);
       return;

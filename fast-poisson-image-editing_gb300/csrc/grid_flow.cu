@@ -528,8 +528,9 @@ void launch_flow_tables(const GridGeom& G, const uint8_t* code, int depth, const
   flow_rec_kernel<<<(tiles + 255) / 256, 256, 0, st>>>(list + 1, inv, flags, tiles_x,
                                                        tiles / tiles_x,
                                                        static_cast<FlowRec*>(rec));
-  flow_body_kernel<<<tiles, 256, 0, st>>>(G, code, list + 1, tiles_x, flow_tile_h(depth),
-                                          flow_tile_w(depth), depth, static_cast<FlowRec*>(rec));
+  if (code)
+    flow_body_kernel<<<tiles, 256, 0, st>>>(G, code, list + 1, tiles_x, flow_tile_h(depth),
+                                            flow_tile_w(depth), depth, static_cast<FlowRec*>(rec));
 }
 
 size_t flow_rec_bytes() { return sizeof(FlowRec); }

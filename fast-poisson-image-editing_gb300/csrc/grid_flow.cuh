@@ -19,7 +19,8 @@ int flow_ctas();
 
 // Per-mask tables of the depth-`depth` tiling from the active-tile list
 // `list` (count + indices, as built by launch_tma_list), the tile flags and
-// the code plane (launch_grid_code, built before): inv (tiles ints) and rec
+// the code plane (launch_grid_code, built before; NULL: no pinned-boundary
+// sweeps will read the records): inv (tiles ints) and rec
 // (tiles x flow_rec_bytes(): each active tile's index, sweep body and the
 // done offsets of its 3x3 neighbourhood).
 void launch_flow_tables(const GridGeom& G, const uint8_t* code, int depth, const int* list,

@@ -1,7 +1,7 @@
 """Steps too short for the autotuner: launches at first, the flow kernel once
-256 sweeps have been asked for since the reset, and launches of tall regions on
-grids of more than 1800x1800; the oracle's states, bit for bit, through the
-change and after a new reset."""
+100 (large grids: 200) sweeps have been asked for since the reset, and launches
+of tall regions on grids of more than 1800x1800; the oracle's states, bit for
+bit, through the change and after a new reset."""
 
 from __future__ import annotations
 
@@ -24,19 +24,19 @@ def _inputs(n, m, seed):
     return mask, tgt, grad
 
 
-@pytest.mark.parametrize("size,flow", [((845, 850), True), ((100, 8000), True), ((1800, 1800), True),
-                                       ((1801, 1800), False)])
-def test_kernel_by_the_sweeps_since_the_reset(size, flow):
+@pytest.mark.parametrize("size,flow_from", [((845, 850), 100), ((100, 8000), 100), ((1500, 1500), 100),
+                                            ((1500, 1501), 200), ((1800, 1800), 200), ((1801, 1800), 0)])
+def test_kernel_by_the_sweeps_since_the_reset(size, flow_from):
     from fpie_gb300 import backend
 
     s = backend.GridSolver(8, 8)
-    early, late = ("p16w8k16", "p16w8k12d") if flow else ("p22w8k16", "p22w8k16")
+    early, late = ("p16w8k16", "p16w8k12d") if flow_from else ("p22w8k16", "p22w8k16")
     for seed in (1, 2):
         mask, tgt, grad = _inputs(*size, seed)
         s.reset(mask.size, mask, tgt, grad)
         assert s.resident == ""
         o = cjacobi.CGrid(mask, tgt, grad)
-        for k, kernel in ((100, early), (155, early), (1, late), (13, late)):
+        for k, kernel in ((60, early), (max(flow_from, 100) - 61, early), (1, late), (13, late)):
             s.step(k)
             o.sweep(k)
             assert s.kernel == kernel
