@@ -265,10 +265,13 @@ int fpie_residual_norms(fpie_solver* s, double* out);
 int fpie_grid_solve(fpie_solver* s, double tol, int max_sweeps, int check_every,
                     int* sweeps_done);
 
-/* Selects the grid sweep kernel by name: "auto" (default: the autotuner
- * times the candidates on the first long step and keeps the fastest for this
- * grid shape), "sweep1" (one sweep per launch), a packed temporally
- * blocked variant "p16w8k16", "p8w16k16" or "p16w8k8" (R rows per thread, W
+/* Selects the grid sweep kernel by name: "auto" (default: FP32 Jacobi sweeps of
+ * a grid whose tiles fit on the device run on a resident kernel chosen by its
+ * size, see fpie_grid_resident; else the autotuner times the candidates on the
+ * first long step and keeps the fastest for this grid shape, and shorter steps
+ * take a kernel by the grid's size and the sweeps since the reset), "sweep1"
+ * (one sweep per launch), a packed temporally blocked variant "p16w8k16",
+ * "p8w16k16", "p16w8k8", "p8w8k8" or "p22w8k16" (R rows per thread, W
  * warps, K sweeps per launch), "p16w8k16d" (the whole step in one
  * cooperative launch, items started by neighbourhood dependencies, levels
  * of 16 sweeps on 96x96 tiles), "p16w8k12d" (the same with levels of 12
@@ -392,7 +395,9 @@ int fpie_batch_state(fpie_batch* b, int job, float* out);
 int fpie_batch_norms(fpie_batch* b, const int* jobs, int count, double* out);
 int fpie_batch_remove(fpie_batch* b, int job);
 int fpie_batch_memory(fpie_batch* b, double* used, double* budget);
-/* "auto" or a variant name ("p16w8k16", "p8w16k16", "p16w8k8"). */
+/* "auto" (default: "p8w8k16" for runs of at most two of its items per SM,
+ * "p16w8k16" for larger ones) or a variant name ("p16w8k16", "p8w16k16",
+ * "p16w8k8", "p8w8k16"). */
 int fpie_batch_set_kernel(fpie_batch* b, const char* name);
 int fpie_batch_kernel(fpie_batch* b, char* buf, int len);
 /* Iterations (about 128 ns each) a CTA may wait for a dependency. */
