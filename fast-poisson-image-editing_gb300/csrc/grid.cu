@@ -877,6 +877,12 @@ struct GridSolverImpl : Solver {
     return used;
   }
 
+  bool capturing() const {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    return cudaStreamIsCapturing(stream, &status) == cudaSuccess &&
+           status != cudaStreamCaptureStatusNone;
+  }
+
   void run_sweeps(int iters) {
     FPIE_REQUIRE(ready, FPIE_ERR_STATE, "step called before reset");
     if (iters <= 0) return;
@@ -891,7 +897,12 @@ struct GridSolverImpl : Solver {
     FPIE_REQUIRE(res_pin.empty() || red_black, FPIE_ERR_ARG,
                  "the grid's tiles do not fit on the device: no '" + res_pin + "' sweeps");
     if (!tuned && !pinned) iters -= autotune(iters);
-    if (!tuned && !pinned && !red_black) select_variant(untuned_variant(iters));
+    if (!tuned && !pinned && !red_black) {
+      const int v = untuned_variant(iters);
+      // The flow kernel's tables are allocated on its first step, which a
+      // caller's capture would refuse.
+      select_variant(is_flow(v) && flow_cap == 0 && capturing() ? default_variant() : v);
+    }
     untuned_sweeps += std::min(iters, kFlowFromLarge - untuned_sweeps);
     if (is_flow(variant)) {
       if (iters > 0) run_flow(iters);

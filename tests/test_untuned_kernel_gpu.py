@@ -56,3 +56,34 @@ def test_tall_regions_at_their_edges(size):
         s.step(k)
         o.sweep(k)
         np.testing.assert_array_equal(s.state(), o.x)
+
+
+@pytest.mark.parametrize("size,warm", [((902, 902), 1), ((902, 902), 3), ((194, 194), 1), ((1900, 1810), 1)])
+def test_a_short_step_in_a_captured_graph(size, warm):
+    """One warm-up step is enough to capture the next, although that one passes
+    the number of sweeps from which the flow kernel is taken."""
+    import torch
+
+    from fpie_gb300 import backend
+
+    mask, tgt, grad = _inputs(*size, 4)
+    stream = torch.cuda.Stream()
+    s = backend.GridSolver(8, 8)
+    s.set_stream(stream.cuda_stream)
+    dev = [torch.from_numpy(a).cuda() for a in (mask, tgt, grad)]
+    img = torch.empty((*size, 3), dtype=torch.uint8, device="cuda")
+    err = torch.empty(3, dtype=torch.float32, device="cuda")
+    torch.cuda.synchronize()
+    s.reset_tensors(*dev)
+    for _ in range(warm):
+        s.step_tensors(50, img, err)
+    s.sync()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        s.step_tensors(50, img, err)
+    with torch.cuda.stream(stream):
+        graph.replay()
+    torch.cuda.synchronize()
+    o = cjacobi.CGrid(mask, tgt, grad)
+    o.sweep(50 * (warm + 1))
+    np.testing.assert_array_equal(img.cpu().numpy(), o.image())
