@@ -244,6 +244,18 @@ struct GridSolverImpl : Solver {
     cur ^= 1;
   }
 
+  // Repeated steps of a few sweeps: a resident step starts with 11 us (whole
+  // grids) to 21 us of loads, tables and the tiles' first exchange, a launch
+  // of up to 16 sweeps takes 7-17 us once its tile flags are there.  us for 1,
+  // 8, 16, 24 sweeps, resident against launches: 38x38 11/7, 11/11, 11/13,
+  // 13/22; 194x194 17/9, 17/13, 19/17, 22/27; 660x660 21/9, 25/13, 28/17,
+  // 35/27.  A reset's first such step would pay for the flags (6 us): it stays.
+  int few_steps = 0;  // since the reset
+  bool few_sweeps(int iters) {
+    if (!res_pin.empty() || iters > (res_whole(res, G.n, G.m) ? 4 : 16)) return false;
+    return few_steps++ > 0;
+  }
+
   // After a reset from floats (uint8 images are always in range).
   void check_range() {
     grid_range_kernel<<<conv_blocks((long long)G.n * ((G.m + 3) / 4)), 256, 0, stream>>>(
@@ -421,10 +433,12 @@ struct GridSolverImpl : Solver {
       mflags_ok = false;
       ft_ok = false;
       untuned_sweeps = 0;
+      few_steps = 0;
       return;
     }
     release();
     untuned_sweeps = 0;
+    few_steps = 0;
     if (!pinned) tuned = false;
     G = make_geom(n, m);
     L = grid_launch(G);
@@ -890,14 +904,19 @@ struct GridSolverImpl : Solver {
       run_mixed(iters);
       return;
     }
-    if (use_res()) {
+    const bool few = use_res() && few_sweeps(iters);
+    if (use_res() && !few) {
       run_res(iters);
       return;
     }
     FPIE_REQUIRE(res_pin.empty() || red_black, FPIE_ERR_ARG,
                  "the grid's tiles do not fit on the device: no '" + res_pin + "' sweeps");
-    if (!tuned && !pinned) iters -= autotune(iters);
-    if (!tuned && !pinned && !red_black) {
+    if (few) {
+      select_variant(default_variant());
+    } else if (!tuned && !pinned) {
+      iters -= autotune(iters);
+    }
+    if (!few && !tuned && !pinned && !red_black) {
       const int v = untuned_variant(iters);
       // The flow kernel's tables are allocated on its first step, which a
       // caller's capture would refuse.

@@ -497,6 +497,8 @@ int res_tiles(const ResShape& s, int n, int m) {
 
 }  // namespace
 
+bool res_whole(const ResShape& s, int n, int m) { return res_tiles(s, n, m) == 1; }
+
 static ResShape res_parse(const char* name) {
   ResShape s{0, 0, 0, 0};
   int used = 0;

@@ -298,7 +298,8 @@ int fpie_grid_kernel(fpie_solver* s, char* buf, int len);
 /* Writes the name of the resident kernel ("p<R>w<W>x<width>k<K>r") that runs the
  * loaded grid's FP32 Jacobi sweeps, or "" if they run on the tile kernel.
  * Unless a kernel is pinned, grids whose tiles all fit on the device at once
- * are resident. */
+ * are resident; repeated steps of a few sweeps run on the tile kernel all the
+ * same (its launch starts sooner). */
 int fpie_grid_resident(fpie_solver* s, char* buf, int len);
 
 /* ---- allocation-free grid step ---------------------------------------------

@@ -245,3 +245,17 @@ def test_solve_stops_where_the_norms_do(size, max_sweeps, every):
             np.testing.assert_array_equal(s.state(), t.state())
         assert s.solve(1e9, 100, 10) == 0  # nothing to do
         np.testing.assert_array_equal(s.state(), t.state())
+
+
+@pytest.mark.parametrize("size", [(30, 40), (150, 200), (830, 300)])
+def test_short_steps_between_long_ones(size):
+    """Steps of a few sweeps run as launches after a reset's first one, long
+    ones on the resident kernel, on the same state."""
+    from fpie_gb300 import backend
+
+    s = backend.GridSolver(8, 8)
+    for seed in (1, 2):
+        mask, tgt, grad = _inputs(*size, seed, 0.8)
+        s.reset(mask.size, mask, tgt, grad)
+        assert s.resident
+        _compare(s, cjacobi.CGrid(mask, tgt, grad), (1, 1, 4, 5, 16, 17, 3, 40, 2, 16, 1, 64, 16))
