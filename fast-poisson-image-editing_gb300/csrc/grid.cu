@@ -630,15 +630,17 @@ struct GridSolverImpl : Solver {
   // 192/202, 306/285, 571/516; 500x2500 164/161, 259/226, 487/406; box of
   // 1800x1800 321/353, 520/522, 990/972.  On larger grids launches of tall
   // regions are faster (grid_tbp.cu; 2300x2300 disk 2,420 for 400 sweeps
-  // against 2,556, 2900x2900 3,550 against 3,945).
-  static constexpr int kFlowFrom = 100, kFlowFromLarge = 200;
+  // against 2,556, 2900x2900 3,550 against 3,945).  Short steps
+  // start sooner as launches: 16, 32, 48 sweeps with the tables there 38/29,
+  // 54/55, 71/82 on 902x902, 67/54, 108/103, 148/154 on 1400x1400.
+  static constexpr int kFlowFrom = 100, kFlowFromLarge = 200, kFlowStep = 48;
   static constexpr long long kFlowLarge = 1500LL * 1500, kFlowPixels = 1800LL * 1800;
   int untuned_sweeps = 0;  // since the reset, up to kFlowFromLarge
   int untuned_variant(int iters) const {
     const long long px = (long long)G.n * G.m;
     if (px > kFlowPixels) return tb_named("p22w8k16");
     const int from = px > kFlowLarge ? kFlowFromLarge : kFlowFrom;
-    return untuned_sweeps >= from || iters >= from - untuned_sweeps ? kFlow12 : default_variant();
+    return iters >= kFlowStep && iters >= from - untuned_sweeps ? kFlow12 : default_variant();
   }
 
   int depth() const {

@@ -36,7 +36,8 @@ def test_kernel_by_the_sweeps_since_the_reset(size, flow_from):
         s.reset(mask.size, mask, tgt, grad)
         assert s.resident == ""
         o = cjacobi.CGrid(mask, tgt, grad)
-        for k, kernel in ((60, early), (max(flow_from, 100) - 61, early), (1, late), (13, late)):
+        for k, kernel in ((8, early), (max(flow_from, 100) - 56, early),
+                          (47, early), (48, late), (47, early), (100, late), (1, early)):
             s.step(k)
             o.sweep(k)
             assert s.kernel == kernel
