@@ -330,6 +330,9 @@ batch_persistent_kernel(BQueue Q) {
       atomicOr(reinterpret_cast<unsigned*>(Q.done + j), 0x80000000u);
       *(volatile unsigned*)odd_word = 1u;
     }
+    // The 16-warp form looks at nothing it stores: what it leaves may be
+    // outside the range, and a later launch of another form must not trust it.
+    if (!MIXED && !QUARTER && z == 0 && threadIdx.x == 32) *(volatile unsigned*)odd_word = 1u;
     if (threadIdx.x == 32)
       asm volatile("red.release.gpu.global.add.s32 [%0], 1;" : : "l"(Q.done + j) : "memory");
   }
