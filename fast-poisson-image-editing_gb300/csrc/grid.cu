@@ -159,7 +159,7 @@ struct GridSolverImpl : Solver {
   int N_user = 0;
   bool ready = false;
   GridGeom G{};
-  void* arena = nullptr;   // the arrays that a geometry needs, x to d_part
+  void* arena = nullptr;   // the arrays that a geometry needs, x to flags
   size_t plane_bytes = 0;  // of x, g and mask, its first
   float* x[2] = {nullptr, nullptr};
   float* g = nullptr;
@@ -385,9 +385,7 @@ struct GridSolverImpl : Solver {
     drop_graphs();
     cudaFree(arena);
     arena = nullptr;
-    cudaFree(flags);
-    flags = nullptr;
-    flags_cap = 0;
+    flags[0] = flags[1] = tile_flags = nullptr;
     flags_ok = false;
     release_mixed();
     cudaFree(tma_list);
@@ -454,11 +452,13 @@ struct GridSolverImpl : Solver {
                                 {&d_err, (4 + kResCtl + 2) * sizeof(unsigned)},
                                 {&code, (size_t)G.plane},
                                 {&d_img, (size_t)n * m * 3},
-                                {&d_part, (size_t)L.nparts * 3 * sizeof(double)}};
-    const DeviceLayout l = device_layout(parts, 8, 5);
+                                {&d_part, (size_t)L.nparts * 3 * sizeof(double)},
+                                {&flags[0], most_tiles(n, m)},
+                                {&flags[1], most_tiles(n, m)}};
+    const DeviceLayout l = device_layout(parts, 10, 5);
     plane_bytes = device_layout(parts, 4, 4).clear;
     FPIE_CUDA(cudaMalloc(&arena, l.total));
-    device_place(parts, 8, arena);
+    device_place(parts, 10, arena);
     FPIE_CUDA(cudaMemsetAsync(arena, 0, l.clear, stream));
     d_wait_err = reinterpret_cast<int*>(d_err + 3);
     res_ctl = reinterpret_cast<unsigned*>(d_err + 4);
@@ -610,9 +610,23 @@ struct GridSolverImpl : Solver {
   int variant = default_variant();
   bool tuned = false;       // kernel chosen by the autotuner (or pinned)
   bool pinned = false;      // chosen explicitly with fpie_grid_set_kernel
-  uint8_t* flags = nullptr;  // active-tile flags of `variant`
-  int flags_cap = 0, tiles_x = 0, tiles = 0;
-  bool flags_ok = false;
+  // Active-tile flags of `variant`; [1]: those of a step being captured before
+  // [0] were built, which its graph builds anew at each replay.
+  uint8_t* flags[2] = {nullptr, nullptr};
+  uint8_t* tile_flags = nullptr;  // the ones that the next launch reads
+  int tiles_x = 0, tiles = 0;
+  bool flags_ok = false;          // flags[0] are this mask's and variant's
+
+  // Tiles of the launch kernel with the most, for which flags are allocated
+  // with the planes: no step, captured or not, allocates them.
+  static size_t most_tiles(int n, int m) {
+    const auto count = [&](int th, int tw) {
+      return (size_t)((n + th - 1) / th) * (size_t)((m + tw - 1) / tw);
+    };
+    size_t most = count(tma_tile_h(), tma_tile_w());
+    for (const TbVariant& v : tb_variants()) most = std::max(most, count(v.tile_h, v.tile_w));
+    return most;
+  }
 
   static int tb_named(const char* name) {
     for (size_t k = 0; k < tb_variants().size(); ++k)
@@ -636,11 +650,15 @@ struct GridSolverImpl : Solver {
   static constexpr int kFlowFrom = 100, kFlowFromLarge = 200, kFlowStep = 48;
   static constexpr long long kFlowLarge = 1500LL * 1500, kFlowPixels = 1800LL * 1800;
   int untuned_sweeps = 0;  // since the reset, up to kFlowFromLarge
+  int launch_variant() const {
+    return (long long)G.n * G.m > kFlowPixels ? tb_named("p22w8k16") : default_variant();
+  }
   int untuned_variant(int iters) const {
     const long long px = (long long)G.n * G.m;
-    if (px > kFlowPixels) return tb_named("p22w8k16");
     const int from = px > kFlowLarge ? kFlowFromLarge : kFlowFrom;
-    return iters >= kFlowStep && iters >= from - untuned_sweeps ? kFlow12 : default_variant();
+    return px <= kFlowPixels && iters >= kFlowStep && iters >= from - untuned_sweeps
+               ? kFlow12
+               : launch_variant();
   }
 
   int depth() const {
@@ -655,7 +673,11 @@ struct GridSolverImpl : Solver {
       return;
     }
     // sweep1: no flags
-    if (flags_ok || (variant < 0 && variant != kTma)) return;
+    if (variant < 0 && variant != kTma) return;
+    tile_flags = flags[0];
+    if (flags_ok) return;
+    const bool recorded = capturing();  // not built now, but at each replay
+    tile_flags = flags[recorded];
     const bool tma = variant == kTma;
     const bool listed = tma;  // kernels that take the active-tile list
     const int th = tma ? tma_tile_h() : tb_variants()[variant].tile_h;
@@ -663,16 +685,10 @@ struct GridSolverImpl : Solver {
     const int kd = tma ? tma_depth() : tb_variants()[variant].apron;
     tiles_x = (G.m + tw - 1) / tw;
     tiles = tiles_x * ((G.n + th - 1) / th);
-    if (tiles > flags_cap) {
-      cudaFree(flags);
-      flags = nullptr;
-      FPIE_CUDA(cudaMalloc(&flags, tiles));
-      flags_cap = tiles;
-    }
     if (listed) {
       prepare_tma();
       tma_grid = tma_ctas(tiles * 3);
-        if (tiles + 1 > tma_list_cap) {
+      if (tiles + 1 > tma_list_cap) {
         cudaFree(tma_list);
         tma_list = nullptr;
         FPIE_CUDA(cudaMalloc(&tma_list, (size_t)(tiles + 1) * sizeof(int)));
@@ -681,13 +697,13 @@ struct GridSolverImpl : Solver {
     } else {
       tb_variants()[variant].prepare();
     }
-    launch_tile_flags(G, mask, th, tw, kd, tiles_x, tiles, flags, stream);
+    launch_tile_flags(G, mask, th, tw, kd, tiles_x, tiles, tile_flags, stream);
     post_launch(this);
     if (listed) {
-      launch_tma_list(flags, tiles, tma_list, stream);
+      launch_tma_list(tile_flags, tiles, tma_list, stream);
       post_launch(this);
     }
-    flags_ok = true;
+    flags_ok = !recorded;
   }
 
   // Flags, active-tile list, records and counters of the flow tiling.
@@ -726,7 +742,7 @@ struct GridSolverImpl : Solver {
                        flow_inv, flow_rec, stream);
     post_launch(this, ft_pin ? 4 : 2);
     ft_k = kd;
-    ft_ok = true;
+    ft_ok = !capturing();  // else they are built when the graph is replayed
   }
 
   void select_variant(int v) {
@@ -760,13 +776,13 @@ struct GridSolverImpl : Solver {
   void launch_block(cudaStream_t st, int from, int k) {
     if (variant == kTma) {
       waits = true;
-      launch_tma(G, mask, g, x[from], x[from ^ 1], flags, tma_list, tiles_x, tiles, k, d_wait_err,
+      launch_tma(G, mask, g, x[from], x[from ^ 1], tile_flags, tma_list, tiles_x, tiles, k, d_wait_err,
                  spin_limit, tma_grid, st);
     } else if (variant < 0) {
       launch_grid_sweep(L, G, mask, g, x[from], x[from ^ 1], st);
     } else {
       const TbVariant& v = tb_variants()[variant];
-      v.launch(G, mask, g, x[from], x[from ^ 1], flags, tiles_x, tiles, k, st);
+      v.launch(G, mask, g, x[from], x[from ^ 1], tile_flags, tiles_x, tiles, k, st);
     }
   }
 
@@ -893,10 +909,14 @@ struct GridSolverImpl : Solver {
     return used;
   }
 
+  // Whether the caller is capturing the stream into a graph.
   bool capturing() const {
     cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
-    return cudaStreamIsCapturing(stream, &status) == cudaSuccess &&
-           status != cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &status) != cudaSuccess) {
+      cudaGetLastError();
+      return false;
+    }
+    return status != cudaStreamCaptureStatusNone;
   }
 
   void run_sweeps(int iters) {
@@ -906,8 +926,14 @@ struct GridSolverImpl : Solver {
       run_mixed(iters);
       return;
     }
-    const bool few = use_res() && few_sweeps(iters);
-    if (use_res() && !few) {
+    // Steps being captured, unless a kernel was named or tuned before, are
+    // launches of up to 16 sweeps: each goes on in the other buffer, so a graph
+    // of an even number of them advances the state at every replay, where a
+    // resident step always ends in the buffer it did not start in; and they
+    // need no memory that a step on another kernel had not allocated.
+    const bool cap = capturing(), recorded = cap && !pinned && !tuned;
+    const bool resident = use_res() && !recorded, few = resident && few_sweeps(iters);
+    if (resident && !few) {
       run_res(iters);
       return;
     }
@@ -915,21 +941,18 @@ struct GridSolverImpl : Solver {
                  "the grid's tiles do not fit on the device: no '" + res_pin + "' sweeps");
     if (few) {
       select_variant(default_variant());
+    } else if (recorded) {
+      select_variant(red_black ? red_black_variant() : launch_variant());
     } else if (!tuned && !pinned) {
       iters -= autotune(iters);
-    }
-    if (!few && !tuned && !pinned && !red_black) {
-      const int v = untuned_variant(iters);
-      // The flow kernel's tables are allocated on its first step, which a
-      // caller's capture would refuse.
-      select_variant(is_flow(v) && flow_cap == 0 && capturing() ? default_variant() : v);
+      if (!tuned && !red_black) select_variant(untuned_variant(iters));
     }
     untuned_sweeps += std::min(iters, kFlowFromLarge - untuned_sweeps);
     if (is_flow(variant)) {
       if (iters > 0) run_flow(iters);
       return;
     }
-    while (iters >= kChunk) {
+    while (!cap && iters >= kChunk) {  // a graph cannot be launched into a capture
       run_chunk();
       iters -= kChunk;
     }
@@ -970,7 +993,7 @@ struct GridSolverImpl : Solver {
       }
       launch_tile_flags(G, mask, v.tile_h, v.tile_w, v.depth, mtiles_x, mtiles, mflags, stream);
       post_launch(this);
-      mflags_ok = true;
+      mflags_ok = !capturing();
     }
   }
 

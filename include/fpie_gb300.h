@@ -165,7 +165,13 @@ int fpie_set_precision(fpie_solver* s, int precision);
 /* ---- device-resident forms (torch tensor handoff; no host copies) --------
  * Same meaning as the calls above, with all array pointers in device memory
  * of the solver's device.  The *_device step calls only enqueue work on the
- * solver's stream; img/err may be NULL to skip those outputs. */
+ * solver's stream; img/err may be NULL to skip those outputs.
+ * After one step outside it, a grid step can be captured into a CUDA graph.
+ * Unless a kernel was named or tuned before, it is recorded as launches of up
+ * to 16 sweeps, each of which goes on in the other of the state's two buffers:
+ * with an even number of them (17-32 or 49-64 sweeps, say) a replay goes on
+ * from the state the last one left, with an odd number it repeats the same
+ * sweeps.  A named resident kernel is one launch whatever the step's length. */
 int fpie_grid_reset_device(fpie_solver* s, int n, int m, const int32_t* mask,
                            const float* tgt, const float* grad);
 int fpie_grid_step_device(fpie_solver* s, int iteration, uint8_t* img,
