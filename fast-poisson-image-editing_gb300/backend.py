@@ -336,8 +336,9 @@ class GridSolver(_Solver):
         _abi.call("fpie_grid_set_kernel", self._h, name.encode())
 
     def set_spin_limit(self, spins: int) -> None:
-        """Polls a flow-kernel neighbourhood wait, or a TMA-kernel copy wait,
-        may take before the step fails with FpieTimeoutError."""
+        """Polls a flow-kernel neighbourhood wait, a resident kernel's wait for
+        its neighbours or a TMA-kernel copy wait may take before the step (or
+        solve) fails with FpieTimeoutError."""
         _abi.call("fpie_grid_set_spin_limit", self._h, ctypes.c_longlong(int(spins)))
 
     @property

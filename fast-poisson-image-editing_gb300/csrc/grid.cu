@@ -283,7 +283,9 @@ struct GridSolverImpl : Solver {
   void raise_waits() {
     int flag;
     std::memcpy(&flag, h_err + 3, sizeof flag);
-    if (!flag) return;
+    if (flag) raise_wait();
+  }
+  [[noreturn]] void raise_wait() {
     FPIE_CUDA(cudaMemsetAsync(d_wait_err, 0, sizeof(int), stream));
     FPIE_CUDA(cudaStreamSynchronize(stream));
     throw Error{FPIE_ERR_TIMEOUT, "sweep kernel: a bounded device wait gave up"};
@@ -325,7 +327,7 @@ struct GridSolverImpl : Solver {
   void* e[2] = {nullptr, nullptr};    // correction, FP16 or BF16 planes
   float* r = nullptr;                 // FP32 residual planes
   double* d_part6 = nullptr;          // per-block max|r|, sum|r| (double)
-  double* h_norm = nullptr;           // pinned: [max x3, sum x3], twice (solve_res)
+  double* h_norm = nullptr;           // pinned: [max x3, sum x3, wait flag], twice (solve_res)
   cudaEvent_t norm_done[2] = {nullptr, nullptr};
   uint8_t* mflags = nullptr;
   int mflags_cap = 0, mtiles_x = 0, mtiles = 0;
@@ -1174,13 +1176,16 @@ struct GridSolverImpl : Solver {
     post_launch(this);
   }
 
-  // Queues the norms of the current state into h_norm + 6 * slot.
+  // Queues the norms of the current state, and the wait flag behind them,
+  // into h_norm + kNorm * slot.
+  static constexpr int kNorm = 7;
   void queue_norms(int slot) {
     if (!d_part6) {
       FPIE_CUDA(cudaMalloc(&d_part6, (size_t)L.nparts * 6 * sizeof(double)));
     }
-    if (!h_norm) FPIE_CUDA(cudaMallocHost(&h_norm, 2 * 6 * sizeof(double)));
-    launch_norms(L, G, mask, g, x[cur], d_part6, finish_count(), h_norm + 6 * slot, stream);
+    if (!h_norm) FPIE_CUDA(cudaMallocHost(&h_norm, 2 * kNorm * sizeof(double)));
+    launch_norms(L, G, mask, g, x[cur], d_part6, finish_count(), h_norm + kNorm * slot, stream,
+                 d_wait_err);
     post_launch(this);
   }
 
@@ -1196,6 +1201,11 @@ struct GridSolverImpl : Solver {
     return std::max(nrm[0], std::max(nrm[1], nrm[2])) > tol;
   }
 
+  // A block whose kernel gave up waiting left a state whose norms mean nothing.
+  void check_norms(int slot) {
+    if (h_norm[kNorm * slot + 6] != 0.0) raise_wait();
+  }
+
   // Sweeps in blocks of `check_every` until every channel's max |r| <= tol
   // or max_sweeps are done; returns the sweeps run.
   int solve(double tol, int max_sweeps, int check_every) {
@@ -1205,11 +1215,13 @@ struct GridSolverImpl : Solver {
     int done = 0;
     double nrm[6];
     residual_norms(nrm);
+    check_norms(0);
     while (done < max_sweeps && beyond(nrm, tol)) {
       const int k = std::min(check_every, max_sweeps - done);
       run_sweeps(k);
       done += k;
       residual_norms(nrm);
+      check_norms(0);
     }
     return done;
   }
@@ -1228,13 +1240,14 @@ struct GridSolverImpl : Solver {
     for (;; slot ^= 1) {
       const int k = std::min(check_every, max_sweeps - done);
       if (k > 0) {
-        run_res(k, h_norm + 6 * slot, tol);
+        run_res(k, h_norm + kNorm * slot, tol);
         queue_norms(slot ^ 1);
         FPIE_CUDA(cudaEventRecord(norm_done[slot ^ 1], stream));
       }
       FPIE_CUDA(cudaEventSynchronize(norm_done[slot]));
+      check_norms(slot);
       if (k <= 0) break;
-      if (!beyond(h_norm + 6 * slot, tol)) {
+      if (!beyond(h_norm + kNorm * slot, tol)) {
         cur ^= 1;  // the queued block did nothing
         FPIE_CUDA(cudaStreamSynchronize(stream));
         break;

@@ -101,7 +101,8 @@ __device__ __forceinline__ void sum3_add(Sum3& s, float v) {
 __global__ void __launch_bounds__(256)
 grid_norms_kernel(GridGeom G, const uint8_t* __restrict__ mask, const float* __restrict__ g,
                   const float* __restrict__ x, double* __restrict__ parts,
-                  unsigned* __restrict__ count, double* __restrict__ out, int rows) {
+                  unsigned* __restrict__ count, double* __restrict__ out, const int* flag,
+                  int rows) {
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
   const int i0 = (blockIdx.y * blockDim.y + threadIdx.y) * rows;
   const int i1 = 4 * q < G.m ? min(i0 + rows, G.n) : i0;
@@ -176,7 +177,7 @@ grid_norms_kernel(GridGeom G, const uint8_t* __restrict__ mask, const float* __r
   __syncthreads();
   if (!last) return;
   __threadfence();
-  // Warp 0 per column of the partials: lanes stride over the blocks.
+  // A warp per column of the partials: lanes stride over the blocks.
   if (warp < 6) {
     double v = 0.0;
     for (unsigned k = lane; k < blocks; k += 32) {
@@ -190,7 +191,10 @@ grid_norms_kernel(GridGeom G, const uint8_t* __restrict__ mask, const float* __r
     }
     if (lane == 0) out[warp] = v;
   }
-  if (tid == 0) *count = 0;
+  if (tid == 0) {
+    if (flag) out[6] = (double)*(const volatile int*)flag;
+    *count = 0;
+  }
 }
 
 void launch_refine(int precision, dim3 grid, dim3 block, const GridGeom& G, const uint8_t* mask,
@@ -208,9 +212,10 @@ void launch_refine(int precision, dim3 grid, dim3 block, const GridGeom& G, cons
 }
 
 void launch_norms(const GridLaunch& L, const GridGeom& G, const uint8_t* mask, const float* g,
-                  const float* x, double* parts, unsigned* count, double* out, cudaStream_t st) {
+                  const float* x, double* parts, unsigned* count, double* out, cudaStream_t st,
+                  const int* flag) {
   grid_norms_kernel<<<L.finish_grid, L.finish_block, 0, st>>>(G, mask, g, x, parts, count, out,
-                                                              L.finish_rows);
+                                                              flag, L.finish_rows);
 }
 
 }  // namespace fpie

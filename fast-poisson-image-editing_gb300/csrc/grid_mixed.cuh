@@ -15,8 +15,9 @@ void launch_refine(int precision, dim3 grid, dim3 block, const GridGeom& G, cons
 
 // out[0..2] = max |residual| of x per channel, out[3..5] = sum |residual|
 // (device or pinned memory).  parts: 6 * L.nparts doubles of scratch; count: a
-// device word that is 0 between launches.
+// device word that is 0 between launches; flag, unless NULL, goes to out[6].
 void launch_norms(const GridLaunch& L, const GridGeom& G, const uint8_t* mask, const float* g,
-                  const float* x, double* parts, unsigned* count, double* out, cudaStream_t st);
+                  const float* x, double* parts, unsigned* count, double* out, cudaStream_t st,
+                  const int* flag = nullptr);
 
 }  // namespace fpie

@@ -291,10 +291,12 @@ int fpie_grid_solve(fpie_solver* s, double tol, int max_sweeps, int check_every,
 int fpie_grid_set_kernel(fpie_solver* s, const char* name);
 
 /* The dependency-flow kernels ("p16w8k16d", "p16w8k12d" and their "dp"
- * forms) wait for neighbour tiles to finish the previous level, the TMA
- * kernel ("p16w8k16t") for its region copies; each wait gives up after
- * `spins` polls (~64 ns apart), and the step (or fpie_sync) then returns
- * FPIE_ERR_TIMEOUT, leaving the state undefined.  Default 2^26. */
+ * forms) wait for neighbour tiles to finish the previous level, the resident
+ * kernels ("...r") for their neighbours' packets, the TMA kernel
+ * ("p16w8k16t") for its region copies; each wait gives up after `spins` polls
+ * (~64 ns apart; a resident kernel's after at most 2^23), and the step,
+ * fpie_grid_solve or fpie_sync then returns FPIE_ERR_TIMEOUT, leaving the
+ * state undefined.  Default 2^26. */
 int fpie_grid_set_spin_limit(fpie_solver* s, long long spins);
 
 /* Writes the current grid sweep kernel's name (NUL-terminated) into buf: the
