@@ -105,13 +105,11 @@ __device__ __noinline__ void batch_fold_item(const GridGeom& G, const uint8_t* m
 }
 
 // An FP32 item by the quartered update (quarter.cuh), for jobs whose values
-// are in its range; whether this thread stored a nonzero value below 2^-60,
+// are in its range; whether this thread stored a nonzero value below 2^-94,
 // from which the next level (16 sweeps) would not be exact.  Most regions of
 // small jobs hold unmasked pixels, for which the packed update selects bit by
 // bit: 4 jobs of up to 400x400 took 1,627 us on 64-row regions, now 1,331, 24
 // of them on 128-row regions 2,452, now 2,330.
-constexpr int kTinyItem = 60;
-
 template <int R, int W, int K, bool FULL>
 __device__ __noinline__ bool batch_quarter_item(const GridGeom& G, const uint8_t* mask,
                                                 const float* gc, const float* xc, float* oc,
@@ -160,7 +158,7 @@ __device__ __noinline__ bool batch_quarter_item(const GridGeom& G, const uint8_t
       }
     }
   }
-  return least < tiny_limit(kTinyItem);
+  return least < tiny_limit(kTiny);
 }
 
 template <int R, int W, int K, typename TS>
@@ -420,16 +418,16 @@ struct BatchJob {
 };
 
 // Sets *odd where a job's inputs are outside the quartered sweep's range:
-// values that are not finite, above 2^40 or nonzero below 2^-60, gradients of
-// masked pixels nonzero below 2^-38 (quarter.cuh).
+// values of the state or gradients of masked pixels that are not finite, above
+// 2^40 or nonzero below 2^-94 (quarter.cuh).
 __global__ void batch_range_kernel(long long px, const int32_t* __restrict__ mk,
                                    const float* __restrict__ t, const float* __restrict__ gr,
                                    unsigned* odd) {
   bool out = false;
   for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < 3 * px;
        k += (long long)gridDim.x * blockDim.x) {
-    out = out || !(fabsf(t[k]) <= 0x1p40f) || tiny_key(t[k]) < tiny_limit(kTinyItem);
-    if (mk[k / 3]) out = out || !(fabsf(gr[k]) <= 0x1p40f) || tiny_key(gr[k]) < tiny_limit(38);
+    out = out || !(fabsf(t[k]) <= 0x1p40f) || tiny_key(t[k]) < tiny_limit(kTiny);
+    if (mk[k / 3]) out = out || !(fabsf(gr[k]) <= 0x1p40f) || tiny_key(gr[k]) < tiny_limit(kTiny);
   }
   if (out) *odd = 1u;
 }

@@ -48,7 +48,7 @@ __global__ void grid_inputs_unpack_kernel(GridGeom G, const uint8_t* __restrict_
 // lie outside the range in which quartered sums are exact (quarter.cuh).
 __device__ __forceinline__ bool out_of_range(float v) { return !(fabsf(v) <= 0x1p40f); }
 __device__ __forceinline__ bool grad_out_of_range(float v) {
-  return out_of_range(v) || (v != 0.f && fabsf(v) < 0x1p-38f);
+  return out_of_range(v) || (v != 0.f && fabsf(v) < 0x1p-94f);
 }
 
 __global__ void grid_range_kernel(GridGeom G, const uint8_t* __restrict__ mask,

@@ -10,10 +10,10 @@
 // 0.266 us (0.71 as launches of 8 sweeps), 251x389 0.385 (0.83), 176x1457
 // 0.523 (0.83).
 //
-// The update is quarter.cuh's.  Each CTA looks for values below 2^-60 every
-// 16 sweeps, before an exchange if there is one; one that finds some takes slow
-// sweeps until its next look and marks the packets it sends, and a CTA that
-// receives a marked packet does the same.
+// The update is quarter.cuh's.  Each CTA looks for values below 2^-94 every
+// 16 sweeps, before an exchange if there is one; one that finds some takes
+// unquartered sweeps until its next look and marks the packets it sends, and a
+// CTA that receives a marked packet does the same.
 //
 // Exchange.  A packet is 16 bytes, three values and an epoch, in one 128-bit
 // store: the reader polls the packet itself, so data and readiness arrive
@@ -65,8 +65,7 @@ struct ResArgs {
   int tiles_x, tiles, sweeps;
 };
 
-constexpr int kCheck = 16;            // sweeps between range checks
-constexpr int kTiny = 60;     // and their limit, 2^-60: exact for 16 sweeps (quarter.cuh)
+constexpr int kCheck = 16;  // sweeps between looks for tiny values (quarter.cuh)
 
 // 128-bit relaxed accesses are single transactions.
 __device__ __forceinline__ void st_packet(uint4* p, float a, float b, float c, unsigned e) {
@@ -183,6 +182,13 @@ __global__ void __launch_bounds__(W * 32, 1) grid_res_kernel(ResArgs A) {
   const int ty = tile / A.tiles_x, tx = tile - ty * A.tiles_x;
   constexpr int ap = WHOLE ? 0 : K, al = WHOLE ? 1 : KL;
   constexpr int period = WHOLE ? kCheck : K;  // sweeps between exchanges
+  // Tiny values are swept by quarter_sweep in the reference's order rather than
+  // by slow_sweep: on an 802x802 grid half of it black 0.975 us a sweep against
+  // 1.11 (0.925 without tiny values, 1.00 on the flow kernel), 660x660 0.715
+  // against 0.815, 176x1457 0.545 against 0.68.  On the other shapes the second
+  // loop cost the first 1-5%, and slow sweeps there are 1-18% slower than it,
+  // twice as fast as the launches' all the same.
+  constexpr bool ORDERED = W == 8 && K != 8 && !WHOLE;
   const long long org = G.at(ty * TH - ap, tx * TW - 4 * al);  // the region's first pixel
   const long long base = org + (long long)(w * R) * G.pitch + 4 * lane;
   const long long co = c * G.plane;
@@ -376,6 +382,14 @@ __global__ void __launch_bounds__(W * 32, 1) grid_res_kernel(ResArgs A) {
         for (; s + 2 <= ks; s += 2) {
           quarter_sweep<R, NS, LW, false, true>(P, Gq, L, 0, lane, w, edge);
           quarter_sweep<R, NS, LW, false, false>(P, Gq, L, 1, lane, w, edge);
+        }
+      } else if (ORDERED && !s_wild && ks >= 2) {
+        post_edges<R, NS, LW>(P, 0, lane, w, edge);
+        __syncthreads();
+#pragma unroll 1
+        for (; s + 2 <= ks; s += 2) {
+          quarter_sweep<R, NS, LW, false, true, false>(P, Gq, L, 0, lane, w, edge);
+          quarter_sweep<R, NS, LW, false, false, false>(P, Gq, L, 1, lane, w, edge);
         }
       }
       // An odd last sweep takes this path too (the same values).

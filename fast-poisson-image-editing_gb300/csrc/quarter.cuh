@@ -13,19 +13,22 @@
 // takes two issue slots, so pairing rows gains nothing and costs register
 // moves; a multiplier register per pixel instead of the maximum, 880.)
 //
-// Where the scaling is exact.  A quartered partial sum is inexact only below
-// 2^-126, an unquartered one overflows only above 2^127, and -inf + inf is no
-// number.  The kernels therefore
+// Where the scaling is exact.  A quartered partial sum that is a multiple of
+// 2^-149 is a quarter of the unquartered one, rounded alike: below 2^-126 both
+// are exact, above both keep 24 bits.  An unquartered one overflows only above
+// 2^127, and -inf + inf is no number.  The kernels therefore
 //  (1) read a mark (`wild`) that a reset sets for inputs that are not finite,
-//      above 2^40, or (gradients) nonzero below 2^-38, and with it take
+//      above 2^40, or (gradients) nonzero below 2^-94, and with it take
 //      slow_sweep, the reference's order of operations, throughout.  Bounded
 //      inputs stay bounded: a sweep adds at most max|g| / 4.
-//  (2) look for nonzero values below a limit every few sweeps, and take slow
-//      sweeps where there are any.  Without any below 2^-e, and with the
-//      gradient's 2^-38, all values are multiples of 2^-(max(e, 38) + 23);
-//      every sweep makes that at most four times finer, so for n sweeps
-//      partial sums are multiples of 2^-(max(e, 38) + 23 + 2n), exact while
-//      that is at least 2^-126.
+//  (2) look for nonzero values below 2^-94 every 16 sweeps.  Without any, all
+//      values and gradients are multiples of 2^-117; every sweep makes that at
+//      most four times finer, so for 16 sweeps partial sums are multiples of
+//      2^-149.  With some, the resident kernel keeps the reference's order of
+//      additions (QUARTER false: six operations instead of five), the batch
+//      its packed update.  Such values are no rarity: on black without a
+//      gradient they run ahead of what diffuses into it (255 / 4^k at the k-th
+//      pixel), on 802x802 for thousands of sweeps.
 #pragma once
 
 #include "common.cuh"
@@ -34,6 +37,7 @@ namespace fpie {
 
 constexpr unsigned kMasked = 0x7fffffffu;   // L of a masked pixel (a NaN)
 constexpr unsigned kNegInf = 0xff800000u;   // g' of an unmasked pixel
+constexpr int kTiny = 94;                   // 2^-kTiny: the limit above
 
 // 2 * |bits| - 1 of v, so that zeros wrap to the top: compare with tiny_limit.
 __device__ __forceinline__ unsigned tiny_key(float v) { return 2u * __float_as_uint(v) - 1u; }
@@ -59,8 +63,10 @@ __device__ __forceinline__ void post_edges(const float (&P)[R][4], int par, int 
 // rows stored before the last rows' (fully masked region of 8 rows, 4 warps:
 // 302 cycles a sweep against 318 from the top row down; through an mbarrier
 // with arrival and wait apart, 424).
-// FULL: all of the region is masked.
-template <int R, int NS, int LW, bool FULL, bool FWD>
+// FULL: all of the region is masked.  !QUARTER: the reference's order, with
+// finite values only (an unmasked pixel's sum has to stay -inf); 4 g' + up
+// rounds as g + up does.
+template <int R, int NS, int LW, bool FULL, bool FWD, bool QUARTER = true>
 __device__ __forceinline__ void quarter_sweep(float (&P)[R][4], const float (&Gq)[R][4],
                                               const float (&L)[FULL ? 1 : R][4], int par, int lane,
                                               int w, float4 (&edge)[2][2][NS][LW]) {
@@ -85,7 +91,7 @@ __device__ __forceinline__ void quarter_sweep(float (&P)[R][4], const float (&Gq
                        : FWD && k > 0         ? keep[j]
                        : !FWD && k == R - 1   ? first[j]
                                               : P[i > 0 ? i - 1 : 0][j];
-      t[j] = __fmaf_rn(up, 0.25f, Gq[i][j]);
+      t[j] = QUARTER ? __fmaf_rn(up, 0.25f, Gq[i][j]) : __fmaf_rn(Gq[i][j], 4.f, up);
     }
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -93,14 +99,19 @@ __device__ __forceinline__ void quarter_sweep(float (&P)[R][4], const float (&Gq
                          : !FWD && k > 0        ? keep[j]
                          : FWD && k == R - 1    ? first[j]
                                                 : P[i < R - 1 ? i + 1 : i][j];
-      t[j] = __fmaf_rn(down, 0.25f, t[j]);
+      t[j] = QUARTER ? __fmaf_rn(down, 0.25f, t[j]) : __fadd_rn(t[j], down);
     }
 #pragma unroll
-    for (int j = 0; j < 4; ++j) t[j] = __fmaf_rn(j > 0 ? cur[j > 0 ? j - 1 : 0] : lf, 0.25f, t[j]);
+    for (int j = 0; j < 4; ++j) {
+      const float left = j > 0 ? cur[j > 0 ? j - 1 : 0] : lf;
+      t[j] = QUARTER ? __fmaf_rn(left, 0.25f, t[j]) : __fadd_rn(t[j], left);
+    }
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       keep[j] = cur[j];
-      const float o = __fmaf_rn(j < 3 ? cur[j < 3 ? j + 1 : 0] : rt, 0.25f, t[j]);
+      const float right = j < 3 ? cur[j < 3 ? j + 1 : 0] : rt;
+      const float o = QUARTER ? __fmaf_rn(right, 0.25f, t[j])
+                              : __fmul_rn(__fadd_rn(t[j], right), 0.25f);
       P[i][j] = FULL ? o : fmaxf(o, L[FULL ? 0 : i][j]);
     }
     if (i == (FWD ? 0 : R - 1)) post_edges<R, NS, LW>(P, par ^ 1, lane, w, edge);
@@ -108,8 +119,8 @@ __device__ __forceinline__ void quarter_sweep(float (&P)[R][4], const float (&Gq
   __syncthreads();
 }
 
-// The same sweep in the reference's order of operations, for values outside
-// the quartered form's range: gs * G is the gradient (gs 4, or 1 where G is
+// The same sweep in the reference's order of operations, for any values and
+// for a single sweep: gs * G is the gradient (gs 4, or 1 where G is
 // not quartered), `on(i, j)` tells the masked pixels.
 template <int R, int NS, int LW, typename On>
 __device__ __forceinline__ void slow_sweep(float (&P)[R][4], const float (&G)[R][4], On on,
