@@ -599,11 +599,14 @@ struct Batch {
           j.G, reinterpret_cast<int32_t*>(stage), reinterpret_cast<float*>(stage + px * 4),
           reinterpret_cast<float*>(stage + px * 16), j.mask, j.x[0], j.x[1], j.g);
       FPIE_CUDA(cudaGetLastError());
-      batch_range_kernel<<<blocks, 256, 0, stream>>>(
-          (long long)px, reinterpret_cast<int32_t*>(stage), reinterpret_cast<float*>(stage + px * 4),
-          reinterpret_cast<float*>(stage + px * 16), j.odd());
-      FPIE_CUDA(cudaGetLastError());
-      launches += 2;
+      ++launches;
+      if (precision == FPIE_FP32) {  // nothing else reads the mark
+        batch_range_kernel<<<blocks, 256, 0, stream>>>(
+            (long long)px, reinterpret_cast<int32_t*>(stage), reinterpret_cast<float*>(stage + px * 4),
+            reinterpret_cast<float*>(stage + px * 16), j.odd());
+        FPIE_CUDA(cudaGetLastError());
+        ++launches;
+      }
       FPIE_CUDA(cudaStreamSynchronize(stream));  // the caller may reuse its arrays
     } catch (...) {
       free_job(j);

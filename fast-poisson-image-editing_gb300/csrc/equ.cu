@@ -168,7 +168,7 @@ static int conv_blocks(long long total) { return stride_blocks(total, 256, 32); 
 
 Solver* new_grid_solver(int grid_x, int grid_y);
 void grid_reset_from_equ(Solver* s, cudaStream_t st, int n, int m, int N, const int* pos,
-                         const float* xe, const float* be, long long np);
+                         const float* xe, const float* be, long long np, bool in_range);
 void grid_to_equ(Solver* s, cudaStream_t st, int N, const int* pos, float* xe, long long np);
 void grid_run(Solver* s, cudaStream_t st, int iters);
 void grid_pin_kernel(Solver* s, const std::string& name);
@@ -481,12 +481,13 @@ struct EquSolverImpl : Solver {
   }
 
   // Moves the system into grid mode at crop size n x m (d_pos filled).
-  void enter_grid(int n, int m) {
+  // in_range: it comes from uint8 images.
+  void enter_grid(int n, int m, bool in_range = false) {
     if (!grid) grid = new_grid_solver(8, 8);
     grid_set_spin(grid, spin_limit);
     grid_set_red_black(grid, order == FPIE_ORDER_RED_BLACK);
     if (kernel_req != "auto") grid_pin_kernel(grid, kernel_req);
-    grid_reset_from_equ(grid, stream, n, m, E.N, d_pos, x[0], b, E.np);
+    grid_reset_from_equ(grid, stream, n, m, E.N, d_pos, x[0], b, E.np, in_range);
     use_grid = true;
     grid_newer = false;
   }
@@ -813,7 +814,7 @@ struct EquSolverImpl : Solver {
       equ_pos_kernel<<<conv_blocks(N), 256, 0, stream>>>(N, d_rows, d_cols, t_row + x0,
                                                           t_col + y0, m, d_pos);
       post_launch(this);
-      enter_grid(n, m);
+      enter_grid(n, m, true);
     }
     box_out[0] = t_row + x0;
     box_out[1] = t_row + x1;

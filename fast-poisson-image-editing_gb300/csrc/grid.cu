@@ -226,6 +226,7 @@ struct GridSolverImpl : Solver {
   unsigned* wild() const { return res_ctl + kResCtl; }
   unsigned* finish_count() const { return res_ctl + kResCtl + 1; }
   bool maybe_wild = false;      // the range mark may be set
+  bool range_due = false;       // the state may be out of range and was not looked at
 
   bool use_res() const {
     return precision == FPIE_FP32 && !red_black && res.rows > 0 && (!pinned || !res_pin.empty());
@@ -236,6 +237,10 @@ struct GridSolverImpl : Solver {
       const size_t b = res_exchange_bytes(G);
       FPIE_CUDA(cudaMalloc(&res_exchange, b));
       FPIE_CUDA(cudaMemsetAsync(res_exchange, 0, b, stream));
+    }
+    if (range_due) {
+      check_range();
+      range_due = capturing();  // recorded only: the next step looks again
     }
     waits = true;
     launch_res(G, res, mask, g, x[cur], x[cur ^ 1], res_exchange, res_ctl, wild(), iters,
@@ -256,10 +261,12 @@ struct GridSolverImpl : Solver {
     return few_steps++ > 0;
   }
 
-  // After a reset from floats (uint8 images are always in range).
+  // Before the first resident step after a reset from floats (uint8 images are
+  // always in range) or a change of precision; the other kernels do not need
+  // it (as a part of every reset it took 16 us of 52 on 1800x1800).  5-7 us.
   void check_range() {
     grid_range_kernel<<<conv_blocks((long long)G.n * ((G.m + 3) / 4)), 256, 0, stream>>>(
-        G, mask, x[0], g, wild());
+        G, mask, x[cur], g, wild());
     post_launch(this);
     maybe_wild = true;
   }
@@ -428,6 +435,7 @@ struct GridSolverImpl : Solver {
       // rewritten by the pack kernel.
       cur = 0;
       clear_wild();
+      range_due = false;
       ready = false;
       flags_ok = false;  // the new mask may activate other tiles
       mflags_ok = false;
@@ -464,7 +472,7 @@ struct GridSolverImpl : Solver {
     FPIE_CUDA(cudaMemsetAsync(arena, 0, l.clear, stream));
     d_wait_err = reinterpret_cast<int*>(d_err + 3);
     res_ctl = reinterpret_cast<unsigned*>(d_err + 4);
-    maybe_wild = false;
+    maybe_wild = range_due = false;
     res = res_pin.empty() ? res_pick(n, m) : res_named(res_pin.c_str(), n, m);
     cur = 0;
   }
@@ -474,7 +482,7 @@ struct GridSolverImpl : Solver {
     grid_pack_kernel<<<conv_blocks(total), 256, 0, stream>>>(
         G, dmask, dtgt, dgrad, mask, x[0], x[1], g);
     post_launch(this);
-    check_range();
+    range_due = true;
     ready = true;
   }
 
@@ -500,9 +508,9 @@ struct GridSolverImpl : Solver {
 
   // Loads an equation system that is a 4-neighbour raster stencil (see
   // grid_from_equ_kernel); the sweeps are then bit-identical to the
-  // system's gather sweeps.
+  // system's gather sweeps.  in_range: the system comes from uint8 images.
   void reset_from_equ(int n, int m, int N, const int* pos, const float* xe, const float* be,
-                      long long np) {
+                      long long np, bool in_range) {
     allocate(n, m);
     N_user = n * m;
     FPIE_CUDA(cudaMemsetAsync(arena, 0, plane_bytes, stream));
@@ -510,7 +518,7 @@ struct GridSolverImpl : Solver {
       grid_from_equ_kernel<<<conv_blocks(N), 256, 0, stream>>>(G, N, pos, xe, be, np, mask, x[0],
                                                                x[1], g);
       post_launch(this);
-      check_range();
+      range_due = !in_range;
     }
     ready = true;
   }
@@ -1338,6 +1346,7 @@ struct GridSolverImpl : Solver {
       precision = p;
       pinned = false;
       pin_res("");
+      range_due = true;
       drop_graphs();
     }
   }
@@ -1512,9 +1521,9 @@ void grid_set_precision(Solver* s, int p) { static_cast<GridSolverImpl*>(s)->set
 // Used by the equation solver to run raster-stencil systems on a grid; each
 // call enqueues on stream `st`.
 void grid_reset_from_equ(Solver* s, cudaStream_t st, int n, int m, int N, const int* pos,
-                         const float* xe, const float* be, long long np) {
+                         const float* xe, const float* be, long long np, bool in_range) {
   s->stream = st;
-  static_cast<GridSolverImpl*>(s)->reset_from_equ(n, m, N, pos, xe, be, np);
+  static_cast<GridSolverImpl*>(s)->reset_from_equ(n, m, N, pos, xe, be, np, in_range);
 }
 void grid_to_equ(Solver* s, cudaStream_t st, int N, const int* pos, float* xe, long long np) {
   s->stream = st;
