@@ -207,21 +207,43 @@ __device__ __forceinline__ void block_sum3(double& a, double& b, double& c) {
   }
 }
 
-// A sum of floats as hi + lo (Knuth's error-free addition): FP64 adds run at
-// about two per SM and cycle here, and the residual sum's made up most of the
-// finish kernels' time.  hi + lo is exact to about 2^-46 of the sum, which the
-// block partials and the total then carry in double.
-struct Sum2 {
-  float hi = 0.f, lo = 0.f;
+// A sum of floats as hi + mid + lo (Knuth's error-free addition), exact to
+// about 2^-70 of it: more than a sum of doubles keeps, without FP64 adds, which
+// run at about two per SM and cycle here.  The blocks' partials and the total
+// are doubles.  A finish of a 3603x3603 crop takes 104 us (297 with sums of
+// doubles and one row per thread), of 802x802 13.4 (26.4).
+struct Sum3 {
+  float hi = 0.f, mid = 0.f, lo = 0.f;
 };
-__device__ __forceinline__ void sum2_add(Sum2& s, float v) {
-  const float t = __fadd_rn(s.hi, v), b = __fsub_rn(t, s.hi);
-  s.lo = __fadd_rn(s.lo, __fadd_rn(__fsub_rn(s.hi, __fsub_rn(t, b)), __fsub_rn(v, b)));
-  s.hi = t;
+__device__ __forceinline__ float two_sum(float a, float b, float& err) {
+  const float t = __fadd_rn(a, b), c = __fsub_rn(t, a);
+  err = __fadd_rn(__fsub_rn(a, __fsub_rn(t, c)), __fsub_rn(b, c));
+  return t;
+}
+__device__ __forceinline__ void sum3_add(Sum3& s, float v) {
+  float e, f;
+  s.hi = two_sum(s.hi, v, e);
+  s.mid = two_sum(s.mid, e, f);
+  s.lo = __fadd_rn(s.lo, f);
+}
+__device__ __forceinline__ void sum3_join(Sum3& s, const Sum3& t) {
+  float e;
+  sum3_add(s, t.hi);
+  s.mid = two_sum(s.mid, t.mid, e);
+  s.lo = __fadd_rn(s.lo, __fadd_rn(t.lo, e));
+}
+// The warp's sum, in lane 0.
+__device__ __forceinline__ void sum3_warp(Sum3& s) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const Sum3 t{__shfl_down_sync(0xffffffffu, s.hi, o), __shfl_down_sync(0xffffffffu, s.mid, o),
+                 __shfl_down_sync(0xffffffffu, s.lo, o)};
+    sum3_join(s, t);
+  }
 }
 // The value; where hi overflowed or is no number, hi alone.
-__device__ __forceinline__ double sum2_value(const Sum2& s) {
-  return isfinite(s.hi) ? (double)s.hi + (double)s.lo : (double)s.hi;
+__device__ __forceinline__ double sum3_value(const Sum3& s) {
+  return isfinite(s.hi) ? ((double)s.hi + (double)s.mid) + (double)s.lo : (double)s.hi;
 }
 
 // Block-wide sums of acc[3] to parts[3 * block ...], and by the last block to
@@ -230,29 +252,29 @@ __device__ __forceinline__ double sum2_value(const Sum2& s) {
 // before the first launch; the last block clears it.  err may be pinned host
 // memory: then no copy follows (3-4 us of a step).  flag, unless NULL, goes to
 // err[3] with it.
-__device__ __forceinline__ void finish_sums(Sum2 (&acc)[3], unsigned block, unsigned blocks,
+__device__ __forceinline__ void finish_sums(Sum3 (&acc)[3], unsigned block, unsigned blocks,
                                             double* parts, unsigned* count, float* err,
                                             const int* flag) {
-  __shared__ double sh[3][8];
+  // Two warps per channel, each from half of the threads' sums: all warps
+  // reducing their own three channels was 120 joins a block instead of 48.
+  __shared__ Sum3 sums[3][256];
+  __shared__ double sh[3][2];
   __shared__ bool last;
   const int tid = threadIdx.x + threadIdx.y * blockDim.x, lane = tid & 31, warp = tid >> 5;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1)
+  for (int k = 0; k < 3; ++k) sums[k][tid] = acc[k];
+  __syncthreads();
+  if (warp < 6) {
+    const Sum3* from = sums[warp >> 1] + 128 * (warp & 1) + lane;
+    Sum3 s = from[0];
 #pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      const float h = __shfl_down_sync(0xffffffffu, acc[c].hi, o);
-      const float l = __shfl_down_sync(0xffffffffu, acc[c].lo, o);
-      sum2_add(acc[c], h);
-      acc[c].lo = __fadd_rn(acc[c].lo, l);
-    }
-  if (lane == 0)
-#pragma unroll
-    for (int c = 0; c < 3; ++c) sh[c][warp] = sum2_value(acc[c]);
+    for (int k = 32; k < 128; k += 32) sum3_join(s, from[k]);
+    sum3_warp(s);
+    if (lane == 0) sh[warp >> 1][warp & 1] = sum3_value(s);
+  }
   __syncthreads();
   if (tid < 3) {
-    double t = 0.0;
-    for (int w = 0; w < 8; ++w) t += sh[tid][w];
-    parts[3 * (size_t)block + tid] = t;
+    parts[3 * (size_t)block + tid] = sh[tid][0] + sh[tid][1];
     __threadfence();
   }
   __syncthreads();

@@ -146,7 +146,7 @@ equ_finish_kernel(EquGeom E, const int4* __restrict__ A,
                   uint8_t* __restrict__ img, double* __restrict__ parts,
                   unsigned* __restrict__ count, float* __restrict__ err, const int* flag) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  Sum2 acc[3];
+  Sum3 acc[3];
   if (i < E.N) {
     const int4 a = __ldg(A + i);
 #pragma unroll

@@ -82,7 +82,7 @@ grid_finish_kernel(GridGeom G, const uint8_t* __restrict__ mask,
                    const int* flag, int rows) {
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
   const int i0 = (blockIdx.y * blockDim.y + threadIdx.y) * rows;
-  Sum2 acc[3];
+  Sum3 acc[3];
   const int jn = max(0, min(4, G.m - 4 * q));
   const int i1 = min(i0 + rows, G.n);
   for (int i = i0; i < i1; ++i) {  // uniform per warp
@@ -102,10 +102,10 @@ grid_finish_kernel(GridGeom G, const uint8_t* __restrict__ mask,
           const float rt = __ldg(xc + p + 4);
           const float4 gg = ld4(g + c * G.plane + p);
           // Per-pixel |r| is exact float32 (numpy order).
-          if (mk & 0x000000ffu) sum2_add(acc[c], fabsf(grid_res(ce.x, gg.x, up.x, dn.x, lf, ce.y)));
-          if (mk & 0x0000ff00u) sum2_add(acc[c], fabsf(grid_res(ce.y, gg.y, up.y, dn.y, ce.x, ce.z)));
-          if (mk & 0x00ff0000u) sum2_add(acc[c], fabsf(grid_res(ce.z, gg.z, up.z, dn.z, ce.y, ce.w)));
-          if (mk & 0xff000000u) sum2_add(acc[c], fabsf(grid_res(ce.w, gg.w, up.w, dn.w, ce.z, rt)));
+          if (mk & 0x000000ffu) sum3_add(acc[c], fabsf(grid_res(ce.x, gg.x, up.x, dn.x, lf, ce.y)));
+          if (mk & 0x0000ff00u) sum3_add(acc[c], fabsf(grid_res(ce.y, gg.y, up.y, dn.y, ce.x, ce.z)));
+          if (mk & 0x00ff0000u) sum3_add(acc[c], fabsf(grid_res(ce.z, gg.z, up.z, dn.z, ce.y, ce.w)));
+          if (mk & 0xff000000u) sum3_add(acc[c], fabsf(grid_res(ce.w, gg.w, up.w, dn.w, ce.z, rt)));
         }
         b[c] = clip_u8(ce.x);
         b[3 + c] = clip_u8(ce.y);

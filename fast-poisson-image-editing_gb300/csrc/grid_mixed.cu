@@ -3,7 +3,7 @@
 // The FP32 solution x is kept; every cycle
 //   1. refine: x <- x + e (e: the correction, FP16 or BF16), then the FP32
 //      residual r = grad + up + down + left + right - 4x on masked pixels,
-//      with its per-channel max |r| and sum |r| reduced in FP64;
+//      with its per-channel max |r| and sum |r| in FP64;
 //   2. inner: Jacobi sweeps on the correction equation 4e - sum(e_nb) = r,
 //      e starting at 0 and kept at 0 on unmasked pixels, FP32 arithmetic,
 //      e stored in FP16/BF16 between launches (grid_tbp.cu, storage type TS).
@@ -74,26 +74,6 @@ grid_refine_kernel(GridGeom G, const uint8_t* __restrict__ mask, const float* __
 }
 
 // ---- residual norms ------------------------------------------------------------
-// A sum of floats as hi + mid + lo, exact to about 2^-70 of it: more than a sum
-// of doubles keeps, without FP64 adds (two per SM and cycle).  Values above
-// 2^90, whose float sum could overflow where a double's does not, are added in
-// double.
-struct Sum3 {
-  float hi = 0.f, mid = 0.f, lo = 0.f;
-  double big = 0.0;
-};
-__device__ __forceinline__ float two_sum(float a, float b, float& err) {
-  const float t = __fadd_rn(a, b), c = __fsub_rn(t, a);
-  err = __fadd_rn(__fsub_rn(a, __fsub_rn(t, c)), __fsub_rn(b, c));
-  return t;
-}
-__device__ __forceinline__ void sum3_add(Sum3& s, float v) {
-  float e, f;
-  s.hi = two_sum(s.hi, v, e);
-  s.mid = two_sum(s.mid, e, f);
-  s.lo = __fadd_rn(s.lo, f);
-}
-
 // max |r| and sum |r| per channel of the state x, out[0..2] and out[3..5]; the
 // last block to arrive reduces the blocks' partials (6 doubles each) in a fixed
 // order.  One launch: with a second one for the blocks and FP64 reductions a
@@ -108,6 +88,8 @@ grid_norms_kernel(GridGeom G, const uint8_t* __restrict__ mask, const float* __r
   const int i1 = 4 * q < G.m ? min(i0 + rows, G.n) : i0;
   float mx[3] = {0.f, 0.f, 0.f};
   Sum3 sm[3];
+  // Values above 2^90, whose float sum could overflow where a double's does not.
+  double huge[3] = {0.0, 0.0, 0.0};
   for (int i = i0; i < i1; ++i) {
     const long long p = G.at(i, 4 * q);
     const uint32_t mk = __ldg(reinterpret_cast<const uint32_t*>(mask + p));
@@ -126,7 +108,7 @@ grid_norms_kernel(GridGeom G, const uint8_t* __restrict__ mask, const float* __r
           const float v = fabsf(grid_res(xv[k + 1], gv[k], uv[k], dv[k], xv[k], xv[k + 2]));
           mx[c] = fmaxf(mx[c], v);
           if (v > 0x1p90f)
-            sm[c].big += (double)v;
+            huge[c] += (double)v;
           else
             sum3_add(sm[c], v);
         }
@@ -140,23 +122,14 @@ grid_norms_kernel(GridGeom G, const uint8_t* __restrict__ mask, const float* __r
   for (int c = 0; c < 3; ++c) {
     // Not negative and no NaN (a maximum drops them): bits order as values do.
     const float m = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(mx[c])));
-    const bool big = __any_sync(0xffffffffu, sm[c].big != 0.0);
+    const bool any = __any_sync(0xffffffffu, huge[c] != 0.0);
+    sum3_warp(sm[c]);
+    if (any)
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const float h = __shfl_down_sync(0xffffffffu, sm[c].hi, o);
-      const float d = __shfl_down_sync(0xffffffffu, sm[c].mid, o);
-      const float l = __shfl_down_sync(0xffffffffu, sm[c].lo, o);
-      sum3_add(sm[c], h);
-      float e;
-      sm[c].mid = two_sum(sm[c].mid, d, e);
-      sm[c].lo = __fadd_rn(sm[c].lo, __fadd_rn(l, e));
-      if (big) sm[c].big += __shfl_down_sync(0xffffffffu, sm[c].big, o);
-    }
+      for (int o = 16; o > 0; o >>= 1) huge[c] += __shfl_down_sync(0xffffffffu, huge[c], o);
     if (lane == 0) {
       shm[c][warp] = m;
-      shs[c][warp] = isfinite(sm[c].hi)
-                         ? (((double)sm[c].hi + (double)sm[c].mid) + (double)sm[c].lo) + sm[c].big
-                         : (double)sm[c].hi;
+      shs[c][warp] = sum3_value(sm[c]) + huge[c];
     }
   }
   __syncthreads();
