@@ -662,6 +662,7 @@ struct EquSolverImpl : Solver {
   void allocate(int N) {
     FPIE_REQUIRE(N >= 1, FPIE_ERR_ARG, "N must be at least 1");
     FPIE_REQUIRE(N <= (1 << 29), FPIE_ERR_ARG, "N too large");
+    index_ok = false;
     if (A && E.N == N) {  // same size: keep buffers and captured graphs
       cur = 0;
       ready = false;
@@ -730,6 +731,7 @@ struct EquSolverImpl : Solver {
   int* d_rows = nullptr;
   int* d_cols = nullptr;
   int idx_cap = 0;
+  bool index_ok = false;  // they belong to the system loaded
 
   void ensure_index(int unknowns) {
     if (unknowns <= idx_cap && d_rows) return;
@@ -806,7 +808,7 @@ struct EquSolverImpl : Solver {
     launch_equ_build(m01, mw, x0, y0, n, m, ids, dsrc, sw, s_row + x0, s_col + y0, dtgt, tw,
                      t_row + x0, t_col + y0, mode, E.np, A, x[0], x[1], b, d_rows, d_cols, stream);
     post_launch(this);
-    ready = true;
+    ready = index_ok = true;
     use_grid = false;
     lay_N = 0;  // d_pos is rewritten below; the cached placement no longer matches d_occ
     if (kernel_req != "gather" && N > 1) {  // a mask's system: its pixels are known
@@ -826,7 +828,7 @@ struct EquSolverImpl : Solver {
 
   void check_index(const void* rows, const void* cols) const {
     FPIE_REQUIRE(rows && cols, FPIE_ERR_ARG, "null output array");
-    FPIE_REQUIRE(ready && d_rows && E.N - 1 <= idx_cap, FPIE_ERR_STATE,
+    FPIE_REQUIRE(ready && index_ok, FPIE_ERR_STATE,
                  "no index: the solver was not reset from images");
   }
 
