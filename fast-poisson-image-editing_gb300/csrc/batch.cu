@@ -682,7 +682,7 @@ struct Batch {
       const uint8_t* dtgt = reinterpret_cast<uint8_t*>(stage + al(sb));
       const uint8_t* dm01 = reinterpret_cast<uint8_t*>(stage + al(sb) + al(tb));
       PrepArgs a{j.G, dm01, mw, x0, y0, dsrc, sw, s_row + x0, s_col + y0, dtgt, tw, t_row + x0,
-                 t_col + y0, mode};
+                 t_col + y0, mode, sh, th};
       launch_prep_grid(a, j.mask, j.x[0], j.x[1], j.g, stream);
       FPIE_CUDA(cudaGetLastError());
       ++launches;

@@ -586,7 +586,7 @@ struct GridSolverImpl : Solver {
     allocate(x1 - x0, y1 - y0);
     N_user = G.n * G.m;
     PrepArgs a{G, m01, mw, x0, y0, dsrc, sw, s_row + x0, s_col + y0, dtgt, tw, t_row + x0,
-               t_col + y0, mode};
+               t_col + y0, mode, sh, th};
     launch_prep_grid(a, mask, x[0], x[1], g, stream);
     post_launch(this);
     ready = true;

@@ -126,18 +126,28 @@ __device__ __forceinline__ int mix_int(int a, int b, int mode) {
   return abs(a) < abs(b) ? b : a;
 }
 
-// 6 pixels (18 bytes) of an image row from byte `a` on, as 5 words; only
-// words holding bytes of [lo, hi) are read.
+// 6 pixels (18 bytes) of an image row from byte `a` on, as 5 words, of which
+// the bytes in [lo, hi) are used.  Words are read where all of them lie in the
+// image [im, end), bytes at its first and last pixels.
 __device__ __forceinline__ void load_px6(const uint8_t* a, const uint8_t* lo, const uint8_t* hi,
-                                         unsigned (&o)[5]) {
+                                         const uint8_t* im, const uint8_t* end, unsigned (&o)[5]) {
   const unsigned sh = 8 * (unsigned)(reinterpret_cast<uintptr_t>(a) & 3);
   const uint8_t* w = a - (sh >> 3);
   unsigned v[6];
+  if (w >= im && w + 24 <= end) {
 #pragma unroll
-  for (int k = 0; k < 6; ++k)
-    v[k] = w + 4 * k + 3 >= lo && w + 4 * k < hi
-               ? __ldg(reinterpret_cast<const unsigned*>(w + 4 * k))
-               : 0u;
+    for (int k = 0; k < 6; ++k) v[k] = __ldg(reinterpret_cast<const unsigned*>(w + 4 * k));
+  } else {
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
+      v[k] = 0;
+#pragma unroll
+      for (int b = 0; b < 4; ++b) {
+        const uint8_t* p = w + 4 * k + b;
+        if (p >= lo && p < hi) v[k] |= (unsigned)__ldg(p) << (8 * b);
+      }
+    }
+  }
 #pragma unroll
   for (int k = 0; k < 5; ++k) o[k] = __funnelshift_r(v[k], v[k + 1], sh);
 }
@@ -158,23 +168,23 @@ prep_grid_kernel(PrepArgs A, uint8_t* __restrict__ mask, float* __restrict__ xa,
   const int i0 = (blockIdx.y * 4 + (threadIdx.x >> 6)) * rows;
   if (j0 >= G.m || i0 >= G.n) return;
   const int cl = max(j0 - 1, 0), cr = min(j0 + 5, G.m);  // crop columns read
-  auto row = [&](const uint8_t* im, int w, int r0, int c0, int i, unsigned (&o)[5]) {
+  auto row = [&](const uint8_t* im, int h, int w, int r0, int c0, int i, unsigned (&o)[5]) {
     const uint8_t* p = im + ((long long)(r0 + i) * w + c0) * 3;
-    load_px6(p + 3 * (j0 - 1), p + 3 * cl, p + 3 * cr, o);
+    load_px6(p + 3 * (j0 - 1), p + 3 * cl, p + 3 * cr, im, im + (long long)h * w * 3, o);
   };
   unsigned su[5] = {}, sc[5], sd[5] = {}, tu[5] = {}, tc[5], td[5] = {};
   if (i0 > 0) {
-    row(A.src, A.sw, A.sx, A.sy, i0 - 1, su);
-    row(A.tgt, A.tw, A.tx, A.ty, i0 - 1, tu);
+    row(A.src, A.sh, A.sw, A.sx, A.sy, i0 - 1, su);
+    row(A.tgt, A.th, A.tw, A.tx, A.ty, i0 - 1, tu);
   }
-  row(A.src, A.sw, A.sx, A.sy, i0, sc);
-  row(A.tgt, A.tw, A.tx, A.ty, i0, tc);
+  row(A.src, A.sh, A.sw, A.sx, A.sy, i0, sc);
+  row(A.tgt, A.th, A.tw, A.tx, A.ty, i0, tc);
   const int i1 = min(i0 + rows, G.n);
   const float scale = A.mode == 1 ? 0.5f : 1.0f;
   for (int i = i0; i < i1; ++i) {
     if (i + 1 < G.n) {
-      row(A.src, A.sw, A.sx, A.sy, i + 1, sd);
-      row(A.tgt, A.tw, A.tx, A.ty, i + 1, td);
+      row(A.src, A.sh, A.sw, A.sx, A.sy, i + 1, sd);
+      row(A.tgt, A.th, A.tw, A.tx, A.ty, i + 1, td);
     }
     const uint8_t* mr = A.m01 + (long long)(A.x0 + i) * A.mw + A.y0 + j0;
     unsigned on = 0;

@@ -16,6 +16,7 @@ struct PrepArgs {
   const uint8_t* tgt;
   int tw, tx, ty;  // target width, crop origin in target coordinates
   int mode;        // gradient: 0 'src', 1 'avg', 2 'max'
+  int sh, th;      // source, target height
 };
 
 // Thresholds the mask (3 channels: channel sum >= 384; 1 channel: >= 128),
