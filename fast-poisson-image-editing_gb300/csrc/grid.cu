@@ -1046,8 +1046,7 @@ struct GridSolverImpl : Solver {
   // Adds the pending correction to x (end of a step).
   void mixed_flush(cudaStream_t st) {
     if (!e_pending) return;
-    launch_refine(precision, L.sweep_grid, L.sweep_block, G, mask, g, x[cur], e[e_last],
-                  x[cur ^ 1], nullptr, st);
+    launch_fold(precision, L, G, mask, x[cur], e[e_last], x[cur ^ 1], st);
     cur ^= 1;
     e_pending = false;
   }

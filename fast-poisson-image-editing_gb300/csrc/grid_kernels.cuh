@@ -9,7 +9,7 @@ struct GridLaunch {
   dim3 sweep_block, sweep_grid;    // one-sweep kernel
   dim3 finish_block, finish_grid;  // residual + image kernel
   int finish_rows;                 // rows per thread of the latter
-  int nparts;                      // residual partials (finish blocks)
+  int nparts;                      // residual partials: sweep_grid's blocks, finish_grid has no more
 };
 
 GridLaunch grid_launch(const GridGeom& G);
