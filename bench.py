@@ -155,17 +155,20 @@ def kernel_shape(kernel: str, sweeps: int):
 FP32_OPS_PER_UPDATE = 15  # per pixel update: 4 additions + 1 multiplication, 3 channels
 
 
-def apron_factor(kernel: str) -> float:
+def apron_factor(kernel: str, crop: tuple[int, int] | None = None) -> float:
     """Region pixels a temporally blocked kernel sweeps per tile pixel it
     writes: regions are W*R rows x 128 columns (or as wide as named, with as
     many pixels), tiles lose K pixels (2K for red-black levels) on every side;
-    1 for the one-sweep kernel."""
+    1 for the one-sweep kernel.  A resident kernel whose region holds the whole
+    crop (rows, columns) has no apron but 4 columns on either side."""
     m = re.match(r"(rb|p)(\d+)w(\d+)(?:x(\d+))?k(\d+)", kernel)
     if not m:
         return 1.0
     r, w, width, k = (int(v or 128) for v in m.groups()[1:])
     k = 2 * k if m.group(1) == "rb" else k
     rows = r * w * 128 // width
+    if kernel.endswith("r") and crop and crop[0] <= rows and crop[1] <= width - 8:
+        return width / (width - 8)
     return rows * width / ((rows - 2 * k) * (width - 2 * k))
 
 
@@ -177,8 +180,8 @@ def fp32_peaks(stream_handle: int) -> dict:
     return {k: _abi.fp32_rate(k, stream=stream_handle) for k in ("fadd2", "ffma2", "fadd")}
 
 
-def grid_roofline(kernel: str, crop_px: int, unknowns: int, sweeps: int, avg_launch_s: float,
-                  peaks: dict, traffic) -> dict:
+def grid_roofline(kernel: str, crop: tuple[int, int], unknowns: int, sweeps: int,
+                  avg_launch_s: float, peaks: dict, traffic) -> dict:
     """Roofline object of a grid sweep kernel.  The bound is FP32 issue: the
     useful work of a launch is 15 FP32 operations per pixel update (masked
     pixels only), divided by the launch's average duration, against the
@@ -187,11 +190,12 @@ def grid_roofline(kernel: str, crop_px: int, unknowns: int, sweeps: int, avg_lau
     bandwidth when sweeps stay in registers) and `hbm_compulsory` (one read
     of x/grad/mask and one write of x per pass over the regions)."""
     per_launch, _, passes = kernel_shape(kernel, sweeps)
+    crop_px = crop[0] * crop[1]
     hbm, hbm_kind = measured_peak()
     ops = FP32_OPS_PER_UPDATE * unknowns * per_launch
     achieved = ops / avg_launch_s
     peak = peaks["fadd2"]
-    af = apron_factor(kernel)
+    af = apron_factor(kernel, crop)
     alg_bytes = GRID_BYTES_PER_PX * crop_px * per_launch
     eff = alg_bytes / avg_launch_s / 1e9
     comp = GRID_BYTES_PER_PX * crop_px * passes / avg_launch_s / 1e9
@@ -703,7 +707,7 @@ def large_grid_leg(stream, steps: int = 3, kernel: str = "auto") -> dict:
     pb = workloads.circle1800()
     mc, t, g, _ = prep.grid_inputs(pb.src, pb.mask, pb.tgt, pb.mask_on_src, pb.mask_on_tgt,
                                    pb.gradient)
-    unknowns, crop_px = int((mc != 0).sum()), int(mc.size)
+    unknowns = int((mc != 0).sum())
     dev = torch.device("cuda", torch.cuda.current_device())
     dm, dt_, dg = (torch.from_numpy(a).to(dev) for a in (mc, t, g))
     img = torch.empty((*mc.shape, 3), dtype=torch.uint8, device=dev)
@@ -739,7 +743,7 @@ def large_grid_leg(stream, steps: int = 3, kernel: str = "auto") -> dict:
            "ms_per_step": step_ms, "us_per_sweep": sweep_ms * 1e3 / SWEEPS, "steps": steps,
            "kernel": kernel, "gpu_launches": (s.launches - l0) // steps,
            "l2": "not flushed: the ~480 MB working set is larger than L2",
-           "roofline": grid_roofline(kernel, crop_px, unknowns, SWEEPS, avg_launch_s,
+           "roofline": grid_roofline(kernel, mc.shape, unknowns, SWEEPS, avg_launch_s,
                                      fp32_peaks(stream.cuda_stream),
                                      profiled_traffic(f"grid_{kernel}_circle1800"))}
     s.close()
@@ -1043,7 +1047,7 @@ def run_gb300(args):
                             "api": "GridSolver.reset_images(pinned uint8 src/mask/tgt) + "
                                    "GridSolver.step(5000)",
                             "ms_per_step": e2e_img_dt * 1e3},
-        "roofline": grid_roofline(kernel, crop_px, unknowns, sweeps, avg_launch_s, peaks,
+        "roofline": grid_roofline(kernel, (n, m), unknowns, sweeps, avg_launch_s, peaks,
                                   profiled_traffic(f"grid_{kernel}_square800")),
         "clocks": clk,
         "parity": {"timed_output_equals_fresh_solve": same},
