@@ -907,25 +907,46 @@ struct Batch {
     return ids;
   }
 
-  // Which variant runs the listed jobs, unless one was named.  A launch is
-  // bound either by the chain of levels of its longest job (an item's latency
-  // per level: 11.5 us for "p16w8k16", 7.2 us for "p8w8k16", whose warps hold
-  // half the rows) or by the SMs' throughput, where the small regions' wider
-  // aprons cost more (2.7 region pixels per pixel of a tile instead of 1.8).
-  // Measured with up to 48 uneven jobs, us per launch, items per level of
-  // "p8w8k16" in brackets, FP32: [78] 1,331 against 2,132, [231] 1,717
-  // against 2,126, [279] 1,876 against 2,210, [429] 2,689 against 2,330,
+  // Which variant runs `sw` more sweeps of the listed jobs, unless one was named.
+  // A launch is bound either by the chain of levels of its longest job (an
+  // item's latency per level: 11.8 us for "p16w8k16", 7.4 us for "p8w8k16",
+  // whose warps hold half the rows) or by the SMs' throughput, where the small
+  // regions' wider aprons cost more (2.7 region pixels per pixel of a tile
+  // instead of 1.8).  Measured with up to 48 uneven jobs, us per launch, items
+  // per level of "p8w8k16" in brackets, FP32: [78] 1,331 against 2,132, [231]
+  // 1,717 against 2,126, [279] 1,876 against 2,210, [429] 2,689 against 2,330,
   // [447] 2,725 against 2,591; FP16 [78] 1,701 against 2,685, [333] 2,635
   // against 2,533: the line lies at two items per SM.
-  int pick(const std::vector<int>& ids) {
-    const size_t small = 3;  // "p8w8k16" in batch_variants()
+  // Beyond it, tiles of 112x112 with half the depth ("p16w8k8") against 96x96
+  // depends on how the jobs' sides divide, a job of 110x110 being one tile or
+  // four: 50 of them took 1,432 us for 1,024 sweeps against 2,695, 64 of
+  // 300x300 15,228 against 16,800, 12 of 600x600 10,449 against 9,934.  The
+  // times per 16 sweeps below, of a level in the chain and of an item when all
+  // SMs are busy, were fitted to 25 such mixes in each precision and pick the
+  // better one or lose up to 8% to it.  Jobs of at most 96 rows are one row of
+  // tiles, whose unused rows 16 warps of 8 leave out more finely than 8 of 16:
+  // 50 of 90x90 in FP16 1,175 us against 1,236 (FP32 1,088 against 1,036, whose
+  // quartered items have no 16-warp form).
+  int pick(const std::vector<int>& ids, const std::vector<int>& sw) {
+    const int deep = 0, fine = 1, wide = 2, small = 3;  // in batch_variants()
+    const bool mixed = precision != FPIE_FP32;
     long long items = 0;
-    for (int id : ids) {
-      BatchJob& j = jobs[id];
+    double deep_work = 0.0, wide_work = 0.0, longest = 0.0;
+    int rows = 0;
+    for (size_t k = 0; k < ids.size(); ++k) {
+      BatchJob& j = jobs[ids[k]];
       if (j.tiles_of.size() != batch_variants().size()) tile_lists(j);
       items += 3LL * (long long)j.tiles_of[small].size();
+      deep_work += 3.0 * sw[k] * (double)j.tiles_of[deep].size();
+      wide_work += 3.0 * sw[k] * (double)j.tiles_of[wide].size();
+      longest = std::max(longest, (double)sw[k]);
+      rows = std::max(rows, j.n);
     }
-    return items <= 2LL * sms ? (int)small : 0;
+    if (items <= 2LL * sms) return small;
+    const double deep_us = std::max((mixed ? 16.0 : 13.1) * longest, (mixed ? 15.9 : 13.5) * deep_work / sms);
+    const double wide_us = std::max((mixed ? 20.2 : 17.6) * longest, (mixed ? 20.8 : 20.6) * wide_work / sms);
+    if (wide_us < deep_us) return wide;
+    return mixed && rows <= 96 ? fine : deep;
   }
 
   // Advances every live job by min(limit, its remaining sweeps); limit < 0
@@ -939,7 +960,7 @@ struct Batch {
       if (rem > 0) { run_ids.push_back(id); sw.push_back(rem); }
     }
     if (run_ids.empty()) return;
-    if (!pinned) variant = pick(run_ids);
+    if (!pinned) variant = pick(run_ids, sw);
     launch(run_ids, sw, variant, async);
   }
 

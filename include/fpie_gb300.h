@@ -348,7 +348,7 @@ int fpie_grid_step_noalloc(int n, int m, const int32_t* mask, float* x,
  * fpie_batch_run advances every job by min(max_sweeps, its remaining
  * sweeps) (max_sweeps < 0: to completion) in one persistent kernel whose
  * CTAs pull (job, tile, channel, level) items from a queue; the tile shape
- * follows from the number of items the run has for each SM.  A job's result is bit-identical to a GridSolver run of the same
+ * follows from the jobs' sides and sweeps (fpie_batch_set_kernel).  A job's result is bit-identical to a GridSolver run of the same
  * sweeps.  Dependency waits inside the kernel are bounded: past the spin
  * limit the call returns FPIE_ERR_TIMEOUT and the jobs' states are
  * undefined (remove and re-add them). */
@@ -404,9 +404,10 @@ int fpie_batch_state(fpie_batch* b, int job, float* out);
 int fpie_batch_norms(fpie_batch* b, const int* jobs, int count, double* out);
 int fpie_batch_remove(fpie_batch* b, int job);
 int fpie_batch_memory(fpie_batch* b, double* used, double* budget);
-/* "auto" (default: "p8w8k16" for runs of at most two of its items per SM,
- * "p16w8k16" for larger ones) or a variant name ("p16w8k16", "p8w16k16",
- * "p16w8k8", "p8w8k16"). */
+/* "auto" (default: "p8w8k16" for runs of at most two of its items per SM;
+ * larger ones "p16w8k16" or "p16w8k8", whichever's tiles the jobs divide into
+ * with less work, and "p8w16k16" instead of the former for mixed jobs of at
+ * most 96 rows) or a variant name. */
 int fpie_batch_set_kernel(fpie_batch* b, const char* name);
 int fpie_batch_kernel(fpie_batch* b, char* buf, int len);
 /* Iterations (about 128 ns each) a CTA may wait for a dependency. */
