@@ -66,6 +66,9 @@ struct BQueue {
   long long spin_limit;
 };
 
+// Levels and jobs whose tables a CTA keeps in shared memory.
+constexpr int kQueueLevels = 640, kQueueJobs = 320;
+
 __device__ __forceinline__ int ld_acquire_gpu(const int* p) {
   int v;
   asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
@@ -186,7 +189,7 @@ batch_persistent_kernel(BQueue Q) {
   // The queue tables, in shared memory when they fit: decoding an item is
   // two binary searches, which through global memory would be ~20 dependent
   // L2 round trips on every item's critical path.
-  constexpr int kSL = 640, kSJ = 320;
+  constexpr int kSL = kQueueLevels, kSJ = kQueueJobs;
   __shared__ float4 edge[2][2][W][32];
   __shared__ long long s_lo[kSL + 1], s_ct[kSJ + 1];
   __shared__ int s_act[kSL], s_order[kSJ];
@@ -414,6 +417,8 @@ struct BatchJob {
   // job never changes).
   std::vector<std::vector<int2>> tiles_of;
   std::vector<int> tiles_x_of;
+  std::vector<double> work_of;  // the list's items of a channel, a tile counting half
+                                // and half by its region's share of warps with rows
   void* block = nullptr;  // holds all of the following
   float* x[2] = {nullptr, nullptr};
   float* g = nullptr;
@@ -751,6 +756,7 @@ struct Batch {
     const auto& vs = batch_variants();
     j.tiles_of.assign(vs.size(), {});
     j.tiles_x_of.assign(vs.size(), -1);
+    j.work_of.assign(vs.size(), 0.0);
     for (size_t vi = 0; vi < vs.size(); ++vi) {
       const BatchVariant& v = vs[vi];
       const int tiles_x = (m + v.tile_w - 1) / v.tile_w;
@@ -765,6 +771,8 @@ struct Batch {
           const bool inside = R0 >= 0 && C0 >= 0 && R1 <= n && C1 <= m;
           const bool all = inside && count(R0, R1, C0, C1) == (long long)(R1 - R0) * (C1 - C0);
           out.push_back(make_int2(ty * tiles_x + tx, all ? 2 : 1));
+          const int warps = (std::min(R1, n) - std::max(R0, 0) + v.rows - 1) / v.rows;
+          j.work_of[vi] += 0.5 + 0.5 * std::min(warps, v.warps) / v.warps;
         }
       j.tiles_x_of[vi] = tiles_x;
     }
@@ -922,31 +930,36 @@ struct Batch {
   // four: 50 of them took 1,432 us for 1,024 sweeps against 2,695, 64 of
   // 300x300 15,228 against 16,800, 12 of 600x600 10,449 against 9,934.  The
   // times per 16 sweeps below, of a level in the chain and of an item when all
-  // SMs are busy, were fitted to 25 such mixes in each precision and pick the
-  // better one or lose up to 8% to it.  Jobs of at most 96 rows are one row of
-  // tiles, whose unused rows 16 warps of 8 leave out more finely than 8 of 16:
-  // 50 of 90x90 in FP16 1,175 us against 1,236 (FP32 1,088 against 1,036, whose
-  // quartered items have no 16-warp form).
+  // SMs are busy, were fitted to 51 such mixes in each precision and pick the
+  // better one but for 8 of 194x194 in FP32 (1,228 us against 1,140).  Twice the
+  // levels must still fit the queue tables in shared memory: 256 uneven jobs of
+  // up to 10,000 sweeps took 706 ms in FP16 against 558.
+  // Mixed jobs of at most 96 rows, one row of tiles, are 3-6% faster with 16
+  // warps of 8 rows ("p8w16k16") than with 8 of 16, larger ones 2-4% slower: 50
+  // of 90x90 in FP16 1,175 us against 1,236, 64 of 300x300 20,973 against 20,517
+  // (in FP32 the quartered items have no 16-warp form).
   int pick(const std::vector<int>& ids, const std::vector<int>& sw) {
     const int deep = 0, fine = 1, wide = 2, small = 3;  // in batch_variants()
     const bool mixed = precision != FPIE_FP32;
     long long items = 0;
     double deep_work = 0.0, wide_work = 0.0, longest = 0.0;
-    int rows = 0;
+    double low_work = 0.0;  // in jobs of one row of tiles
+    int wide_levels = 0;
     for (size_t k = 0; k < ids.size(); ++k) {
       BatchJob& j = jobs[ids[k]];
       if (j.tiles_of.size() != batch_variants().size()) tile_lists(j);
       items += 3LL * (long long)j.tiles_of[small].size();
-      deep_work += 3.0 * sw[k] * (double)j.tiles_of[deep].size();
-      wide_work += 3.0 * sw[k] * (double)j.tiles_of[wide].size();
+      deep_work += 3.0 * sw[k] * j.work_of[deep];
+      wide_work += 3.0 * sw[k] * j.work_of[wide];
       longest = std::max(longest, (double)sw[k]);
-      rows = std::max(rows, j.n);
+      wide_levels = std::max(wide_levels, mixed ? mixed_levels(sw[k], 8) : (sw[k] + 7) / 8);
+      if (j.n <= batch_variants()[fine].tile_h) low_work += 3.0 * sw[k] * j.work_of[deep];
     }
     if (items <= 2LL * sms) return small;
-    const double deep_us = std::max((mixed ? 16.0 : 13.1) * longest, (mixed ? 15.9 : 13.5) * deep_work / sms);
-    const double wide_us = std::max((mixed ? 20.2 : 17.6) * longest, (mixed ? 20.8 : 20.6) * wide_work / sms);
-    if (wide_us < deep_us) return wide;
-    return mixed && rows <= 96 ? fine : deep;
+    const double deep_us = std::max((mixed ? 15.9 : 13.0) * longest, (mixed ? 19.0 : 15.6) * deep_work / sms);
+    const double wide_us = std::max((mixed ? 20.1 : 17.3) * longest, (mixed ? 25.4 : 22.0) * wide_work / sms);
+    if (wide_us < deep_us && wide_levels <= kQueueLevels) return wide;
+    return mixed && 2.0 * low_work > deep_work ? fine : deep;
   }
 
   // Advances every live job by min(limit, its remaining sweeps); limit < 0

@@ -406,8 +406,8 @@ int fpie_batch_remove(fpie_batch* b, int job);
 int fpie_batch_memory(fpie_batch* b, double* used, double* budget);
 /* "auto" (default: "p8w8k16" for runs of at most two of its items per SM;
  * larger ones "p16w8k16" or "p16w8k8", whichever's tiles the jobs divide into
- * with less work, and "p8w16k16" instead of the former for mixed jobs of at
- * most 96 rows) or a variant name. */
+ * with less work, and "p8w16k16" instead of the former where most of the work
+ * is in mixed jobs of at most 96 rows) or a variant name. */
 int fpie_batch_set_kernel(fpie_batch* b, const char* name);
 int fpie_batch_kernel(fpie_batch* b, char* buf, int len);
 /* Iterations (about 128 ns each) a CTA may wait for a dependency. */

@@ -82,3 +82,18 @@ def test_epochs_of_an_emptying_batch():
         o = cjacobi.CGrid(mask, t, g)
         o.sweep(sweeps)
         np.testing.assert_array_equal(b.state(jid), o.x)
+
+
+@pytest.mark.parametrize("sweeps,kernel", [(5120, "p16w8k8"), (5121, "p16w8k16")])
+def test_levels_that_do_not_fit_the_queue_tables(sweeps, kernel):
+    from fpie_gb300.batch import BatchSolver
+
+    jobs = [_job(100, 105, k) for k in range(60)]
+    b = BatchSolver(8e9)
+    ids = [b.add(*j, sweeps) for j in jobs]
+    b.run()
+    assert b.kernel == kernel
+    for k in (7, 30):
+        o = cjacobi.CGrid(*jobs[k])
+        o.sweep(sweeps)
+        np.testing.assert_array_equal(b.state(ids[k]), o.x)
