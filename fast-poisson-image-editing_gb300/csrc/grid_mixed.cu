@@ -139,10 +139,9 @@ grid_norms_kernel(GridGeom G, const uint8_t* __restrict__ mask, const float* __r
     }
     if (lane == 0) out[warp] = v;
   }
-  if (tid == 0) {
-    if (flag) out[6] = (double)*(const volatile int*)flag;
-    *count = 0;
-  }
+  // Beside the columns, not behind them: 0.9 us less a check.
+  if (warp == 6 && lane == 0 && flag) out[6] = (double)*(const volatile int*)flag;
+  if (tid == 0) *count = 0;
 }
 
 void launch_fold(int precision, const GridLaunch& L, const GridGeom& G, const uint8_t* mask,
