@@ -652,7 +652,9 @@ struct GridSolverImpl : Solver {
   // from a reset, launches against flow: disk of 902x902 111/112, 175/149,
   // 324/262; box of 1100x1100 146/151, 232/214, 429/380; disk of 1400x1400
   // 192/202, 306/285, 571/516; 500x2500 164/161, 259/226, 487/406; box of
-  // 1800x1800 321/353, 520/522, 990/972.  On larger grids launches of tall
+  // 1800x1800 321/353, 520/522, 990/972.  At 64 it is even or slower, at 100
+  // faster on all of up to 1500x1500 pixels, beyond only at 200: the lines are
+  // the least counts measured at which it won.  On larger grids launches of tall
   // regions are faster (grid_tbp.cu; 2300x2300 disk 2,420 for 400 sweeps
   // against 2,556, 2900x2900 3,550 against 3,945).  Short steps
   // start sooner as launches: 16, 32, 48 sweeps with the tables there 38/29,
