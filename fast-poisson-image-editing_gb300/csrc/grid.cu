@@ -232,6 +232,9 @@ struct GridSolverImpl : Solver {
     return precision == FPIE_FP32 && !red_black && res.rows > 0 && (!pinned || !res_pin.empty());
   }
 
+  // At most as many sweeps as a launch can count in periods of 16: past 2^31 -
+  // 16 its loop would not end.
+  static constexpr int kResSweeps = 1 << 30;
   void run_res(int iters, const double* maxima = nullptr, double tol = 0.0) {
     if (!res_exchange) {
       const size_t b = res_exchange_bytes(G);
@@ -946,6 +949,7 @@ struct GridSolverImpl : Solver {
     const bool cap = capturing(), recorded = cap && !pinned && !tuned;
     const bool resident = use_res() && !recorded, few = resident && few_sweeps(iters);
     if (resident && !few) {
+      for (; iters > kResSweeps; iters -= kResSweeps) run_res(kResSweeps);
       run_res(iters);
       return;
     }
@@ -1247,7 +1251,7 @@ struct GridSolverImpl : Solver {
     queue_norms(slot);
     FPIE_CUDA(cudaEventRecord(norm_done[slot], stream));
     for (;; slot ^= 1) {
-      const int k = std::min(check_every, max_sweeps - done);
+      const int k = std::min({check_every, max_sweeps - done, kResSweeps});
       if (k > 0) {
         run_res(k, h_norm + kNorm * slot, tol);
         queue_norms(slot ^ 1);
