@@ -312,8 +312,10 @@ struct Solver {
   long long launches = 0;
   int precision = FPIE_FP32;
   virtual ~Solver() {}
-  // Raises the error a kernel recorded in device memory (e.g. a bounded wait
-  // that timed out); called after the stream has been synchronised.
+  // The error a kernel recorded in device memory (e.g. a bounded wait that
+  // timed out): queue_check queues a copy of it, check_async raises it once the
+  // stream has been synchronised.
+  virtual void queue_check() {}
   virtual void check_async() {}
   void activate() const { FPIE_CUDA(cudaSetDevice(device)); }
 };

@@ -69,8 +69,11 @@ __global__ void equ_check_kernel(EquGeom E, const int4* __restrict__ A,
   if (nbad) atomicAdd(bad, nbad);
 }
 
+// flag, unless NULL, goes to err[3] (pinned).
 __global__ void equ_unpack_kernel(EquGeom E, const float* __restrict__ x,
-                                  float* __restrict__ out) {
+                                  float* __restrict__ out, float* err, const int* flag) {
+  if (flag && blockIdx.x == 0 && threadIdx.x == 0)
+    err[3] = __int_as_float(*(const volatile int*)flag);
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < E.N;
        i += (long long)gridDim.x * blockDim.x) {
 #pragma unroll
@@ -644,6 +647,11 @@ struct EquSolverImpl : Solver {
     }
   }
 
+  void queue_check() override {
+    if (!grid) return;
+    grid->stream = stream;
+    grid->queue_check();
+  }
   void check_async() override {
     if (grid) grid->check_async();
   }
@@ -1010,11 +1018,12 @@ struct EquSolverImpl : Solver {
     sync_from_grid();
     AsyncScratch scratch((size_t)E.N * 12, stream);
     float* tmp = reinterpret_cast<float*>(scratch.bytes());
-    equ_unpack_kernel<<<conv_blocks(E.N), 256, 0, stream>>>(E, x[cur], tmp);
+    equ_unpack_kernel<<<conv_blocks(E.N), 256, 0, stream>>>(E, x[cur], tmp, h_err,
+                                                            grid_wait_flag(grid));
     post_launch(this);
     FPIE_CUDA(cudaMemcpyAsync(out, tmp, (size_t)E.N * 12, cudaMemcpyDeviceToHost, stream));
     FPIE_CUDA(cudaStreamSynchronize(stream));
-    check_async();
+    grid_raise(grid, h_err + 3);
   }
 };
 

@@ -138,8 +138,12 @@ __global__ void grid_pack_kernel(GridGeom G, const int32_t* __restrict__ mk,
   }
 }
 
+// flag, unless NULL, goes to err[3] (pinned): a copy of its own and a second
+// wait for it made 10 us of a state's 32.
 __global__ void grid_unpack_kernel(GridGeom G, const float* __restrict__ x,
-                                   float* __restrict__ out) {
+                                   float* __restrict__ out, float* err, const int* flag) {
+  if (flag && blockIdx.x == 0 && threadIdx.x == 0)
+    err[3] = __int_as_float(*(const volatile int*)flag);
   const long long total = (long long)G.n * G.m;
   for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
        idx < total; idx += (long long)gridDim.x * blockDim.x) {
@@ -179,7 +183,9 @@ struct GridSolverImpl : Solver {
   // kernel's copy waits) give up after spin_limit rounds and set d_wait_err.
   long long spin_limit = 1LL << 26;  // x ~64 ns sleeps: a few seconds at most
   int* d_wait_err = nullptr;  // in d_err
-  bool waits = false;         // a launch that may set it was queued
+  bool waits = false;         // a launch that may set it alone was queued
+  // Set by the resident kernel beside it, in pinned memory.
+  volatile int* gave_up() const { return reinterpret_cast<int*>(h_err + 4); }
 
   // ---- persistent TMA-prefetch kernel (variant index kTma; by name only) -----
   static constexpr int kTma = -3;
@@ -245,9 +251,8 @@ struct GridSolverImpl : Solver {
       check_range();
       range_due = capturing();  // recorded only: the next step looks again
     }
-    waits = true;
     launch_res(G, res, mask, g, x[cur], x[cur ^ 1], res_exchange, res_ctl, wild(), iters,
-               d_wait_err, spin_limit, stream, maxima, tol);
+               d_wait_err, const_cast<int*>(gave_up()), spin_limit, stream, maxima, tol);
     post_launch(this);
     cur ^= 1;
   }
@@ -257,10 +262,11 @@ struct GridSolverImpl : Solver {
   // of up to 16 sweeps takes 7-17 us once its tile flags are there.  us for 1,
   // 8, 16, 24 sweeps, resident against launches: 38x38 11/7, 11/11, 11/13,
   // 13/22; 194x194 17/9, 17/13, 19/17, 22/27; 660x660 21/9, 25/13, 28/17,
-  // 35/27.  A reset's first such step would pay for the flags (6 us): it stays.
+  // 35/27; back to back 38x38 5 sweeps 8.3/6.3, 6 8.3/8.3.  A reset's first such
+  // step would pay for the flags (6 us): it stays.
   int few_steps = 0;  // since the reset
   bool few_sweeps(int iters) {
-    if (!res_pin.empty() || iters > (res_whole(res, G.n, G.m) ? 4 : 16)) return false;
+    if (!res_pin.empty() || iters > (res_whole(res, G.n, G.m) ? 5 : 16)) return false;
     return few_steps++ > 0;
   }
 
@@ -280,14 +286,21 @@ struct GridSolverImpl : Solver {
     maybe_wild = false;
   }
 
-  // Reads and clears the wait-error flag (a flow-kernel neighbourhood wait
-  // or a TMA copy wait that gave up); call after the stream has been
-  // synchronised.
+  // Reads and clears the wait-error flag (a flow-kernel neighbourhood wait, a
+  // resident kernel's wait for packets or a TMA copy wait that gave up).
   void check_waits() {
-    if (!d_wait_err || !waits) return;
-    FPIE_CUDA(cudaMemcpyAsync(h_err + 3, d_wait_err, sizeof(int), cudaMemcpyDeviceToHost, stream));
+    queue_check();
     FPIE_CUDA(cudaStreamSynchronize(stream));
-    raise_waits();
+    check_async();
+  }
+  void queue_check() override {
+    if (d_wait_err && waits)
+      FPIE_CUDA(cudaMemcpyAsync(h_err + 3, d_wait_err, sizeof(int), cudaMemcpyDeviceToHost, stream));
+  }
+  void check_async() override {
+    if (!d_wait_err) return;
+    if (*gave_up()) raise_wait();
+    if (waits) raise_waits();
   }
   // The flag as h_err[3] holds it.
   void raise_waits() {
@@ -298,9 +311,9 @@ struct GridSolverImpl : Solver {
   [[noreturn]] void raise_wait() {
     FPIE_CUDA(cudaMemsetAsync(d_wait_err, 0, sizeof(int), stream));
     FPIE_CUDA(cudaStreamSynchronize(stream));
+    *gave_up() = 0;
     throw Error{FPIE_ERR_TIMEOUT, "sweep kernel: a bounded device wait gave up"};
   }
-  void check_async() override { check_waits(); }
 
   // All `iters` sweeps in one launch of the dependency-flow kernel.  A wait
   // that timed out is reported at the next host synchronisation.
@@ -352,7 +365,8 @@ struct GridSolverImpl : Solver {
     FPIE_CUDA(cudaGetDevice(&device));
     FPIE_CUDA(cudaStreamCreateWithFlags(&own_stream, cudaStreamNonBlocking));
     stream = own_stream;
-    FPIE_CUDA(cudaMallocHost(&h_err, 4 * sizeof(float)));
+    FPIE_CUDA(cudaMallocHost(&h_err, 5 * sizeof(float)));
+    *gave_up() = 0;
   }
 
   ~GridSolverImpl() override {
@@ -394,6 +408,7 @@ struct GridSolverImpl : Solver {
 
   void release() {
     cudaStreamSynchronize(stream);  // NULL (legacy default stream) included
+    *gave_up() = 0;
     drop_graphs();
     cudaFree(arena);
     arena = nullptr;
@@ -1405,11 +1420,11 @@ struct GridSolverImpl : Solver {
     const long long total = (long long)G.n * G.m;
     AsyncScratch scratch(total * 12, stream);
     float* tmp = reinterpret_cast<float*>(scratch.bytes());
-    grid_unpack_kernel<<<conv_blocks(total), 256, 0, stream>>>(G, x[cur], tmp);
+    grid_unpack_kernel<<<conv_blocks(total), 256, 0, stream>>>(G, x[cur], tmp, h_err, d_wait_err);
     post_launch(this);
     FPIE_CUDA(cudaMemcpyAsync(out, tmp, total * 12, cudaMemcpyDeviceToHost, stream));
     FPIE_CUDA(cudaStreamSynchronize(stream));
-    check_waits();
+    raise_waits();
   }
 };
 

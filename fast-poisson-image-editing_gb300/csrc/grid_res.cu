@@ -57,6 +57,7 @@ struct ResArgs {
   unsigned* ctl;                // [0] epoch base, [1] CTAs that left
   const unsigned* wild;
   int* error;
+  int* host_error;
   long long spin_limit;
   // Host or device: the residual maxima of xin; nothing is done if they are
   // within tol.  NULL: none.
@@ -415,6 +416,7 @@ __global__ void __launch_bounds__(W * 32, 1) grid_res_kernel(ResArgs A) {
   }
   __syncthreads();
   if (threadIdx.x == 0) {
+    if (s_stop) *(volatile int*)A.host_error = 1;
     // Every CTA read the base before it comes here, so the last one may move it.
     __threadfence();
     if (atomicAdd(A.ctl + 1, 1u) == gridDim.x - 1) {
@@ -569,8 +571,8 @@ size_t res_exchange_bytes(const GridGeom& G) {
 
 void launch_res(const GridGeom& G, const ResShape& s, const uint8_t* mask, const float* g,
                 const float* xin, float* xout, void* exchange, unsigned* ctl,
-                const unsigned* wild, int sweeps, int* error, long long spin_limit,
-                cudaStream_t st, const double* maxima, double tol) {
+                const unsigned* wild, int sweeps, int* error, int* host_error,
+                long long spin_limit, cudaStream_t st, const double* maxima, double tol) {
   const ResKernel* k = res_kernel(s);
   FPIE_REQUIRE(k != nullptr, FPIE_ERR_STATE, "no such resident kernel");
   const int tiles = res_tiles(s, G.n, G.m);
@@ -582,8 +584,8 @@ void launch_res(const GridGeom& G, const ResShape& s, const uint8_t* mask, const
   uint4* packets = reinterpret_cast<uint4*>(static_cast<char*>(exchange) + 4096);
   ResArgs a{G,    mask,       g,       xin,
             xout, packets,    act,     ctl,
-            wild, error,      std::min(spin_limit, 1LL << 23), maxima, tol,
-            tiles_x, tiles, sweeps};
+            wild, error,      host_error, std::min(spin_limit, 1LL << 23),
+            maxima, tol,      tiles_x, tiles, sweeps};
   void* args[] = {&a};
   FPIE_CUDA(cudaLaunchCooperativeKernel(tiles > 1 ? k->kernel : k->whole, dim3(3 * tiles),
                                         dim3(s.warps * 32), args, tiles > 1 ? res_smem(s) : 0, st));

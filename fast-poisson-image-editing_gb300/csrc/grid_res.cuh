@@ -41,12 +41,14 @@ constexpr int kResCtl = 4;
 // `sweeps` Jacobi sweeps from xin; every tile holding a masked pixel is
 // written to xout.  wild: nonzero where the inputs are outside the range in
 // which the quartered form is exact (wild in grid.cu).  A wait that exceeds
-// spin_limit polls sets *error and the launch stops early.  maxima: the three
+// spin_limit polls sets *error and *host_error (pinned memory: the host needs no
+// copy to know) and the launch stops early.  maxima: the three
 // channels' largest residuals of xin, where a launch is queued before the host
 // knows them; if none is beyond tol the launch leaves everything as it is.
 void launch_res(const GridGeom& G, const ResShape& s, const uint8_t* mask, const float* g,
                 const float* xin, float* xout, void* exchange, unsigned* ctl,
-                const unsigned* wild, int sweeps, int* error, long long spin_limit,
-                cudaStream_t st, const double* maxima = nullptr, double tol = 0.0);
+                const unsigned* wild, int sweeps, int* error, int* host_error,
+                long long spin_limit, cudaStream_t st, const double* maxima = nullptr,
+                double tol = 0.0);
 
 }  // namespace fpie

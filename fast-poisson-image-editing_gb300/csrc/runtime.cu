@@ -133,6 +133,7 @@ int fpie_destroy(fpie_solver* s) {
 int fpie_sync(fpie_solver* s) {
   return guarded([&] {
     Solver* h = check_handle(s, 0);
+    h->queue_check();
     FPIE_CUDA(cudaStreamSynchronize(h->stream));
     h->check_async();
   });
