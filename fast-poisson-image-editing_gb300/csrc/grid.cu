@@ -257,16 +257,17 @@ struct GridSolverImpl : Solver {
     cur ^= 1;
   }
 
-  // Repeated steps of a few sweeps: a resident step starts with 11 us (whole
+  // Repeated steps of a few sweeps: a resident step starts with 8 us (whole
   // grids) to 21 us of loads, tables and the tiles' first exchange, a launch
-  // of up to 16 sweeps takes 7-17 us once its tile flags are there.  us for 1,
-  // 8, 16, 24 sweeps, resident against launches: 38x38 11/7, 11/11, 11/13,
-  // 13/22; 194x194 17/9, 17/13, 19/17, 22/27; 660x660 21/9, 25/13, 28/17,
-  // 35/27; back to back 38x38 5 sweeps 8.3/6.3, 6 8.3/8.3.  A reset's first such
-  // step would pay for the flags (6 us): it stays.
+  // of up to 16 sweeps takes 6-15 us once its tile flags are there.  Resident
+  // against launches, back to back: one region of 38x38 5 sweeps 8.3/6.3 us, 6
+  // 8.3/8.3; by a step's sweeps 194x194 16 1.13, 17 0.90; 400x300 17 1.01, 20
+  // 0.94; 333x517 20 1.02, 24 0.98; 176x1457 32 1.07, 40 0.91; 660x660 48 1.06,
+  // 64 1.02-1.06, 72 0.98; 802x802 17 1.03, 20 0.94 (grid_res.cu: few).  A
+  // reset's first such step would pay for the flags (6 us): it stays.
   int few_steps = 0;  // since the reset
   bool few_sweeps(int iters) {
-    if (!res_pin.empty() || iters > (res_whole(res, G.n, G.m) ? 5 : 16)) return false;
+    if (!res_pin.empty() || iters > res_few(res, G.n, G.m)) return false;
     return few_steps++ > 0;
   }
 

@@ -432,14 +432,16 @@ struct ResKernel {
   // the whole grid in one tile (no exchange).  Neither depends on the grid:
   // every CTA does the same work, whatever their number.
   float many, one;
+  int few;  // steps of up to so many sweeps are faster as launches (GridSolverImpl::few_sweeps)
   const void *kernel, *whole;
 };
 
 template <int R, int W, int LW, int K>
-ResKernel res_make(float many, float one) {
+ResKernel res_make(float many, float one, int few) {
   return {{R, W, 4 * LW, K},
           many,
           one,
+          few,
           (const void*)grid_res_kernel<R, W, LW, K, false>,
           (const void*)grid_res_kernel<R, W, LW, 8, true>};
 }
@@ -449,16 +451,16 @@ ResKernel res_make(float many, float one) {
 // for the largest tiles, where deeper ones would not fit on the SMs.
 const std::vector<ResKernel>& res_kernels() {
   static const std::vector<ResKernel> v = {
-      res_make<6, 4, 16, 8>(0.310f, 0.128f),    // tiles of 32 x 48
-      res_make<8, 4, 16, 8>(0.345f, 0.161f),    // 48 x 48
-      res_make<8, 8, 32, 8>(0.461f, 0.267f),    // 48 x 112
-      res_make<6, 4, 16, 16>(0.220f, 0.128f),   // 16 x 32
-      res_make<8, 4, 16, 16>(0.266f, 0.161f),   // 32 x 32
-      res_make<8, 8, 16, 16>(0.383f, 0.275f),   // 96 x 32
-      res_make<8, 8, 32, 16>(0.385f, 0.267f),   // 32 x 96
-      res_make<12, 8, 32, 16>(0.523f, 0.376f),  // 64 x 96
-      res_make<16, 8, 32, 16>(0.645f, 0.488f),  // 96 x 96
-      res_make<16, 8, 32, 4>(0.925f, 0.490f),   // 120 x 120
+      res_make<6, 4, 16, 8>(0.310f, 0.128f, 16),    // tiles of 32 x 48
+      res_make<8, 4, 16, 8>(0.345f, 0.161f, 16),    // 48 x 48
+      res_make<8, 8, 32, 8>(0.461f, 0.267f, 20),    // 48 x 112
+      res_make<6, 4, 16, 16>(0.220f, 0.128f, 16),   // 16 x 32
+      res_make<8, 4, 16, 16>(0.266f, 0.161f, 16),   // 32 x 32
+      res_make<8, 8, 16, 16>(0.383f, 0.275f, 17),   // 96 x 32
+      res_make<8, 8, 32, 16>(0.385f, 0.267f, 17),   // 32 x 96
+      res_make<12, 8, 32, 16>(0.523f, 0.376f, 32),  // 64 x 96
+      res_make<16, 8, 32, 16>(0.645f, 0.488f, 64),  // 96 x 96
+      res_make<16, 8, 32, 4>(0.925f, 0.490f, 17),   // 120 x 120
   };
   return v;
 }
@@ -513,7 +515,11 @@ int res_tiles(const ResShape& s, int n, int m) {
 
 }  // namespace
 
-bool res_whole(const ResShape& s, int n, int m) { return res_tiles(s, n, m) == 1; }
+// A one-region grid needs no exchange before it sweeps.
+int res_few(const ResShape& s, int n, int m) {
+  const ResKernel* k = res_kernel(s);
+  return !k ? 0 : res_tiles(s, n, m) == 1 ? 5 : k->few;
+}
 
 static ResShape res_parse(const char* name) {
   ResShape s{0, 0, 0, 0};

@@ -28,8 +28,9 @@ ResShape res_pick(int n, int m);
 // its tiles of an n x m grid do not fit.
 ResShape res_named(const char* name, int n, int m);
 bool res_is_name(const char* name);
-// Whether one region of shape s holds the whole n x m grid.
-bool res_whole(const ResShape& s, int n, int m);
+// The sweeps up to which repeated steps of an n x m grid on shape s are faster
+// as launches.
+int res_few(const ResShape& s, int n, int m);
 
 // Device memory of an exchange over geometry G: two buffers of packets for
 // any shape that fits, and the activity words; must be zero before the first
